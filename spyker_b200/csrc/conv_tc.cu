@@ -31,6 +31,7 @@
 #include <type_traits>
 
 #include "conv_tc.cuh"
+#include "search_write.cuh"
 #include "tc_ptx.cuh"
 
 #include <cuda_bf16.h>
@@ -2651,243 +2652,6 @@ __global__ void __launch_bounds__(128) search_fix_kernel(TcParams P, const float
     }
 }
 
-// Per-pixel winner and first-step bytes (t0 = T: never) of maps too large to
-// stage in shared memory: wbytes [npix], then tbytes [npix].
-__global__ void search_codes_kernel(const int4 *__restrict__ records, uint8_t *__restrict__ codes, int64_t npix,
-                                    int T, const int *negw, const int *flag)
-{
-    if (*negw || *flag) return;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < npix; i += int64_t(gridDim.x) * blockDim.x)
-    {
-        const int4 r = records[i];
-        codes[i] = uint8_t(r.x);
-        codes[npix + i] = uint8_t(min(r.y, T));
-    }
-}
-
-// Byte-parallel tests on four pixels at once (bytes below 0x80): the bytes
-// of w that equal c, and the bytes of t0 at or below t, as 0x80 flags.
-__device__ __forceinline__ uint32_t bytes_eq(uint32_t w, uint32_t c4)
-{
-    const uint32_t x = w ^ c4;
-    return ~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x | 0x7F7F7F7Fu);
-}
-__device__ __forceinline__ uint32_t bytes_le(uint32_t t0, uint32_t t4) { return ((t4 | 0x80808080u) - t0) & 0x80808080u; }
-
-// Spikes (and pooled spikes) of the search path from the per-pixel records:
-// channel w fires from step t0 on.  A CTA per sample writes its
-// [T, C, OH, OW] block; per pixel the winner and first-step bytes sit in
-// shared memory (or in global memory for maps above 16384 pixels).  Pooled
-// spikes [T, C, POH, POW] come from a byte table of the first firing step
-// per (channel, cell): a cell fires from the earliest t0 of its window's
-// pixels won by that channel.  Off the search path (negative weights or
-// other input) it writes zeros, which the dense kernel then fills.
-//
-// The block is written by (channel, pixel) slabs of one step: when a slab of
-// C x HW bytes is a multiple of V (16 or 4) and a plane a multiple of 4
-// pixels, a thread takes one V-byte chunk of the slab (4-pixel words, each
-// inside one plane), reads its pixels' winner and first-step bytes once and
-// writes that chunk for every step (T stores of one byte-parallel compare
-// and mask per word); other shapes take a byte per thread.
-template <int V>
-__device__ __forceinline__ void write_slab_words(uint8_t *dst, int T, int C, int hw, bool lean, bool pass0,
-                                                 const uint8_t *wsrc, const uint8_t *tsrc, int tstride)
-{
-    constexpr int NW = V / 4;
-    using Vec = typename std::conditional<V == 16, uint4, uint32_t>::type;
-    const int slab = C * hw, nq = slab / V;
-    for (int q = threadIdx.x; q < nq; q += blockDim.x)
-    {
-        uint32_t eq[NW], tw[NW];
-#pragma unroll
-        for (int r = 0; r < NW; ++r)
-        {
-            const int f = V * q + 4 * r, c = f / hw, px = f - c * hw;
-            if (pass0)
-            {
-                eq[r] = bytes_eq(*reinterpret_cast<const uint32_t *>(wsrc + px), uint32_t(c) * 0x01010101u);
-                tw[r] = *reinterpret_cast<const uint32_t *>(tsrc + px);
-            }
-            else
-            {
-                eq[r] = 0x80808080u;
-                tw[r] = *reinterpret_cast<const uint32_t *>(tsrc + c * tstride + px);
-            }
-            if (!lean) eq[r] = 0u;
-        }
-        Vec *d = reinterpret_cast<Vec *>(dst) + q;
-        for (int t = 0; t < T; ++t)
-        {
-            const uint32_t t4 = uint32_t(t) * 0x01010101u;
-            if constexpr (V == 16)
-                d[int64_t(t) * nq] =
-                    make_uint4((eq[0] & bytes_le(tw[0], t4)) >> 7, (eq[1] & bytes_le(tw[1], t4)) >> 7,
-                               (eq[2] & bytes_le(tw[2], t4)) >> 7, (eq[3] & bytes_le(tw[3], t4)) >> 7);
-            else
-                d[int64_t(t) * nq] = (eq[0] & bytes_le(tw[0], t4)) >> 7;
-        }
-    }
-}
-
-// Maps above 16384 pixels (per-pixel winner and first-step bytes in global
-// memory): a grid of CTAs per sample (blockIdx.y), each thread one 16-byte
-// chunk of a step's (channel, pixel) slab for every step; pooled spikes a
-// 4-cell word at a time, each cell's first firing step for the word's channel
-// taken over its window (T: never) and compared with every step.  Needs
-// C x OH x OW a multiple of 16, OH x OW and the pooled width multiples of 4.
-__global__ void __launch_bounds__(256) search_write_large_kernel(const uint8_t *__restrict__ codes, int64_t npix,
-                                                                 const int *negw, const int *flag,
-                                                                 uint8_t *__restrict__ spikes,
-                                                                 uint8_t *__restrict__ pooled, int T, int C, int ohw,
-                                                                 int ow, int pky, int pkx, int poh, int pow_)
-{
-    const bool lean = !*negw && !*flag;
-    const int64_t smp = blockIdx.y;
-    const uint8_t *wb = codes + smp * ohw, *tb = codes + npix + smp * ohw;
-    const int64_t step = int64_t(gridDim.x) * blockDim.x;
-    {
-        const int64_t slab = int64_t(C) * ohw, nq = slab / 16;
-        uint4 *dst = reinterpret_cast<uint4 *>(spikes + smp * T * slab);
-        for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < nq; q += step)
-        {
-            uint32_t eq[4], tw[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-            {
-                const int64_t f = 16 * q + 4 * r;
-                const int c = int(f / ohw), px = int(f - int64_t(c) * ohw);
-                eq[r] = lean ? bytes_eq(*reinterpret_cast<const uint32_t *>(wb + px), uint32_t(c) * 0x01010101u) : 0u;
-                tw[r] = *reinterpret_cast<const uint32_t *>(tb + px);
-            }
-            for (int t = 0; t < T; ++t)
-            {
-                const uint32_t t4 = uint32_t(t) * 0x01010101u;
-                dst[int64_t(t) * nq + q] =
-                    make_uint4((eq[0] & bytes_le(tw[0], t4)) >> 7, (eq[1] & bytes_le(tw[1], t4)) >> 7,
-                               (eq[2] & bytes_le(tw[2], t4)) >> 7, (eq[3] & bytes_le(tw[3], t4)) >> 7);
-            }
-        }
-    }
-    if (pooled == nullptr) return;
-    const int phw = poh * pow_;
-    const int64_t slab = int64_t(C) * phw, nw = slab / 4;
-    uint32_t *dst = reinterpret_cast<uint32_t *>(pooled + smp * T * slab);
-    for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < nw; q += step)
-    {
-        const int64_t f = 4 * q;
-        const int c = int(f / phw), cell = int(f - int64_t(c) * phw), py = cell / pow_, px = cell - py * pow_;
-        uint32_t first = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-        {
-            int m = T;
-            for (int dy = 0; dy < pky; ++dy)
-                for (int dx = 0; dx < pkx; ++dx)
-                {
-                    const int i = (py * pky + dy) * ow + (px + j) * pkx + dx;
-                    if (int(wb[i]) == c) m = min(m, int(tb[i]));
-                }
-            first |= uint32_t(m) << (8 * j);
-        }
-        for (int t = 0; t < T; ++t)
-            dst[int64_t(t) * nw + q] = lean ? bytes_le(first, uint32_t(t) * 0x01010101u) >> 7 : 0u;
-    }
-}
-
-__global__ void __launch_bounds__(256) search_write_kernel(const int4 *__restrict__ records,
-                                                           const uint8_t *__restrict__ gcodes, int64_t npix,
-                                                           const int *negw, const int *flag,
-                                                           uint8_t *__restrict__ spikes, uint8_t *__restrict__ pooled,
-                                                           int64_t b, int T, int C, int ohw, int ow, int pky,
-                                                           int pkx, int poh, int pow_, int ptab)
-{
-    // [ohw16] winner bytes, [ohw16] first-step bytes, then [C][phw16] pooled first steps
-    extern __shared__ __align__(16) uint8_t wsm_[];
-    const bool lean = !*negw && !*flag;
-    const int ohw16 = (ohw + 15) & ~15, phw = poh * pow_, phw16 = (phw + 15) & ~15;
-    // (maps above 16384 pixels keep their bytes in global memory: the table
-    // then starts at byte 32, as the launch sizes it)
-    uint8_t *sw = wsm_, *st = wsm_ + ohw16, *first = wsm_ + (gcodes ? 32 : 2 * ohw16);
-    for (int64_t smp = blockIdx.x; smp < b; smp += gridDim.x)
-    {
-        const uint8_t *wsrc = gcodes ? gcodes + smp * ohw : sw;
-        const uint8_t *tsrc = gcodes ? gcodes + npix + smp * ohw : st;
-        if (lean && !gcodes)
-            for (int p = threadIdx.x; p < ohw; p += blockDim.x)
-            {
-                const int4 r = records[smp * ohw + p];
-                sw[p] = uint8_t(r.x), st[p] = uint8_t(min(r.y, T));
-            }
-        if (lean && ptab)
-            for (int i = threadIdx.x; i < C * phw16; i += blockDim.x) first[i] = uint8_t(T);
-        __syncthreads();
-        if (lean && ptab)
-        {
-            // earliest t0 per (channel, cell): bytes updated through their word
-            for (int p = threadIdx.x; p < ohw; p += blockDim.x)
-            {
-                const int y = p / ow, x = p - y * ow, py = y / pky, px = x / pkx;
-                const int t0 = int(tsrc[p]);
-                if (py < poh && px < pow_ && t0 < T)
-                {
-                    const int idx = int(wsrc[p]) * phw16 + py * pow_ + px;
-                    unsigned *word = reinterpret_cast<unsigned *>(first + (idx & ~3));
-                    const int sh = 8 * (idx & 3);
-                    unsigned old = *word;
-                    while (int((old >> sh) & 0xFF) > t0)
-                    {
-                        const unsigned nw = (old & ~(0xFFu << sh)) | (unsigned(t0) << sh);
-                        const unsigned seen = atomicCAS(word, old, nw);
-                        if (seen == old) break;
-                        old = seen;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-        for (int pass = 0; pass < (pooled ? 2 : 1); ++pass)
-        {
-            const int hw = pass == 0 ? ohw : phw;
-            const int64_t n = int64_t(T) * C * hw;
-            uint8_t *dst = (pass == 0 ? spikes : pooled) + smp * n;
-            const bool table = pass == 0 || ptab || !lean;
-            const uintptr_t a = reinterpret_cast<uintptr_t>(dst);
-            if (table && (int64_t(C) * hw) % 16 == 0 && hw % 4 == 0 && (a & 15) == 0 &&
-                (gcodes == nullptr || ohw % 4 == 0))
-                write_slab_words<16>(dst, T, C, hw, lean, pass == 0, wsrc, pass == 0 ? tsrc : first, phw16);
-            else if (table && (int64_t(C) * hw) % 4 == 0 && hw % 4 == 0 && (a & 3) == 0 &&
-                     (gcodes == nullptr || ohw % 4 == 0))
-                write_slab_words<4>(dst, T, C, hw, lean, pass == 0, wsrc, pass == 0 ? tsrc : first, phw16);
-            else
-                for (int64_t f = threadIdx.x; f < n; f += blockDim.x)
-                {
-                    uint8_t v = 0;
-                    if (lean)
-                    {
-                        const int plane = int(f / hw), px = int(f - int64_t(plane) * hw);
-                        const int t = plane / C, c = plane - t * C;
-                        if (pass == 0)
-                            v = (int(wsrc[px]) == c && int(tsrc[px]) <= t) ? 1 : 0;
-                        else if (ptab)
-                            v = int(first[c * phw16 + px]) <= t ? 1 : 0;
-                        else
-                        {
-                            const int py = px / pow_, pxx = px - py * pow_;
-                            for (int dy = 0; dy < pky; ++dy)
-                                for (int dx = 0; dx < pkx; ++dx)
-                                {
-                                    const int q = (py * pky + dy) * ow + pxx * pkx + dx;
-                                    v |= (int(wsrc[q]) == c && int(tsrc[q]) <= t) ? 1 : 0;
-                                }
-                        }
-                    }
-                    dst[f] = v;
-                }
-        }
-        __syncthreads();
-    }
-}
-
 inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
 // Schedule overrides of the tensor-core kernels (0 = automatic), set by an
@@ -3571,39 +3335,11 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
         // the next bisection round's list (round 0 without a list: all pixels)
         if (r < nsr) compact(r == 0 && !prefilter ? nullptr : P.count_in, r & 1 ? lb : la, cnt + r + 1);
     }
-    const int ohw = int(L.oh * L.ow);
-    uint8_t *gcodes = nullptr;
-    const size_t ohw16 = size_t((ohw + 15) & ~15);
-    size_t wsm = 2 * ohw16;
-    if (ohw > 16384)
-    {
-        // the bisection state is no longer needed: its bytes hold the codes
-        gcodes = reinterpret_cast<uint8_t *>(P.state);
-        wsm = 2 * 16;
-        search_codes_kernel<<<grid_for(L.npix, 256), 256, 0, s>>>(P.records, gcodes, L.npix, P.T, P.negw, P.flag);
-        SPK_LAUNCHED();
-    }
-    if (gcodes && (int64_t(P.cout) * ohw) % 16 == 0 && ohw % 4 == 0 && reinterpret_cast<uintptr_t>(spikes) % 16 == 0 &&
-        (pool_ky == 0 || (pow_ % 4 == 0 && reinterpret_cast<uintptr_t>(pooled) % 4 == 0)) && b <= 65535)
-    {
-        const int64_t nq = int64_t(P.cout) * ohw / 16;
-        const unsigned xb = unsigned(std::max<int64_t>(1, std::min<int64_t>(ceil_div(nq, 256 * 8),
-                                                                            ceil_div(int64_t(sm_count()) * 8, b))));
-        search_write_large_kernel<<<dim3(xb, unsigned(b)), 256, 0, s>>>(
-            gcodes, L.npix, P.negw, P.flag, spikes, pool_ky > 0 ? pooled : nullptr, P.T, P.cout, ohw, int(L.ow),
-            int(pool_ky), int(pool_kx), int(poh), int(pow_));
-        SPK_LAUNCHED();
-        return;
-    }
-    // byte table of first firing steps per (channel, pooled cell) when it fits
-    const size_t tab_bytes = size_t(P.cout) * size_t(((poh * pow_) + 15) & ~15);
-    const int ptab = pool_ky > 0 && wsm + tab_bytes <= 160 * 1024 ? 1 : 0;
-    if (ptab) wsm += tab_bytes;
-    SPK_CUDA(cudaFuncSetAttribute(search_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wsm)));
-    search_write_kernel<<<unsigned(std::min<int64_t>(b, int64_t(sm_count()) * 16)), 256, wsm, s>>>(
-        P.records, gcodes, L.npix, P.negw, P.flag, spikes, pool_ky > 0 ? pooled : nullptr, b, P.T, P.cout, ohw,
-        int(L.ow), int(pool_ky), int(pool_kx), int(poh), int(pow_), ptab);
-    SPK_LAUNCHED();
+    // (the bisection state is no longer needed: its bytes hold the writer's codes)
+    search_write(SearchWrite{P.records, reinterpret_cast<uint8_t *>(P.state), P.negw, P.flag, spikes,
+                             pool_ky > 0 ? pooled : nullptr, b, P.T, P.cout, int(L.oh), int(L.ow), int(pool_ky),
+                             int(pool_kx), int(poh), int(pow_)},
+                 s);
 }
 
 void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b, int64_t t, int64_t cin, int64_t h,
