@@ -10,6 +10,8 @@
 // Each round takes the first index of the maximum key (std::max_element),
 // stops on the sentinel, records the winner and suppresses the
 // (2ry+1) x (2rx+1) box over all channels plus (convwta) the whole channel.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace spk
@@ -19,54 +21,53 @@ namespace
 constexpr int kWtaThreads = 1024;
 constexpr int64_t kWtaSmemKeys = 40 * 1024;  // keys kept in shared memory up to 160 KB
 
-struct BestPair
+// A key as an order-preserving word (0: none) and its position k * blockDim +
+// tid (k: the thread's k-th position), so that positions compare as (k, tid).
+struct Best
 {
-    float v;
-    int64_t i;
+    unsigned e, k;
 };
 
-__device__ __forceinline__ BestPair better(BestPair a, BestPair b)
+__device__ __forceinline__ unsigned order_enc(float v)
 {
-    if (b.v > a.v) return b;
-    if (a.v > b.v) return a;
-    return (b.i < a.i) ? b : a;
+    const unsigned u = __float_as_uint(v + 0.0f);  // (-0 counts as 0)
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// Block-wide first-index argmax with std::max_element semantics.
-__device__ int64_t block_argmax(const float *keys, int64_t n, BestPair *s_pairs)
+// A thread's first largest key among its positions (tid, tid + blockDim, ...).
+__device__ __forceinline__ Best own_best(const float *keys, int64_t n)
 {
-    BestPair best{-INFINITY, INT64_MAX};
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
+    float v = -INFINITY;
+    unsigned best = 0, k = 0;
+    bool any = false;
+#pragma unroll 4
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x, ++k)
     {
-        float v = keys[i];
-        if (v != v) continue;  // NaN never replaces the running maximum
-        if (best.i == INT64_MAX || best.v < v) best = {v, i};
+        const float f = keys[i];
+        if (f != f) continue;  // NaN never replaces the running maximum
+        if (!any || v < f) v = f, best = k, any = true;
     }
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        BestPair other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
-        best = better(best, other);
-    }
+    return Best{any ? order_enc(v) : 0u, best};
+}
+
+// Block-wide first-index argmax with std::max_element semantics, from the
+// threads' own bests: per warp the largest word, its smallest k, its first
+// lane (two redux instructions and a ballot), then the same over the warps.
+__device__ __forceinline__ int64_t block_argmax(Best best, const float *keys, uint3 *s_best)
+{
+    const unsigned all = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) s_pairs[warp] = best;
+    unsigned e = __reduce_max_sync(all, best.e);
+    unsigned k = __reduce_min_sync(all, best.e == e ? best.k : all);
+    const unsigned who = __ballot_sync(all, best.e == e && best.k == k);
+    if (lane == 0) s_best[warp] = make_uint3(e, k, unsigned(warp * 32 + __ffs(who) - 1));
     __syncthreads();
-    if (warp == 0)
-    {
-        int nw = blockDim.x >> 5;
-        best = lane < nw ? s_pairs[lane] : BestPair{-INFINITY, INT64_MAX};
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            BestPair other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
-            best = better(best, other);
-        }
-        if (lane == 0) s_pairs[32] = best;
-    }
-    __syncthreads();
-    int64_t idx = s_pairs[32].i;
-    float k0 = keys[0];
-    if (k0 != k0 || idx == INT64_MAX) idx = 0;
-    __syncthreads();
-    return idx;
+    const uint3 w = lane < int(blockDim.x >> 5) ? s_best[lane] : make_uint3(0, all, all);
+    e = __reduce_max_sync(all, w.x);
+    k = __reduce_min_sync(all, w.x == e ? w.y : all);
+    const unsigned tid = __reduce_min_sync(all, w.x == e && w.y == k ? w.z : all);
+    const float k0 = keys[0];
+    return k0 != k0 || e == 0 ? 0 : int64_t(k) * blockDim.x + tid;
 }
 
 template <typename T>
@@ -76,13 +77,87 @@ __device__ __forceinline__ void minmax_update(T v, T &mn, T &mx)
     mx = (mx < v) ? v : mx;  // std::max(mx, v)
 }
 
+// F32 input, read once by the whole chip: per position the first step above
+// the threshold and its value, per block the smallest and largest value.
+// Bound by the read (T x X values a sample).  One CTA per sample read its
+// potentials twice and left SMs idle: 128 samples of 15 x 23520 took 228 us,
+// this scan and the rounds below 36 and 42 us.  V: 4 neighbouring positions per thread
+// where alignment allows, else 1.
+constexpr int kScanThreads = 256;
+constexpr uint16_t kNever = 0xFFFF;
+
+struct WtaCandidates
+{
+    float *value;     // [b][x], where step is not kNever
+    uint16_t *step;   // [b][x]
+    float2 *extreme;  // [b][blocks]
+    int blocks;
+};
+
+template <int V>
+__global__ void __launch_bounds__(kScanThreads)
+    wta_scan_kernel(const float *__restrict__ in, int t, int64_t x, float thr, WtaCandidates C)
+{
+    using Vec = typename std::conditional<V == 4, float4, float>::type;
+    __shared__ float s_mn[kScanThreads / 32], s_mx[kScanThreads / 32];
+    const int64_t b = blockIdx.y;
+    const float *sample = in + b * int64_t(t) * x;
+    float mn = sample[0], mx = mn;
+    const int64_t j = (int64_t(blockIdx.x) * kScanThreads + threadIdx.x) * V;
+    if (j < x)
+    {
+        float val[V];
+        int at[V];
+#pragma unroll
+        for (int l = 0; l < V; ++l) at[l] = kNever, val[l] = 0.f;
+        for (int q0 = 0; q0 < t; q0 += 8)
+        {
+            Vec r[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)  // (a step past the last reads the last again)
+                r[u] = __ldcs(reinterpret_cast<const Vec *>(sample + int64_t(min(q0 + u, t - 1)) * x + j));
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+            {
+                const float *v = reinterpret_cast<const float *>(&r[u]);
+#pragma unroll
+                for (int l = 0; l < V; ++l)
+                {
+                    minmax_update(v[l], mn, mx);
+                    if (at[l] == kNever && v[l] > thr) at[l] = min(q0 + u, t - 1), val[l] = v[l];
+                }
+            }
+        }
+#pragma unroll
+        for (int l = 0; l < V; ++l)
+        {
+            C.step[b * x + j + l] = uint16_t(at[l]);
+            if (at[l] != kNever) C.value[b * x + j + l] = val[l];
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        const float a = __shfl_xor_sync(0xffffffffu, mn, o), z = __shfl_xor_sync(0xffffffffu, mx, o);
+        minmax_update(a, mn, mx);
+        minmax_update(z, mn, mx);
+    }
+    if ((threadIdx.x & 31) == 0) s_mn[threadIdx.x >> 5] = mn, s_mx[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        for (int q = 1; q < kScanThreads / 32; ++q) minmax_update(s_mn[q], mn, mx), minmax_update(s_mx[q], mn, mx);
+        C.extreme[b * C.blocks + blockIdx.x] = make_float2(mn, mx);
+    }
+}
+
 template <typename T, bool kFloat>
 __global__ void __launch_bounds__(kWtaThreads)
     wta_kernel(const T *__restrict__ in, int t, int64_t x, int c, int h, int w, int ry, int rx, int count, bool whole,
-               T thr, int32_t *__restrict__ winners, int32_t *__restrict__ counts, float *__restrict__ gkeys)
+               T thr, int32_t *__restrict__ winners, int32_t *__restrict__ counts, float *__restrict__ gkeys,
+               WtaCandidates C)
 {
     extern __shared__ __align__(16) float smem_keys[];
-    __shared__ BestPair s_pairs[33];
+    __shared__ uint3 s_best[32];
     __shared__ T s_mn[32], s_mx[32];
     const int64_t b = blockIdx.x;
     float *keys = gkeys ? gkeys + b * x : smem_keys;
@@ -93,7 +168,14 @@ __global__ void __launch_bounds__(kWtaThreads)
     {
         T mn = sample[0], mx = sample[0];
         const int64_t tot = int64_t(t) * x;
-        for (int64_t i = threadIdx.x; i < tot; i += blockDim.x) minmax_update(sample[i], mn, mx);
+        if (C.step)
+            for (int i = threadIdx.x; i < C.blocks; i += blockDim.x)
+            {
+                const float2 e = C.extreme[b * C.blocks + i];
+                minmax_update(T(e.x), mn, mx), minmax_update(T(e.y), mn, mx);
+            }
+        else
+            for (int64_t i = threadIdx.x; i < tot; i += blockDim.x) minmax_update(sample[i], mn, mx);
         for (int o = 16; o > 0; o >>= 1)
         {
             T a = __shfl_xor_sync(0xffffffffu, mn, o), bb = __shfl_xor_sync(0xffffffffu, mx, o);
@@ -106,6 +188,30 @@ __global__ void __launch_bounds__(kWtaThreads)
         for (int q = 1; q < int(blockDim.x >> 5); ++q) minmax_update(s_mn[q], mn, mx), minmax_update(s_mx[q], mn, mx);
         const float fmn = float(mn);
         const float diff = __fmul_rn(__fsub_rn(float(mx), fmn), 2.0f);
+        if (C.step)
+            for (int64_t j0 = threadIdx.x; j0 < x; j0 += 8 * int64_t(blockDim.x))
+            {
+                int at[8];
+                float val[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                {
+                    const int64_t j = j0 + u * int64_t(blockDim.x);
+                    at[u] = j < x ? C.step[b * x + j] : kNever;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    val[u] = at[u] != kNever ? C.value[b * x + j0 + u * int64_t(blockDim.x)] : 0.f;
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                {
+                    const int64_t j = j0 + u * int64_t(blockDim.x);
+                    if (j < x)
+                        keys[j] = at[u] == kNever ? -FLT_MAX
+                                                  : __fadd_rn(float(t - at[u] - 1), __fdiv_rn(__fsub_rn(val[u], fmn), diff));
+                }
+            }
+        else
         for (int64_t j = threadIdx.x; j < x; j += blockDim.x)
         {
             float key = -FLT_MAX;
@@ -139,12 +245,18 @@ __global__ void __launch_bounds__(kWtaThreads)
     }
     __syncthreads();
 
+    // Keys only ever fall to `low`: a thread scans its positions again only
+    // when its own best was suppressed.
     const int64_t len = int64_t(h) * w;
+    Best best = own_best(keys, x);
     int found = 0;
     for (int r = 0; r < count; ++r)
     {
-        int64_t idx = block_argmax(keys, x, s_pairs);
+        if (r > 0 && best.e != 0 && order_enc(keys[int64_t(best.k) * blockDim.x + threadIdx.x]) != best.e)
+            best = own_best(keys, x);
+        int64_t idx = block_argmax(best, keys, s_best);
         float kv = keys[idx];
+        __syncthreads();  // every thread has read the key and the warps' bests
         bool stop = kFloat ? (fabsf(__fsub_rn(kv, -FLT_MAX)) < 1e-5f) : (fabsf(kv) < 1e-5f);
         if (stop) break;
         const int z = int(idx / len), y = int((idx % len) / w), xx = int((idx % len) % w);
@@ -155,12 +267,13 @@ __global__ void __launch_bounds__(kWtaThreads)
         }
         const int sj = max(0, y - ry), ej = min(h, y + ry + 1);
         const int sk = max(0, xx - rx), ek = min(w, xx + rx + 1);
-        const int bw = ek - sk, bh = ej - sj;
-        const int64_t box = int64_t(c) * bh * bw;
-        for (int64_t i = threadIdx.x; i < box; i += blockDim.x)
+        // a row of the box in one channel per thread
+        const unsigned bh = unsigned(ej - sj), rows = unsigned(c) * bh;
+        for (unsigned i = threadIdx.x; i < rows; i += blockDim.x)
         {
-            int64_t ch = i / (int64_t(bh) * bw), rem = i % (int64_t(bh) * bw);
-            keys[(ch * h + sj + rem / bw) * w + sk + rem % bw] = low;
+            const unsigned ch = i / bh;
+            float *row = keys + (int64_t(ch) * h + sj + (i - ch * bh)) * w;
+            for (int k = sk; k < ek; ++k) row[k] = low;
         }
         if (whole)
             for (int64_t i = threadIdx.x; i < len; i += blockDim.x) keys[int64_t(z) * len + i] = low;
@@ -170,6 +283,18 @@ __global__ void __launch_bounds__(kWtaThreads)
     if (threadIdx.x == 0) counts[b] = found;
 }
 
+size_t keys_bytes(int64_t b, int64_t x) { return x <= kWtaSmemKeys ? 0 : (size_t(b) * size_t(x) * 4 + 7) / 8 * 8; }
+
+// the scan's candidates: block extremes, values, steps
+size_t candidate_bytes(int64_t b, int64_t x) { return size_t(b) * (size_t(ceil_div(x, kScanThreads)) * 8 + size_t(x) * 6); }
+
+bool scan_applies(int64_t t, int64_t x) { return t * x >= 16384 && t < kNever && x < (int64_t(1) << 31); }
+
+size_t wta_workspace(int64_t b, int64_t t, int64_t x)
+{
+    return keys_bytes(b, x) + (scan_applies(t, x) ? candidate_bytes(b, x) : 0);
+}
+
 template <typename T, bool kFloat>
 void launch_wta(const void *in, int64_t b, int64_t t, int64_t c, int64_t h, int64_t w, int64_t ry, int64_t rx,
                 int64_t count, bool whole, double thr, int32_t *winners, int32_t *counts, void *ws, size_t ws_bytes,
@@ -177,18 +302,41 @@ void launch_wta(const void *in, int64_t b, int64_t t, int64_t c, int64_t h, int6
 {
     const int64_t x = c * h * w;
     float *gkeys = nullptr;
-    size_t smem = 0;
+    size_t smem = 0, used = 0;
     if (x <= kWtaSmemKeys)
         smem = size_t(x) * 4;
     else
     {
-        SPK_REQUIRE(ws != nullptr && ws_bytes >= size_t(b) * size_t(x) * 4, "workspace is too small");
+        used = keys_bytes(b, x);
+        SPK_REQUIRE(ws != nullptr && ws_bytes >= used, "workspace is too small");
         gkeys = reinterpret_cast<float *>(ws);
+    }
+    // F32 input goes through the scan where the caller's workspace has room
+    // for its candidates (else, and for samples that one CTA reads in a
+    // microsecond or two, the selection reads the input itself)
+    WtaCandidates C{};
+    if constexpr (std::is_same<T, float>::value)
+    {
+        const size_t all = used + candidate_bytes(b, x);
+        if (scan_applies(t, x) && b <= 65535 && ws != nullptr && ws_bytes >= all &&
+            reinterpret_cast<uintptr_t>(ws) % 8 == 0)
+        {
+            char *base = static_cast<char *>(ws) + used;
+            const bool vec = x % 4 == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0;
+            C.blocks = int(ceil_div(x, kScanThreads * (vec ? 4 : 1)));
+            C.extreme = reinterpret_cast<float2 *>(base);
+            C.value = reinterpret_cast<float *>(base + size_t(b) * ceil_div(x, kScanThreads) * 8);
+            C.step = reinterpret_cast<uint16_t *>(C.value + b * x);
+            const dim3 grid(unsigned(C.blocks), unsigned(b));
+            const auto scan = vec ? wta_scan_kernel<4> : wta_scan_kernel<1>;
+            scan<<<grid, kScanThreads, 0, s>>>((const float *)in, int(t), x, scalar_to<float>(thr), C);
+            SPK_LAUNCHED();
+        }
     }
     auto k = wta_kernel<T, kFloat>;
     SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     k<<<unsigned(b), kWtaThreads, smem, s>>>((const T *)in, int(t), x, int(c), int(h), int(w), int(ry), int(rx),
-                                             int(count), whole, scalar_to<T>(thr), winners, counts, gkeys);
+                                             int(count), whole, scalar_to<T>(thr), winners, counts, gkeys, C);
     SPK_LAUNCHED();
 }
 
@@ -216,10 +364,9 @@ using namespace spk;
 
 extern "C" {
 
-size_t spk_rank_convwta_workspace(int64_t b, int64_t, int64_t c, int64_t h, int64_t w)
+size_t spk_rank_convwta_workspace(int64_t b, int64_t t, int64_t c, int64_t h, int64_t w)
 {
-    int64_t x = c * h * w;
-    return x <= kWtaSmemKeys ? 0 : size_t(b) * size_t(x) * 4;
+    return wta_workspace(b, t, c * h * w);
 }
 
 spk_status spk_rank_convwta(const void *in, spk_dtype type, int64_t b, int64_t t, int64_t c, int64_t h, int64_t w,
@@ -232,7 +379,7 @@ spk_status spk_rank_convwta(const void *in, spk_dtype type, int64_t b, int64_t t
     });
 }
 
-size_t spk_rank_fcwta_workspace(int64_t b, int64_t, int64_t n) { return n <= kWtaSmemKeys ? 0 : size_t(b) * size_t(n) * 4; }
+size_t spk_rank_fcwta_workspace(int64_t b, int64_t t, int64_t n) { return wta_workspace(b, t, n); }
 
 spk_status spk_rank_fcwta(const void *in, spk_dtype type, int64_t b, int64_t t, int64_t n, int64_t radius,
                           int64_t count, double threshold, int32_t *winners, int32_t *counts, void *ws, size_t ws_bytes,
