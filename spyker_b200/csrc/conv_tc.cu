@@ -31,6 +31,7 @@
 #include <type_traits>
 
 #include "conv_tc.cuh"
+#include "fst_walk.cuh"
 #include "search_write.cuh"
 #include "tc_ptx.cuh"
 
@@ -3471,7 +3472,8 @@ size_t spk_fst_conv_times_workspace(int64_t b, int64_t cin, int64_t h, int64_t w
     {
         const Plan pl = make_plan(b * time, cin, h, w, cout, kh, kw, precision, true, time, true);
         if (pl.n_tiles != 1 || pl.nsplit * pl.n_tile > 512) return 0;
-        return align256(pl.wimg_bytes) + align256(pl.xt_bytes);
+        return std::max(align256(pl.wimg_bytes) + align256(pl.xt_bytes),
+                        fst_walk_workspace(b, cin, h, w, cout, kh, kw));
     }
     catch (...)
     {
@@ -3502,6 +3504,18 @@ spk_status spk_fst_conv_times(const float *t_in, int64_t b, int64_t cin, int64_t
         SPK_REQUIRE(npix < (int64_t(1) << 31), "at most 2^31 - 1 output pixels per call");
         if (b == 0) return;
         cudaStream_t s = stream_of(stream);
+        // Walking each pixel's inputs in time order costs K additions a
+        // channel against the dense kernel's T x K products; the dense kernel
+        // is left to layers whose weights fit neither shared memory nor L1.
+        const size_t walk = fst_walk_workspace(b, cin, h, w, cout, kh, kw);
+        if (walk > 0 && ws_bytes >= walk && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && oh * ow < (1 << 30))
+        {
+            fst_walk(FstWalk{t_in, kernel, t_out, b, int(cin), int(h), int(w), int(cout), int(kh), int(kw), int(sy),
+                             int(sx), int(p.top), int(p.left), int(oh), int(ow), int(time), float(threshold),
+                             precision == SPK_CONV_BF16X3 ? 3 : 2},
+                     ws, s);
+            return;
+        }
         TcParams P = prepare(pl, nullptr, kernel, b * time, cin, h, w, cout, kh, kw, sy, sx, p, oh, ow,
                              static_cast<uint8_t *>(ws), s, time, 1, t_in);
         int tp = 1, lg = 0;

@@ -21,7 +21,10 @@
 // spike, times held fixed), which `spk_fst_conv_prespike` evaluates in FP64.
 // Only first-spike times are kept between forward and backward (T times less
 // memory than the potentials); nothing here needs the potentials.
+#include <algorithm>
+
 #include "common.cuh"
+#include "fst_grad.cuh"
 
 namespace spk
 {
@@ -95,6 +98,37 @@ __global__ void fst_pool_backward_kernel(const float *__restrict__ in, const flo
                 if (bi == iy * g.w + ix) acc += gp[oy * g.ow + ox];
             }
         gi[i] = acc;
+    }
+}
+
+// The same for windows that neither overlap nor touch padding (stride =
+// window): a thread per window reads it once and writes its inputs' gradients
+// (and the zeros of inputs past the last whole window).  Bound by the bytes
+// moved; the general kernel above searches each window once per input.
+__global__ void fst_pool_backward_tiles_kernel(const float *__restrict__ in, const float *__restrict__ go,
+                                               float *__restrict__ gi, int64_t planes, Geo g)
+{
+    const int ny = (g.h + g.kh - 1) / g.kh, nx = (g.w + g.kw - 1) / g.kw;
+    const int64_t total = planes * ny * nx;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x)
+    {
+        const int64_t row = i / nx, pl = row / ny;
+        const int ox = int(i - row * nx), oy = int(row - pl * ny);
+        const int64_t corner = (pl * g.h + int64_t(oy) * g.kh) * g.w + ox * g.kw;
+        const bool whole = oy < g.oh && ox < g.ow;
+        const float v = whole ? go[(pl * g.oh + oy) * g.ow + ox] : 0.f;
+        float best = INFINITY;
+        int by = -1, bx = -1;
+        if (whole)
+            for (int dy = 0; dy < g.kh; ++dy)
+                for (int dx = 0; dx < g.kw; ++dx)
+                {
+                    const float t = in[corner + int64_t(dy) * g.w + dx];
+                    if (t < best) best = t, by = dy, bx = dx;
+                }
+        for (int dy = 0; dy < min(g.kh, g.h - oy * g.kh); ++dy)
+            for (int dx = 0; dx < min(g.kw, g.w - ox * g.kw); ++dx)
+                gi[corner + int64_t(dy) * g.w + dx] = dy == by && dx == bx ? 0.f + v : 0.f;
     }
 }
 
@@ -379,6 +413,14 @@ spk_status spk_fst_pool_backward(const float *in, int64_t b, int64_t c, int64_t 
         const Geo g = geometry(h, w, oh, ow, kernel2[0], kernel2[1], stride2, pad4);
         SPK_REQUIRE(b >= 0 && c >= 1, "invalid dims");
         if (b == 0) return;
+        if (g.sy == g.kh && g.sx == g.kw && g.top == 0 && g.left == 0 && g.oh * g.kh <= g.h && g.ow * g.kw <= g.w)
+        {
+            const int64_t windows = b * c * ceil_div(h, g.kh) * ceil_div(w, g.kw);
+            fst_pool_backward_tiles_kernel<<<grid_for(windows, 256, 16), 256, 0, stream_of(stream)>>>(in, grad_out, grad_in,
+                                                                                                  b * c, g);
+            SPK_LAUNCHED();
+            return;
+        }
         fst_pool_backward_kernel<<<grid_for(b * c * h * w, 256), 256, 0, stream_of(stream)>>>(in, grad_out, grad_in,
                                                                                                 b * c, g);
         SPK_LAUNCHED();
@@ -388,7 +430,8 @@ spk_status spk_fst_pool_backward(const float *in, int64_t b, int64_t c, int64_t 
 size_t spk_fst_conv_backward_workspace(int64_t b, int64_t cin, int64_t cout, int64_t kh, int64_t kw)
 {
     if (b <= 0 || cin <= 0 || cout <= 0 || kh <= 0 || kw <= 0) return 0;
-    return size_t(ceil_div(b, kGwSamples)) * size_t(cout) * size_t(cin * kh * kw) * sizeof(double);
+    const int64_t n = cout * cin * kh * kw;
+    return size_t(fst_grad_w_groups(b, n, ceil_div(b, kGwSamples))) * size_t(n) * sizeof(double);
 }
 
 spk_status spk_fst_conv_backward(const float *t_in, int64_t b, int64_t cin, int64_t h, int64_t w,
@@ -402,6 +445,9 @@ spk_status spk_fst_conv_backward(const float *t_in, int64_t b, int64_t cin, int6
         SPK_REQUIRE(b >= 0 && cin >= 1 && cout >= 1, "invalid dims");
         SPK_REQUIRE(cin * kh * kw < (int64_t(1) << 31) && cout < 65536, "kernel is too large");
         cudaStream_t s = stream_of(stream);
+        const Pad4 pad = pad_of(pad4);
+        const FstGrad F{t_in,      kernel,   t_out,    grad_out, b,        int(cin),  int(h),         int(w), int(cout), int(kh),
+                        int(kw),   int(oh),  int(ow),  g.sy,     g.sx,     g.top,     g.left,         int(pad.bottom),   int(pad.right)};
         if (b == 0)
         {
             if (grad_kernel) SPK_CUDA(cudaMemsetAsync(grad_kernel, 0, size_t(cout * cin * kh * kw) * 4, s));
@@ -421,21 +467,29 @@ spk_status spk_fst_conv_backward(const float *t_in, int64_t b, int64_t cin, int6
             SPK_REQUIRE(b <= 65535, "batch too large for one call (split it)");
             const dim3 grid(unsigned(ceil_div(cin, cb)), unsigned(b));
             const size_t smem = size_t(zc) * per_z * 4;
-            if (g.sy == 1 && g.sx == 1)
-                fst_conv_grad_in_kernel<true><<<grid, kGiThreads, smem, s>>>(t_in, kernel, t_out, grad_out, grad_in,
-                                                                               int(cin), int(cout), g, cb, zc);
-            else
-                fst_conv_grad_in_kernel<false><<<grid, kGiThreads, smem, s>>>(t_in, kernel, t_out, grad_out, grad_in,
-                                                                                int(cin), int(cout), g, cb, zc);
-            SPK_LAUNCHED();
+            if (!fst_grad_in(F, grad_in, s))
+            {
+                const auto k = g.sy == 1 && g.sx == 1 ? fst_conv_grad_in_kernel<true> : fst_conv_grad_in_kernel<false>;
+                k<<<grid, kGiThreads, smem, s>>>(t_in, kernel, t_out, grad_out, grad_in, int(cin), int(cout), g, cb, zc);
+                SPK_LAUNCHED();
+            }
         }
         if (grad_kernel)
         {
-            const size_t need = spk_fst_conv_backward_workspace(b, cin, cout, kh, kw);
-            SPK_REQUIRE(workspace != nullptr && workspace_bytes >= need, "workspace too small");
             const int groups = int(ceil_div(b, kGwSamples));
+            const size_t need = size_t(groups) * size_t(cout) * size_t(cin * kh * kw) * sizeof(double);
+            SPK_REQUIRE(workspace != nullptr && workspace_bytes >= need, "workspace too small");
             SPK_REQUIRE(groups <= 65535, "batch too large for one call (split it)");
             double *part = static_cast<double *>(workspace);
+            const int64_t n = cout * cin * kh * kw;
+            // as many partial sums as the workspace holds
+            const int64_t many = std::min<int64_t>(fst_grad_w_groups(b, n, groups), int64_t(workspace_bytes / (size_t(n) * 8)));
+            if (const int64_t used = fst_grad_w(F, part, many, s))
+            {
+                fst_conv_grad_w_reduce_kernel<<<grid_for(n, 256), 256, 0, s>>>(part, grad_kernel, n, int(used));
+                SPK_LAUNCHED();
+                return;
+            }
             // row slices per weight: enough pairs to fill the threads, at most one per row
             const int64_t wk = cin * kh * kw, cap = int64_t(kGwThreads) * kGwRounds;
             int slices = 1;  // a power of two
@@ -450,7 +504,6 @@ spk_status spk_fst_conv_backward(const float *t_in, int64_t b, int64_t cin, int6
             fst_conv_grad_w_kernel<<<dim3(unsigned(cout), unsigned(groups), unsigned(wblocks)), kGwThreads, smem, s>>>(
                 t_in, t_out, grad_out, part, b, int(cin), int(cout), g, kGwSamples, slices, rows, stage_in ? 1 : 0);
             SPK_LAUNCHED();
-            const int64_t n = cout * cin * kh * kw;
             fst_conv_grad_w_reduce_kernel<<<grid_for(n, 256), 256, 0, s>>>(part, grad_kernel, n, groups);
             SPK_LAUNCHED();
         }
