@@ -32,6 +32,7 @@ namespace
 constexpr int kListWarps = 8;          // warps per CTA of the warp-per-list kernels
 constexpr int64_t kMaxSparseT = 16384; // steps per sample on this path
 constexpr int kNone = 0x7f7f7f7f;      // "no event" of the atomicMin maps (memset 0x7f)
+constexpr int64_t kSmemCells = 40 * 1024;  // cells (int32) of a sample's map in shared memory
 
 __device__ __forceinline__ uint32_t ev_pack(int z, int y, int x)
 {
@@ -196,6 +197,28 @@ __global__ void min_time_map_kernel(const int64_t *__restrict__ offsets, const u
     }
 }
 
+// First event times of one sample per CTA (its map in shared memory).
+template <typename O>
+__global__ void __launch_bounds__(256)
+    gather_sample_kernel(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ events, int t, int c, int h,
+                         int w, O *__restrict__ out)
+{
+    extern __shared__ int32_t first[];
+    const int64_t u = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = c * h * w;
+    for (int i = threadIdx.x; i < n; i += 256) first[i] = t;
+    __syncthreads();
+    for (int step = warp; step < t; step += 8)
+        for (int64_t k = offsets[u * t + step] + lane; k < offsets[u * t + step + 1]; k += 32)
+        {
+            const uint32_t e = events[k];
+            const int z = ev_z(e), y = ev_y(e), x = ev_x(e);
+            if (z < c && y < h && x < w) atomicMin(&first[(z * h + y) * w + x], step);
+        }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 256) out[u * n + i] = O(first[i]);
+}
+
 template <typename O>
 __global__ void map_to_gather_kernel(const int32_t *__restrict__ map, O *__restrict__ out, int64_t n, int t)
 {
@@ -316,11 +339,115 @@ __global__ void remap_offsets_kernel(const int64_t *__restrict__ offsets, int64_
         out[i] = pos[min(offsets[i], cap)];
 }
 
+// The same filter with a sample's cells in shared memory (int32 per cell),
+// bound by the events themselves: a CTA per sample finds the cells' first
+// events, flags the events that stay (a byte each) and counts them per list;
+// after a scan of the lists' counts a warp per list moves its events.  Nothing
+// is sized by the lists' capacity: filling and scanning maps of all cells and
+// all possible events took 2.3 ms of the 4096-image event step (9.5 ms).
+constexpr int kFilterThreads = 256;
+
+template <bool POOL, typename Cell>
+__global__ void __launch_bounds__(kFilterThreads)
+    filter_sample_kernel(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ events, int64_t cap, int t,
+                         Cell cell, uint8_t *__restrict__ keep, int32_t *__restrict__ counts)
+{
+    extern __shared__ int32_t first[];
+    const int64_t u = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cells = int(cell.cells());
+    for (int i = threadIdx.x; i < cells; i += kFilterThreads) first[i] = kNone;
+    __syncthreads();
+    const int64_t begin = offsets[u * t], end = min(offsets[u * t + t], cap);
+    for (int64_t k = begin + threadIdx.x; k < end; k += kFilterThreads)
+    {
+        const int64_t q = cell.cell(events[k]);
+        if (q >= 0) atomicMin(&first[q], int32_t(k - begin));
+    }
+    __syncthreads();
+    if (!POOL)
+    {
+        // the channel of the pixel's first event
+        for (int i = threadIdx.x; i < cells; i += kFilterThreads)
+            if (first[i] != kNone) first[i] = ev_z(events[begin + first[i]]);
+        __syncthreads();
+    }
+    for (int step = warp; step < t; step += kFilterThreads / 32)
+    {
+        const int64_t b = offsets[u * t + step], e = min(offsets[u * t + step + 1], cap);
+        int n = 0;
+        for (int64_t k0 = b; k0 < e; k0 += 32)
+        {
+            const int64_t k = k0 + lane;
+            bool kept = false;
+            if (k < e)
+            {
+                const uint32_t ev = events[k];
+                const int64_t q = cell.cell(ev);
+                kept = q >= 0 && first[q] == (POOL ? int32_t(k - begin) : ev_z(ev));
+                keep[k] = kept;
+            }
+            n += __popc(__ballot_sync(0xffffffffu, kept));
+        }
+        if (lane == 0) counts[u * t + step] = n;
+    }
+}
+
+template <bool POOL, typename Cell>
+__global__ void filter_move_kernel(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ events,
+                                   int64_t lists, int64_t cap, Cell cell, const uint8_t *__restrict__ keep,
+                                   const int64_t *__restrict__ out_offsets, uint32_t *__restrict__ out)
+{
+    const int64_t list = int64_t(blockIdx.x) * kListWarps + (threadIdx.x >> 5);
+    if (list >= lists) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t b = offsets[list], e = min(offsets[list + 1], cap);
+    int64_t dst = out_offsets[list];
+    for (int64_t k0 = b; k0 < e; k0 += 32)
+    {
+        const int64_t k = k0 + lane;
+        const bool kept = k < e && keep[k];
+        const unsigned m = __ballot_sync(0xffffffffu, kept);
+        if (kept)
+        {
+            const uint32_t ev = events[k];
+            uint32_t o = ev;
+            if constexpr (POOL) o = ev_pack(ev_z(ev), cell.oy(ev), cell.ox(ev));
+            out[dst + __popc(m & ((1u << lane) - 1u))] = o;
+        }
+        dst += __popc(m);
+    }
+}
+
+size_t filter_ws(int64_t u, int64_t ncells, int64_t in_cap)
+{
+    return al(size_t(u * ncells) * 4) + al(size_t(in_cap) * 4) + al(size_t(in_cap + 1) * 8) +
+           al(scan_workspace(in_cap));
+}
+
 template <bool POOL, typename Cell>
 void filter_lists(const int64_t *offsets, const uint32_t *events, int64_t in_cap, int64_t u, int64_t t, Cell cell,
                   int64_t ncells, int64_t *out_offsets, uint32_t *out_events, Carve &ws, cudaStream_t s)
 {
     const int64_t lists = u * t;
+    // (very many empty lists need more than the workspace the callers have)
+    if (ncells <= kSmemCells && u > 0 &&
+        al(size_t(in_cap)) + al(size_t(lists) * 4) + al(scan_workspace(lists)) <= filter_ws(u, ncells, in_cap))
+    {
+        uint8_t *keep = ws.take<uint8_t>(size_t(in_cap));
+        int32_t *counts = ws.take<int32_t>(size_t(lists));
+        void *scan_ws = ws.take<char>(scan_workspace(lists));
+        const size_t smem = size_t(ncells) * 4;
+        const auto k = filter_sample_kernel<POOL, Cell>;
+        SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        k<<<unsigned(u), kFilterThreads, smem, s>>>(offsets, events, in_cap, int(t), cell, keep, counts);
+        SPK_LAUNCHED();
+        scan_exclusive<int32_t>(counts, out_offsets, lists, scan_ws, s);
+        filter_move_kernel<POOL, Cell><<<list_grid(lists), kListWarps * 32, 0, s>>>(offsets, events, lists, in_cap, cell,
+                                                                                   keep, out_offsets, out_events);
+        SPK_LAUNCHED();
+        return;
+    }
     int32_t *first = ws.take<int32_t>(size_t(u * ncells));
     int32_t *keep = ws.take<int32_t>(size_t(in_cap));
     int64_t *pos = ws.take<int64_t>(size_t(in_cap + 1));
@@ -339,12 +466,6 @@ void filter_lists(const int64_t *offsets, const uint32_t *events, int64_t in_cap
     SPK_LAUNCHED();
     remap_offsets_kernel<<<grid_for(lists + 1, 256), 256, 0, s>>>(offsets, lists, in_cap, pos, out_offsets);
     SPK_LAUNCHED();
-}
-
-size_t filter_ws(int64_t u, int64_t ncells, int64_t in_cap)
-{
-    return al(size_t(u * ncells) * 4) + al(size_t(in_cap) * 4) + al(size_t(in_cap + 1) * 8) +
-           al(scan_workspace(in_cap));
 }
 
 // ---------------------------------------------------------------------------
@@ -419,6 +540,255 @@ __global__ void sparse_conv_kernel(const int64_t *__restrict__ offsets, const ui
         if (lane == 0) counts[(s * t + step) * cout + q] = nf;
         done += nf;
     }
+}
+
+// The same with a lane per output map.  A warp takes one sample, 32 maps and a
+// band of output rows, whose potentials sit in shared memory as [neuron][map]:
+// an event costs its taps once for 32 maps (the kernel above spends a warp per
+// map on each event and scans the map's whole plane after every step; 4096
+// samples of 2 x 28 x 28 through 30 and 100 maps of 5 x 5: 4565 us),
+// conflict-free, with the weights of the band's next event (one 128-byte line
+// per tap) already on their way.  After a step only rows that an event touched
+// are compared, 8 neurons at a time.  Every neuron still sees its additions in
+// list order, and a map's neurons fire in (step, y, x) order: band after band.
+// Bound by latency (a warp's dependent accesses); bands of about 14 KB put 15
+// warps on an SM: 1934 us (whole planes of 28 x 28, two warps: 3787 us).
+//
+// Needs thr >= 0 (an untouched neuron stays below it) and rows of at most 64
+// neurons.
+constexpr int kBandBytes = 14 * 1024;
+
+// [group of 32 maps][input map and tap][32]
+__global__ void sparse_weights_kernel(const float *__restrict__ kernel, float *__restrict__ wt, int cout, int groups,
+                                      int k)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < groups * k * 32; i += gridDim.x * blockDim.x)
+    {
+        const int l = i & 31, r = (i >> 5) % k, q = (i >> 5) / k * 32 + l;
+        wt[i] = q < cout ? kernel[int64_t(q) * k + r] : 0.f;
+    }
+}
+
+struct MapsArgs
+{
+    const int64_t *offsets;
+    const uint32_t *events;
+    const float *wt;
+    uint16_t *fired;   // [u][cout][oh * ow]: band b's from its first neuron's slot on
+    uint16_t *ends;    // [u * t][bands][cout]: fired neurons of the band up to the step
+    int32_t *counts;   // [u * t]
+    int64_t tasks;
+    int t, c, cout, groups, bands, rows, top, left, oh, ow;
+    float thr;
+};
+
+template <int KH, int KW>
+__global__ void __launch_bounds__(128) sparse_conv_maps_kernel(MapsArgs A)
+{
+    extern __shared__ __align__(16) float splanes[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ow = A.ow;
+    const int64_t task = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
+    if (task >= A.tasks) return;
+    const int64_t s = task / (A.groups * A.bands);
+    const int gb = int(task - s * (A.groups * A.bands)), g = gb / A.bands, band = gb - g * A.bands;
+    const int q = g * 32 + lane, y0 = band * A.rows, ny = min(A.rows, A.oh - y0), most = ny * ow;
+    float *pot = splanes + int64_t(warp) * A.rows * ow * 32 + lane;
+    for (int i = 0; i < most; ++i) pot[i * 32] = 0.f;
+    uint64_t mask = 0;  // lane r: the touched neurons of the band's row r
+    uint16_t *slot = A.fired + (s * A.cout + q) * (int64_t(A.oh) * ow) + y0 * ow;
+    const float *wg = A.wt + int64_t(g) * A.c * KH * KW * 32 + lane;
+    int done = 0;
+
+    // an event's weights of the taps that reach the band
+    float wn[KH * KW];
+    auto fetch = [&](uint32_t ev) {
+        const float *w = wg + ev_z(ev) * (KH * KW * 32);
+        const int yb = ev_y(ev) + A.top - y0;
+#pragma unroll
+        for (int ky = 0; ky < KH; ++ky)
+            if (yb - ky >= 0 && yb - ky < ny)
+            {
+#pragma unroll
+                for (int kx = 0; kx < KW; ++kx) wn[ky * KW + kx] = __ldg(w + (ky * KW + kx) * 32);
+            }
+    };
+    const int64_t k1 = A.offsets[s * A.t + A.t];
+    int64_t k = A.offsets[s * A.t], chunk = k - 32;  // 32 events at a time, one per lane
+    uint32_t mine = 0;
+    unsigned hits = 0;  // of the chunk, the events still to come that reach the band
+    for (int step = 0; step < A.t; ++step)
+    {
+        const int64_t e = A.offsets[s * A.t + step + 1];
+        const int before = done;
+        bool any = false;
+        while (k < e)
+        {
+            if (k >= chunk + 32)
+            {
+                chunk = k;
+                mine = k + lane < k1 ? A.events[k + lane] : 0u;
+                const int yb = ev_y(mine) + A.top - y0, xx = ev_x(mine) + A.left;
+                hits = __ballot_sync(0xffffffffu, k + lane < k1 && ev_z(mine) < A.c && yb >= 0 && yb - KH + 1 < ny &&
+                                                      xx >= 0 && xx - KW + 1 < ow);
+                if (hits) fetch(__shfl_sync(0xffffffffu, mine, __ffs(hits) - 1));
+            }
+            const int64_t stop = min(e, chunk + 32);
+            const unsigned upto = stop - chunk == 32 ? 0xffffffffu : (1u << int(stop - chunk)) - 1u;
+            while (hits & upto)
+            {
+                const uint32_t ev = __shfl_sync(0xffffffffu, mine, __ffs(hits) - 1);
+                hits &= hits - 1;
+                float w[KH * KW];
+#pragma unroll
+                for (int i = 0; i < KH * KW; ++i) w[i] = wn[i];
+                if (hits) fetch(__shfl_sync(0xffffffffu, mine, __ffs(hits) - 1));
+                any = true;
+                const int yb = ev_y(ev) + A.top - y0, xx = ev_x(ev) + A.left;
+                const int xlo = max(0, xx - KW + 1), xhi = min(ow - 1, xx);
+                const uint64_t m = ((xhi == 63 ? 0ull : (1ull << (xhi + 1))) - 1ull) & ~((1ull << xlo) - 1ull);
+                if (lane <= yb && lane > yb - KH) mask |= m;
+                float *p = pot + (yb * ow + xx) * 32;
+                const bool inside = xx >= KW - 1 && xx < ow;
+#pragma unroll
+                for (int ky = 0; ky < KH; ++ky, p -= ow * 32)
+                {
+                    if (yb - ky < 0 || yb - ky >= ny) continue;
+                    if (inside)
+                    {
+                        float v[KW];
+#pragma unroll
+                        for (int kx = 0; kx < KW; ++kx) v[kx] = p[-kx * 32];
+#pragma unroll
+                        for (int kx = 0; kx < KW; ++kx) p[-kx * 32] = v[kx] + w[ky * KW + kx];
+                    }
+                    else
+                    {
+#pragma unroll
+                        for (int kx = 0; kx < KW; ++kx)
+                            if (xx - kx >= 0 && xx - kx < ow) p[-kx * 32] += w[ky * KW + kx];
+                    }
+                }
+            }
+            k = stop;
+        }
+        if (any)
+        {
+            unsigned rows = __ballot_sync(0xffffffffu, lane < ny && mask != 0);
+            while (rows)
+            {
+                const int r = __ffs(rows) - 1;
+                rows &= rows - 1;
+                uint64_t mm = __shfl_sync(0xffffffffu, mask, r);
+                while (mm)
+                {
+                    const int x0 = (__ffsll(static_cast<long long>(mm)) - 1) & ~7;
+                    mm &= ~(0xFFull << x0);
+                    float *p = pot + (r * ow + x0) * 32;
+                    unsigned hit = 0;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (x0 + j < ow && p[j * 32] > A.thr) hit |= 1u << j;
+                    while (__any_sync(0xffffffffu, hit))
+                        if (hit)
+                        {
+                            const int j = __ffs(hit) - 1;
+                            hit &= hit - 1;
+                            p[j * 32] = -FLT_MAX;
+                            // (a parked neuron fires again only if additions of
+                            // about FLT_MAX lift it back; extra events are dropped)
+                            if (done < most) slot[done++] = uint16_t((y0 + r) * ow + x0 + j);
+                        }
+                }
+            }
+            mask = 0;
+            const int n = __reduce_add_sync(0xffffffffu, done - before);
+            if (lane == 0 && n) atomicAdd(&A.counts[s * A.t + step], n);
+        }
+        if (q < A.cout) A.ends[((s * A.t + step) * A.bands + band) * A.cout + q] = uint16_t(done);
+    }
+}
+
+// The lists of the lane-per-map kernel: a warp per (sample, step) places each
+// map's runs (band after band) behind the runs of the maps before it.
+__global__ void conv_runs_kernel(const uint16_t *__restrict__ fired, const uint16_t *__restrict__ ends,
+                                 const int64_t *__restrict__ offsets, int64_t lists, int t, int cout, int bands,
+                                 int rows, int ow, int ohw, uint32_t *__restrict__ out)
+{
+    const int64_t list = int64_t(blockIdx.x) * kListWarps + (threadIdx.x >> 5);
+    if (list >= lists) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t s = list / t;
+    const int step = int(list - s * t);
+    int64_t dst = offsets[list];
+    if (offsets[list + 1] == dst) return;
+    const uint16_t *now = ends + list * bands * cout, *was = now - int64_t(bands) * cout;
+    for (int q0 = 0; q0 < cout; q0 += 32)
+    {
+        const int q = q0 + lane;
+        int n = 0;
+        if (q < cout)
+            for (int b = 0; b < bands; ++b) n += now[b * cout + q] - (step > 0 ? was[b * cout + q] : 0);
+        int x = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (n > 0)
+        {
+            const uint16_t *slot = fired + (s * cout + q) * int64_t(ohw);
+            uint32_t *o = out + dst + (x - n);
+            for (int b = 0; b < bands; ++b, slot += rows * ow)
+            {
+                const int to = now[b * cout + q];
+                for (int j = step > 0 ? was[b * cout + q] : 0; j < to; ++j)
+                {
+                    const int p = slot[j], y = p / ow;
+                    *o++ = ev_pack(q, y, p - y * ow);
+                }
+            }
+        }
+        dst += __shfl_sync(0xffffffffu, x, 31);
+    }
+}
+
+// The lane-per-map form of a whole call; false where it does not apply.
+bool conv_maps(const int64_t *offsets, const uint32_t *events, int64_t u, int t, int c, const float *kernel, int cout,
+               int kh, int kw, Pad4 p, int oh, int ow, float thr, uint16_t *fired, char *rest, size_t rest_bytes,
+               int64_t *out_offsets, uint32_t *out_events, cudaStream_t s)
+{
+    const bool k5 = kh == 5 && kw == 5, k3 = kh == 3 && kw == 3;
+    if (!(thr >= 0.f) || ow > 64 || !(k5 || k3) || p.top > 65535 || p.left > 65535) return false;
+    // bands of equal height; at most 32 rows (a lane per row)
+    int bands = std::max(1, oh * ow * 128 / kBandBytes);
+    int rows = (oh + bands - 1) / bands;
+    if (rows > 32) rows = 32;
+    bands = (oh + rows - 1) / rows;
+    const int groups = (cout + 31) / 32, k = c * kh * kw;
+    const int64_t lists = u * t, tasks = u * groups * bands;
+    Carve cv{rest};
+    float *wt = cv.take<float>(size_t(k) * groups * 32);
+    uint16_t *ends = cv.take<uint16_t>(size_t(lists) * bands * cout);
+    int32_t *counts = cv.take<int32_t>(size_t(lists));
+    void *scan_ws = cv.take<char>(scan_workspace(lists));
+    if (cv.used > rest_bytes || ceil_div(tasks, 4) > 0x7FFFFFFF) return false;
+    sparse_weights_kernel<<<grid_for(int64_t(k) * groups * 32, 256), 256, 0, s>>>(kernel, wt, cout, groups, k);
+    SPK_LAUNCHED();
+    SPK_CUDA(cudaMemsetAsync(counts, 0, size_t(lists) * 4, s));
+    const int64_t plane = int64_t(rows) * ow * 128;
+    const int wpc = plane * 4 <= 100 * 1024 ? 4 : 1;
+    const MapsArgs A{offsets, events, wt,     fired, ends,       counts,      tasks, t, c, cout,
+                     groups,  bands,  rows,   int(p.top), int(p.left), oh,    ow,    thr};
+    const auto kern = k5 ? sparse_conv_maps_kernel<5, 5> : sparse_conv_maps_kernel<3, 3>;
+    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wpc * plane)));
+    kern<<<unsigned(ceil_div(tasks, wpc)), wpc * 32, size_t(wpc * plane), s>>>(A);
+    SPK_LAUNCHED();
+    scan_exclusive<int32_t>(counts, out_offsets, lists, scan_ws, s);
+    conv_runs_kernel<<<list_grid(lists), kListWarps * 32, 0, s>>>(fired, ends, out_offsets, lists, t, cout, bands, rows,
+                                                                 ow, oh * ow, out_events);
+    SPK_LAUNCHED();
+    return true;
 }
 
 // Output lists: per (sample, step) the fired neurons map after map.
@@ -561,6 +931,45 @@ __global__ void sparse_prepost_kernel(const int32_t *__restrict__ last, int t, i
     if (threadIdx.x == 0) post[s * count + j] = uint16_t(e[1] < 0 ? 0 : (e[1] > 65535 ? 65535 : e[1]));
 }
 
+// The two kernels above for one sample per CTA, its map of last steps in
+// shared memory (no map of the batch to clear and update by global atomics).
+__global__ void __launch_bounds__(256)
+    sparse_prepost_sample_kernel(const int64_t *__restrict__ offsets, const uint32_t *__restrict__ events, int t, int c,
+                                 int hp, int wp, int top, int left, int kh, int kw, const int32_t *__restrict__ winners,
+                                 const int32_t *__restrict__ counts, int count, uint16_t *__restrict__ pre,
+                                 uint16_t *__restrict__ post)
+{
+    extern __shared__ int32_t last[];  // [c][hp][wp]
+    const int64_t u = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = min(counts[u], count);
+    if (n <= 0) return;
+    for (int i = threadIdx.x; i < c * hp * wp; i += 256) last[i] = 0;
+    __syncthreads();
+    for (int step = warp; step < t; step += 8)
+        for (int64_t k = offsets[u * t + step] + lane; k < offsets[u * t + step + 1]; k += 32)
+        {
+            const uint32_t e = events[k];
+            const int z = ev_z(e), y = ev_y(e) + top, x = ev_x(e) + left;
+            if (z < c && y < hp && x < wp) atomicMax(&last[(z * hp + y) * wp + x], step + 1);
+        }
+    __syncthreads();
+    const int taps = kh * kw, k = c * taps;
+    for (int j = 0; j < n; ++j)
+    {
+        const int32_t *e = winners + (u * count + j) * 5;
+        const int wy = e[3], wx = e[4];
+        uint16_t *p = pre + (u * count + j) * int64_t(k);
+        for (int i = threadIdx.x; i < k; i += 256)
+        {
+            const int z = i / taps, r = i - z * taps, ky = r / kw, y = wy + ky, x = wx + r - ky * kw;
+            int v = 0;
+            if (y >= 0 && y < hp && x >= 0 && x < wp) v = last[(z * hp + y) * wp + x];
+            p[i] = uint16_t(v == 0 ? t : v - 1);
+        }
+        if (threadIdx.x == 0) post[u * count + j] = uint16_t(e[1] < 0 ? 0 : (e[1] > 65535 ? 65535 : e[1]));
+    }
+}
+
 void check_shape(int64_t u, int64_t t, int64_t c, int64_t h, int64_t w)
 {
     SPK_REQUIRE(u >= 0 && t >= 1 && c >= 1 && h >= 1 && w >= 1, "invalid dims");
@@ -673,6 +1082,17 @@ spk_status spk_sparse_gather(const int64_t *offsets, const uint32_t *events, int
         SPK_REQUIRE(ws && ws_bytes >= spk_sparse_dense_workspace(u, c, h, w), "workspace is too small");
         if (u == 0) return;
         cudaStream_t s = stream_of(stream);
+        if (c * h * w <= kSmemCells)
+        {
+            const size_t smem = size_t(c * h * w) * 4;
+            dispatch(otype, [&](auto z) {
+                const auto k = gather_sample_kernel<decltype(z)>;
+                SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+                k<<<unsigned(u), 256, smem, s>>>(offsets, events, int(t), int(c), int(h), int(w), (decltype(z) *)out);
+                SPK_LAUNCHED();
+            });
+            return;
+        }
         int32_t *map = static_cast<int32_t *>(ws);
         min_map(offsets, events, u, t, c, h, w, map, s);
         dispatch(otype, [&](auto z) {
@@ -817,6 +1237,12 @@ spk_status spk_sparse_conv(const int64_t *offsets, const uint32_t *events, int64
         float *planes = cv.take<float>(size_t(maps * ohw));
         const size_t plane_bytes = size_t(ohw) * 4;
         const float thr = float(threshold);
+        // (the lane-per-map form takes the bytes of the other's counts,
+        // starts and planes)
+        if (conv_maps(offsets, events, u, int(t), int(c), kernel, int(cout), int(kh), int(kw), p, int(oh), int(ow), thr,
+                      fired, reinterpret_cast<char *>(counts), cv.used - al(size_t(maps * ohw) * 2), out_offsets,
+                      out_events, s))
+            return;
         if (plane_bytes <= 24 * 1024)
         {
             const int wpc = int(std::max<size_t>(1, std::min<size_t>(8, (48 * 1024) / plane_bytes)));
@@ -882,6 +1308,19 @@ spk_status spk_sparse_stdp(const int64_t *offsets, const uint32_t *events, int64
         int32_t *last = cv.take<int32_t>(size_t(u * c * hp * wp));
         uint16_t *pre = cv.take<uint16_t>(size_t(u * count * k));
         uint16_t *post = cv.take<uint16_t>(size_t(u * count));
+        if (c * hp * wp <= kSmemCells)
+        {
+            const size_t smem = size_t(c * hp * wp) * 4;
+            SPK_CUDA(cudaFuncSetAttribute(sparse_prepost_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          int(smem)));
+            sparse_prepost_sample_kernel<<<unsigned(u), 256, smem, s>>>(offsets, events, int(t), int(c), int(hp),
+                                                                        int(wp), int(p.top), int(p.left), int(kh),
+                                                                        int(kw), winners, counts, int(count), pre, post);
+            SPK_LAUNCHED();
+            launch_stdp_scan(kernel, k, cout, u, count, 2, winners, counts, pre, count * k, k, post, configs_host, nconf,
+                             true, s);
+            return;
+        }
         SPK_CUDA(cudaMemsetAsync(last, 0, size_t(u * c * hp * wp) * 4, s));
         last_time_map_kernel<<<list_grid(u * t), kListWarps * 32, 0, s>>>(offsets, events, u * t, int(t), int(c),
                                                                           int(hp), int(wp), int(p.top), int(p.left),
