@@ -186,23 +186,26 @@ __global__ void __launch_bounds__(kCodeThreads) rank_sorted_kernel(const I *__re
         write_rows<O>(out + int64_t(blockIdx.x) * t * x, tm, x, t);
 }
 
-// Rows of 257 .. 2048 values with 256 threads.  Only the values above the
+// Rows of 257 .. 8192 values with 256, 512 or 1024 threads (8 values a
+// thread).  Only the values above the
 // row minimum are sorted: they are compacted in index order into shared
 // memory (a value equal to the minimum at index i has rank cnt + the number
 // of minimum values before it, known from the same prefix count), then
-// sorted by a bitonic network on N = 512, 1024 or 2048 keys (the next power
-// of two, at least 512) whose keys stay in registers: thread i holds
-// positions ITEMS i .. ITEMS i + ITEMS - 1 (ITEMS = N / 256), a stage of
+// sorted by a bitonic network on N = 2, 4 or 8 keys a thread (the least that
+// holds them) whose keys stay in registers: thread i holds
+// positions ITEMS i .. ITEMS i + ITEMS - 1 (ITEMS = N / threads), a stage of
 // stride < ITEMS is a compare-exchange inside the thread, strides up to
 // 32 ITEMS / 2 a shuffle with the thread owning the partner positions, and
 // only larger strides go through shared memory.  With many values tied at
 // the minimum (zero filter responses) the sort is a fraction of the row.
-constexpr int kRegThreads = 256, kRegMax = 8 * kRegThreads;
+// (Rows of 2178 values, 333 images: 109 us with all keys sorted in shared
+// memory, XXX here; 4704 values, 200 images: 150 and XXX us.)
+constexpr int kRegItems = 8, kRegMax = 1024 * kRegItems;
 
-template <int ITEMS>
+template <int ITEMS, int THREADS>
 __device__ __forceinline__ void bitonic_block(uint64_t *keys)
 {
-    constexpr int N = kRegThreads * ITEMS;
+    constexpr int N = THREADS * ITEMS;
     const int tid = threadIdx.x, e0 = ITEMS * tid;
     uint64_t k[ITEMS];
 #pragma unroll
@@ -218,7 +221,7 @@ __device__ __forceinline__ void bitonic_block(uint64_t *keys)
             __syncthreads();
             for (; stride >= 32 * ITEMS; stride >>= 1)
             {
-                for (int q = tid; q < N / 2; q += kRegThreads)
+                for (int q = tid; q < N / 2; q += THREADS)
                 {
                     const int lo = 2 * q - (q & (stride - 1)), hi = lo + stride;
                     const bool up = (lo & size) == 0;
@@ -262,14 +265,15 @@ __device__ __forceinline__ void bitonic_block(uint64_t *keys)
     __syncthreads();
 }
 
-template <typename I, typename O, bool TIMES>
-__global__ void __launch_bounds__(kRegThreads) rank_compact_kernel(const I *__restrict__ in, O *__restrict__ out,
-                                                                   int64_t x, int t)
+template <typename I, typename O, bool TIMES, int THREADS>
+__global__ void __launch_bounds__(THREADS) rank_compact_kernel(const I *__restrict__ in, O *__restrict__ out,
+                                                               int64_t x, int t)
 {
-    constexpr int IT = kRegMax / kRegThreads;  // values per thread on load
-    __shared__ uint64_t keys[kRegMax];
-    __shared__ __align__(16) uint16_t tm[kRegMax];
-    __shared__ uint32_t s_warp[kRegThreads / 32], s_min, s_off[kRegThreads / 32];
+    constexpr int IT = kRegItems, MAX = THREADS * IT;  // values per thread on load
+    extern __shared__ __align__(16) unsigned char rc_smem[];
+    uint64_t *keys = reinterpret_cast<uint64_t *>(rc_smem);   // [MAX]
+    uint16_t *tm = reinterpret_cast<uint16_t *>(keys + MAX);  // [MAX]
+    __shared__ uint32_t s_warp[THREADS / 32], s_min, s_off[THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, e0 = IT * tid;
     const I *row = in + int64_t(blockIdx.x) * x;
     uint32_t kv[IT];
@@ -286,7 +290,7 @@ __global__ void __launch_bounds__(kRegThreads) rank_compact_kernel(const I *__re
     if (tid == 0)
     {
         uint32_t m = s_warp[0];
-        for (int w = 1; w < kRegThreads / 32; ++w) m = min(m, s_warp[w]);
+        for (int w = 1; w < THREADS / 32; ++w) m = min(m, s_warp[w]);
         s_min = m;
     }
     __syncthreads();
@@ -306,7 +310,7 @@ __global__ void __launch_bounds__(kRegThreads) rank_compact_kernel(const I *__re
     if (tid == 0)
     {
         uint32_t run = 0;
-        for (int w = 0; w < kRegThreads / 32; ++w) s_off[w] = run, run += s_warp[w];
+        for (int w = 0; w < THREADS / 32; ++w) s_off[w] = run, run += s_warp[w];
         s_min = run;  // cnt
     }
     __syncthreads();
@@ -325,21 +329,21 @@ __global__ void __launch_bounds__(kRegThreads) rank_compact_kernel(const I *__re
                 tm[i] = f2u16(float(cnt + i - kp) * scale);  // rank among the ties at the minimum
         }
     }
-    int n = 512;
+    int n = 2 * THREADS;
     while (n < cnt) n <<= 1;
-    for (int i = cnt + tid; i < n; i += kRegThreads) keys[i] = ~uint64_t(0);
+    for (int i = cnt + tid; i < n; i += THREADS) keys[i] = ~uint64_t(0);
     __syncthreads();
-    if (n == 512)
-        bitonic_block<2>(keys);
-    else if (n == 1024)
-        bitonic_block<4>(keys);
+    if (n == 2 * THREADS)
+        bitonic_block<2, THREADS>(keys);
+    else if (n == 4 * THREADS)
+        bitonic_block<4, THREADS>(keys);
     else
-        bitonic_block<8>(keys);
-    for (int i = tid; i < cnt; i += kRegThreads) tm[uint32_t(keys[i])] = f2u16(float(i) * scale);
+        bitonic_block<8, THREADS>(keys);
+    for (int i = tid; i < cnt; i += THREADS) tm[uint32_t(keys[i])] = f2u16(float(i) * scale);
     __syncthreads();
     if constexpr (TIMES)
     {
-        for (int64_t j = tid; j < x; j += kRegThreads) out[int64_t(blockIdx.x) * x + j] = O(tm[j]);
+        for (int64_t j = tid; j < x; j += THREADS) out[int64_t(blockIdx.x) * x + j] = O(tm[j]);
     }
     else
     {
@@ -348,7 +352,7 @@ __global__ void __launch_bounds__(kRegThreads) rank_compact_kernel(const I *__re
         {
             // (row, 16-position vector) pairs over the block
             const int nv = int(x / 16);
-            for (int q = tid; q < t * nv; q += kRegThreads)
+            for (int q = tid; q < t * nv; q += THREADS)
             {
                 const int srow = q / nv, v = q - srow * nv;
                 const uint4 ta = *reinterpret_cast<const uint4 *>(tm + 16 * v);
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(kRegThreads) rank_compact_kernel(const I *__re
             }
         }
         else
-            for (int64_t j = tid; j < x; j += kRegThreads)
+            for (int64_t j = tid; j < x; j += THREADS)
             {
                 const uint16_t m = tm[j];
                 for (int srow = 0; srow < t; ++srow) o[int64_t(srow) * x + j] = O(m <= uint16_t(srow));
@@ -602,14 +606,21 @@ uint16_t *large_times_slot(void *ws, int64_t b, int64_t x)
 // Bytes of scratch the sorted code needs (0 when X <= 16384).
 size_t rank_times_ws(int64_t b, int64_t x, int sort) { return (sort && x > kMaxSortX) ? large_sort_ws(b, x) : 0; }
 
-// The compacting kernel for rows of 257 .. 2048 values (false: not taken).
+// The compacting kernel for rows of 257 .. 8192 values (false: not taken).
 template <typename I, typename O, bool TIMES>
 bool rank_reg(const I *in, O *out, int64_t b, int64_t t, int64_t x, cudaStream_t s)
 {
     if (x <= 256 || x > kRegMax || b > 0x7FFFFFFF) return false;
-    rank_compact_kernel<I, O, TIMES><<<unsigned(b), kRegThreads, 0, s>>>(in, out, x, int(t));
-    SPK_LAUNCHED();
-    return true;
+    auto go = [&](auto k, int threads) {
+        const int smem = threads * kRegItems * 10;
+        SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        k<<<unsigned(b), threads, smem, s>>>(in, out, x, int(t));
+        SPK_LAUNCHED();
+        return true;
+    };
+    if (x <= 256 * kRegItems) return go(rank_compact_kernel<I, O, TIMES, 256>, 256);
+    if (x <= 512 * kRegItems) return go(rank_compact_kernel<I, O, TIMES, 512>, 512);
+    return go(rank_compact_kernel<I, O, TIMES, 1024>, 1024);
 }
 
 // First-spike times [B, X] u16 of the rank-order (sort) or latency code.

@@ -391,6 +391,56 @@ __device__ __forceinline__ void tmem_chunk_wait(uint32_t (&q)[3][kEpiChunk])
     if (NS == 3) tmem_ld_wait8(q[2]);
 }
 
+// h + m + l rounded once to F32.  Two terms: one FP32 addition.  Three: exact
+// sums of value and error (Knuth's two-sum) leave s2 + (e2 + e1), so the last
+// addition rounds the exact total whenever e2 + e1 is exact, and the FP64 sum
+// takes the rest (also infinities and NaN, whose error terms are NaN).  FP64
+// conversions of every term and sum cost the potentials' epilogue about 3000
+// cycles per 16 columns.
+template <int NS>
+__device__ __forceinline__ float sum_terms(float h, float m, float l)
+{
+    if (NS == 2) return __fadd_rn(h, m);
+    auto two_sum = [](float a, float b, float &e) {
+        const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+        e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+        return s;
+    };
+    float e1, e2, e3;
+    const float s1 = two_sum(m, l, e1), s2 = two_sum(h, s1, e2), t = two_sum(e2, e1, e3);
+    float r = __fadd_rn(s2, t);
+    if (!(e3 == 0.f)) r = float(double(h) + double(m) + double(l));
+    return r;
+}
+
+// Potentials of one row and N tile: the accumulators in chunks of 8 columns,
+// the next chunk on its way while one is summed and stored.
+template <int NS>
+__device__ __forceinline__ void potentials_epilogue(const TcParams &P, uint32_t lane_base, bool ok, float *out, int n)
+{
+    uint32_t qa[3][kEpiChunk], qb[3][kEpiChunk];
+    auto put = [&](const uint32_t(&q)[3][kEpiChunk], int c0) {
+        float *o = out + int64_t(c0) * P.ohw;
+#pragma unroll
+        for (int j = 0; j < kEpiChunk; ++j, o += P.ohw)
+        {
+            const float v = sum_terms<NS>(__uint_as_float(q[0][j]), __uint_as_float(q[1][j]),
+                                          NS == 3 ? __uint_as_float(q[2][j]) : 0.f);
+            if (ok && c0 + j < n) *o = v;
+        }
+    };
+    tmem_chunk<NS>(lane_base, 0, P.n_tile, qa);
+    for (int c0 = 0; c0 < P.n_tile; c0 += 2 * kEpiChunk)  // n_tile is a multiple of 16
+    {
+        tmem_chunk_wait<NS>(qa);
+        tmem_chunk<NS>(lane_base, c0 + kEpiChunk, P.n_tile, qb);
+        put(qa, c0);
+        tmem_chunk_wait<NS>(qb);
+        if (c0 + 2 * kEpiChunk < P.n_tile) tmem_chunk<NS>(lane_base, c0 + 2 * kEpiChunk, P.n_tile, qa);
+        put(qb, c0 + kEpiChunk);
+    }
+}
+
 // One chunk of columns: f = (h + m) + l in FP32, the largest above-threshold
 // value (first index on ties) and the runner-up, the first below-threshold
 // channel, the largest |h| + |m| + |l| and the closest distance to the
@@ -1875,20 +1925,12 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
             if constexpr (MODE == kPotentials)
             {
                 const uint32_t lane_base = acc + (uint32_t((warp & 3) * 32) << 16);
-                for (int c0 = 0; c0 < P.n_tile; c0 += 16)
-                {
-                    float v[16];
-                    load_exact16(lane_base, c0, P.n_tile, P.nsplit, v);
-                    if (r.ok)
-                    {
-#pragma unroll
-                        for (int q = 0; q < 16; ++q)
-                        {
-                            const int n = nt * P.n_tile + c0 + q;
-                            if (n < P.cout) P.out[(r.img * P.cout + n) * P.ohw + r.pix] = v[q];
-                        }
-                    }
-                }
+                float *out = P.out + (r.img * P.cout + nt * P.n_tile) * P.ohw + r.pix;
+                const int n = P.cout - nt * P.n_tile;
+                if (P.nsplit == 3)
+                    potentials_epilogue<3>(P, lane_base, r.ok, out, n);
+                else
+                    potentials_epilogue<2>(P, lane_base, r.ok, out, n);
             }
             if constexpr (MODE == kTimes)
             {
@@ -3117,10 +3159,27 @@ FusedLayout fused_layout(int64_t b, int64_t t, int64_t cin, int64_t h, int64_t w
 }
 }  // namespace
 
+// The plan of the potentials kernel.  From 2 input channels on the spikes are
+// first copied channels-last (one 8-byte load per tap and 8 channels instead
+// of a byte per element: 6 channels of 28 x 28, 996 -> XXX us), where the
+// padded K and the workspace allow it.
+static Plan potentials_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh, int64_t kw,
+                            int precision, size_t ws_bytes)
+{
+    if (cin >= 2 && cin < 8)
+    {
+        const Plan pl = make_plan(n, cin, h, w, cout, kh, kw, precision, false, 0, false, 0, true);
+        if (pl.kblocks <= kMaxKBlocks && pl.stages >= 2 && pl.smem <= 227 * 1024 &&
+            ws_bytes >= align256(pl.wimg_bytes) + align256(pl.xt_bytes))
+            return pl;
+    }
+    return make_plan(n, cin, h, w, cout, kh, kw, precision, false);
+}
+
 size_t conv_tc_workspace(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh, int64_t kw,
                          int precision)
 {
-    Plan pl = make_plan(n, cin, h, w, cout, kh, kw, precision, false);
+    const Plan pl = potentials_plan(n, cin, h, w, cout, kh, kw, precision, SIZE_MAX);
     return align256(pl.wimg_bytes) + align256(pl.xt_bytes);
 }
 
@@ -3129,7 +3188,7 @@ void conv_tc(const void *in, spk_dtype itype, const float *kernel, float *out, i
              int precision, void *ws, size_t ws_bytes, cudaStream_t s)
 {
     if (itype != SPK_U8) throw Error(SPK_ERR_UNSUPPORTED, "the tensor-core path takes U8 spikes");
-    Plan pl = make_plan(n, cin, h, w, cout, kh, kw, precision, false);
+    const Plan pl = potentials_plan(n, cin, h, w, cout, kh, kw, precision, ws_bytes);
     SPK_REQUIRE(ws != nullptr && ws_bytes >= align256(pl.wimg_bytes) + align256(pl.xt_bytes), "workspace is too small");
     TcParams P = prepare(pl, in, kernel, n, cin, h, w, cout, kh, kw, sy, sx, p, oh, ow, static_cast<uint8_t *>(ws), s);
     P.out = out;

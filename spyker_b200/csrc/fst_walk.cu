@@ -257,6 +257,69 @@ __global__ void __launch_bounds__(max_warps(NG) * 32) fst_walk_kernel(WalkArgs A
     }
 }
 
+// Layers with few output pixels (fc layers: one per sample) leave most SMs with
+// a single warp in the walk.  Here a CTA takes one pixel and kStepMaps maps: its
+// warps add their slices of the weights into per-step sums (shared memory,
+// every warp its own, so the order is fixed), which are then run through in
+// step order.  All K additions are made, by kStepWarps times the warps.
+constexpr int kStepWarps = 16, kStepMaps = 32;
+
+__global__ void __launch_bounds__(kStepWarps * 32) fst_steps_kernel(WalkArgs A)
+{
+    extern __shared__ __align__(16) unsigned char sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int64_t pix = blockIdx.x;
+    const int z0 = blockIdx.y * kStepMaps, nz = min(kStepMaps, A.cout - z0), T = A.time;
+    double *sums = reinterpret_cast<double *>(sm);  // [warps][T][nz]
+    for (int i = threadIdx.x; i < nw * T * nz; i += blockDim.x) sums[i] = 0.0;
+    __syncthreads();
+    const int64_t smp = pix / A.P;
+    const int q = int(pix - smp * A.P), oy = q / A.ow, ox = q - oy * A.ow;
+    const int iy0 = oy * A.sy - A.top, ix0 = ox * A.sx - A.left, KK = A.kh * A.kw;
+    const uint8_t *src = A.map + smp * (int64_t(A.cin) * A.h * A.w) + iy0 * A.w + ix0;
+    double *mine = sums + warp * T * nz;
+    // 32 inputs' times at a time, one per lane; then each input's weights,
+    // one map per lane, 8 inputs in flight
+    for (int k0 = warp * 32; k0 < A.K; k0 += nw * 32)
+    {
+        const int k = k0 + lane;
+        int t = T;
+        if (k < A.K)
+        {
+            const int c = k / KK, r = k - c * KK, ky = r / A.kw, kx = r - ky * A.kw;
+            const unsigned iy = unsigned(iy0 + ky), ix = unsigned(ix0 + kx);
+            if (iy < unsigned(A.h) && ix < unsigned(A.w)) t = __ldg(src + (c * A.h + ky) * A.w + kx);
+        }
+        unsigned on = __ballot_sync(0xffffffffu, t < T);
+        while (on)
+        {
+            double w[8];
+            int ts[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+            {
+                const int l = on ? __ffs(on) - 1 : 0;
+                ts[u] = on ? __shfl_sync(0xffffffffu, t, l) : T;
+                w[u] = on && lane < nz ? __ldg(A.wt + int64_t(k0 + l) * A.cout + z0 + lane) : 0.0;
+                on &= on - 1;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (ts[u] < T && lane < nz) mine[ts[u] * nz + lane] += w[u];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x >= nz) return;
+    double v = 0.0;
+    int at = T;
+    for (int t = 0; t < T && at == T; ++t)
+    {
+        for (int w = 0; w < nw; ++w) v += sums[(w * T + t) * nz + threadIdx.x];
+        if (v > A.bound) at = t;
+    }
+    A.t_out[(smp * A.cout + z0 + threadIdx.x) * A.P + q] = float(at);
+}
+
 // F32(v) > thr, as v > bound: the midpoint between thr and the next float,
 // which itself rounds to the even of the two.
 double rounding_bound(float thr)
@@ -320,6 +383,17 @@ void fst_walk(const FstWalk &F, void *ws, cudaStream_t s)
     WalkArgs A{map,  wt,     F.t_out, npix,   F.cin, F.h,           F.w,    F.cout, F.kh,    F.kw,
                F.sy, F.sx,   F.top,   F.left, F.ow,  F.oh * F.ow,   F.time, K,      pl.tile, pl.smem_weights,
                rounding_bound(F.threshold)};
+    // at most four pixels per SM: per-step sums by all warps of a CTA
+    if (npix <= 4 * sm_count() && K >= 256 && ceil_div(F.cout, kStepMaps) <= 65535)
+    {
+        const int nz = std::min(F.cout, kStepMaps);
+        const int warps = int(std::min<int64_t>(kStepWarps, std::min<int64_t>(ceil_div(K, 32), 160 * 1024 / (F.time * nz * 8))));
+        const size_t smem = size_t(warps) * F.time * nz * 8;
+        SPK_CUDA(cudaFuncSetAttribute(fst_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        fst_steps_kernel<<<dim3(unsigned(npix), unsigned(ceil_div(F.cout, kStepMaps))), warps * 32, smem, s>>>(A);
+        SPK_LAUNCHED();
+        return;
+    }
     const auto k = pl.ng == 1 ? fst_walk_kernel<1> : pl.ng == 2 ? fst_walk_kernel<2> : fst_walk_kernel<4>;
     SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.smem)));
     int occ = 0;

@@ -761,7 +761,7 @@ bool conv_maps(const int64_t *offsets, const uint32_t *events, int64_t u, int t,
     const bool k5 = kh == 5 && kw == 5, k3 = kh == 3 && kw == 3;
     if (!(thr >= 0.f) || ow > 64 || !(k5 || k3) || p.top > 65535 || p.left > 65535) return false;
     // bands of equal height; at most 32 rows (a lane per row)
-    int bands = std::max(1, oh * ow * 128 / kBandBytes);
+    int bands = (oh * ow * 128 + kBandBytes - 1) / kBandBytes;
     int rows = (oh + bands - 1) / bands;
     if (rows > 32) rows = 32;
     bands = (oh + rows - 1) / rows;
