@@ -32,6 +32,7 @@
 
 #include "conv_tc.cuh"
 #include "fst_walk.cuh"
+#include "rounding.cuh"
 #include "search_write.cuh"
 #include "tc_ptx.cuh"
 
@@ -2047,6 +2048,7 @@ __global__ void wta_records_kernel(const int4 *__restrict__ records, const unsig
         ++found;
     }
     if (threadIdx.x == 0) counts[b] = found;
+    for (int i = found * 5 + threadIdx.x; i < count * 5; i += blockDim.x) winners[b * count * 5 + i] = 0;
 }
 
 // The same selection with one warp per sample for maps of up to 32 * KPL
@@ -2128,6 +2130,7 @@ __global__ void __launch_bounds__(128) wta_records_warp_kernel(const int4 *__res
         ++found;
     }
     if (lane == 0) counts[b] = found;
+    for (int i = found * 5 + lane; i < count * 5; i += 32) winners[b * count * 5 + i] = 0;
 }
 
 // ---- search path: weight split, exact recompute, outputs ---------------------
@@ -2695,6 +2698,8 @@ __global__ void __launch_bounds__(128) search_fix_kernel(TcParams P, const float
     }
 }
 
+#include "search_walk.cuh"
+
 inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
 // Schedule overrides of the tensor-core kernels (0 = automatic), set by an
@@ -2984,7 +2989,7 @@ TcParams prepare(const Plan &pl, const void *in, const float *kernel, int64_t n,
         const int64_t cp = pl.nhwc ? pl.cpad : cin;
         negw = reinterpret_cast<int *>(ws + size_t(nnets) * align256(pl.wimg_bytes) +
                                        align256(size_t(n / t_fused) * h * w * cp) + 128);
-        SPK_CUDA(cudaMemsetAsync(negw, 0, sizeof(int), s));
+        SPK_CUDA(cudaMemsetAsync(negw - 32, 0, 256, s));  // the flag, this word and the search's largest weight
     }
     const dim3 sgrid(grid_for(wthreads, 256), unsigned(nnets));
     split_weights_kernel<<<sgrid, 256, 0, s>>>(kernel, reinterpret_cast<uint4 *>(wimg), int(cout), int(cin),
@@ -3000,7 +3005,6 @@ TcParams prepare(const Plan &pl, const void *in, const float *kernel, int64_t n,
     {
         const int64_t b = n / t_fused, cp = pl.nhwc ? pl.cpad : cin;
         int *flag = reinterpret_cast<int *>(xt + align256(size_t(b) * h * w * cp));
-        SPK_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
         if (times)
         {
             times_fst_kernel<<<grid_for(b * h * w * cp, 256), 256, 0, s>>>(times, xt, b, int(cin), h * w, int(cp),
@@ -3161,7 +3165,8 @@ FusedLayout fused_layout(int64_t b, int64_t t, int64_t cin, int64_t h, int64_t w
 
 // The plan of the potentials kernel.  From 2 input channels on the spikes are
 // first copied channels-last (one 8-byte load per tap and 8 channels instead
-// of a byte per element: 6 channels of 28 x 28, 996 -> XXX us), where the
+// of a byte per element: the three layers of the reward-modulated network on 200 images 2432 ->
+// 1757 us with the FP32 epilogue), where the
 // padded K and the workspace allow it.
 static Plan potentials_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh, int64_t kw,
                             int precision, size_t ws_bytes)
@@ -3283,6 +3288,17 @@ struct Nets
 // device (each launch reads them).  Off the search path (device flags) every
 // one of these kernels leaves at once, except the writer, which zero-fills
 // the spikes for the dense kernel.
+// Up to how many output pixels the walk (search_walk.cuh) is the faster
+// search: its time grows with the pixels from a few microseconds, the rounds
+// start near 100 us (some 20 dependent launches) and then spend less per
+// pixel.  2 -> 30 channels 5 x 5: 50k pixels 60 against 140 us, 363k 340
+// against 230; 30 -> 100 channels: 0.2k 17 against 120, 85k 515 against 233.
+bool walk_pays(int64_t npix, int groups, int cout)
+{
+    const bool small = groups <= 32 && cout <= 32;  // one load and one channel per lane
+    return npix <= (small ? 128 * 1024 : 20 * 1024);
+}
+
 void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel, int64_t count, int64_t pool_ky,
                   int64_t pool_kx, int64_t poh, int64_t pow_, uint8_t *spikes, uint8_t *pooled, uint8_t *base,
                   cudaStream_t s)
@@ -3311,6 +3327,34 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
     const int taps = P.kh * P.kw;
     P.kreal = P.nhwc ? taps * P.cpad : taps * P.cin;
     P.tiles = ceil_div(L.npix, BM);
+    // (the bisection state's bytes hold the writer's codes)
+    auto write = [&] {
+        search_write(SearchWrite{P.records, reinterpret_cast<uint8_t *>(P.state), P.negw, P.flag, spikes,
+                                 pool_ky > 0 ? pooled : nullptr, b, P.T, P.cout, int(L.oh), int(L.ow), int(pool_ky),
+                                 int(pool_kx), int(poh), int(pow_)},
+                     s);
+    };
+    // Walking each pixel's inputs in spike order (search_walk.cuh) instead of
+    // the rounds below.
+    const int groups = taps * (P.cpad / 8);
+    if (P.nhwc && P.T <= 32 && groups <= 256 && P.cout <= 256 && walk_pays(L.npix, groups, P.cout))
+    {
+        // (the integers take the digit image's bytes: 128 rows per K block,
+        // four bytes per channel and row)
+        uint32_t *wd = reinterpret_cast<uint32_t *>(base + L.w4_off);
+        unsigned *wtop = reinterpret_cast<unsigned *>(P.negw - 16);
+        walk_split_kernel<<<unsigned(nch), 256, 0, s>>>(kernel, wd, P.cout, P.cin, taps, P.cpad, nch, echan, cscale,
+                                                        P.negw, wtop);
+        SPK_LAUNCHED();
+        if (count > 0)
+        {
+            search_init_kernel<<<grid_for(b, 256), 256, 0, s>>>(P.mins, P.maxs, b, P.negw, P.flag);
+            SPK_LAUNCHED();
+        }
+        launch_search_walk(P, WalkSearch{wd, kernel, wtop, nch, groups, rounding_bound(P.thr)}, s);
+        write();
+        return;
+    }
     // the bound pre-filter of round 0, for layers with few inputs per output
     const int cp = P.nhwc ? P.cpad : P.cin;
     const int kr = P.cin * taps;
@@ -3395,11 +3439,7 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
         // the next bisection round's list (round 0 without a list: all pixels)
         if (r < nsr) compact(r == 0 && !prefilter ? nullptr : P.count_in, r & 1 ? lb : la, cnt + r + 1);
     }
-    // (the bisection state is no longer needed: its bytes hold the writer's codes)
-    search_write(SearchWrite{P.records, reinterpret_cast<uint8_t *>(P.state), P.negw, P.flag, spikes,
-                             pool_ky > 0 ? pooled : nullptr, b, P.T, P.cout, int(L.oh), int(L.ow), int(pool_ky),
-                             int(pool_kx), int(poh), int(pow_)},
-                 s);
+    write();
 }
 
 void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b, int64_t t, int64_t cin, int64_t h,

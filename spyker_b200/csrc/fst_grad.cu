@@ -58,24 +58,27 @@ struct Stage
     int hp, wp, plane;  // padded height, row stride, plane stride
 };
 
-// The strides near the tight ones that spread 32 neighbouring taps best.
+// The first strides from the tight ones on that spread 32 neighbouring taps
+// best.
 Stage stage_of(const FstGrad &F)
 {
     const int hp = std::max((F.oh - 1) * F.sy + F.kh, F.h + F.top), w0 = std::max((F.ow - 1) * F.sx + F.kw, F.w + F.left);
     const int KK = F.kh * F.kw, taps = std::min(32, F.cin * KK);
+    int tc[32], ty[32], tx[32];
+    for (int k = 0; k < taps; ++k) tc[k] = k / KK, ty[k] = k % KK / F.kw, tx[k] = k % KK % F.kw;
     Stage best{hp, w0, hp * w0};
-    int best_ways = 1 << 30;
-    for (int dw = 0; dw < 8; ++dw)
-        for (int dp = 0; dp < 32; ++dp)
+    int best_ways = taps + 1;
+    // (a few microseconds of host time: it stops at the first strides without
+    // conflicts, and gives a pair up at the best count so far)
+    for (int dw = 0; dw < 8 && best_ways > 1; ++dw)
+        for (int dp = 0; dp < 32 && best_ways > 1; ++dp)
         {
             const int wp = w0 + dw, plane = hp * wp + dp;
-            int n[32] = {}, ways = 0;
-            for (int k = 0; k < taps; ++k)
-            {
-                const int c = k / KK, r = k % KK;
-                ways = std::max(ways, ++n[(c * plane + r / F.kw * wp + r % F.kw) & 31]);
-            }
-            if (ways < best_ways || (ways == best_ways && plane < best.plane)) best_ways = ways, best = {hp, wp, plane};
+            uint8_t n[32] = {};
+            int ways = 0;
+            for (int k = 0; k < taps && ways < best_ways; ++k)
+                ways = std::max<int>(ways, ++n[(tc[k] * plane + ty[k] * wp + tx[k]) & 31]);
+            if (ways < best_ways) best_ways = ways, best = {hp, wp, plane};
         }
     return best;
 }

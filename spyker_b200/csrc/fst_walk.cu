@@ -23,12 +23,11 @@
 // dense kernel's per-term sums add up to; F32(sum) > threshold is tested as
 // sum > bound with the FP64 bound of that rounding.
 #include <algorithm>
-#include <cmath>
-#include <cstring>
 
 #include <cuda_bf16.h>
 
 #include "fst_walk.cuh"
+#include "rounding.cuh"
 
 namespace spk
 {
@@ -318,20 +317,6 @@ __global__ void __launch_bounds__(kStepWarps * 32) fst_steps_kernel(WalkArgs A)
         if (v > A.bound) at = t;
     }
     A.t_out[(smp * A.cout + z0 + threadIdx.x) * A.P + q] = float(at);
-}
-
-// F32(v) > thr, as v > bound: the midpoint between thr and the next float,
-// which itself rounds to the even of the two.
-double rounding_bound(float thr)
-{
-    if (thr != thr || thr == INFINITY) return INFINITY;
-    if (thr == -INFINITY) return -INFINITY;
-    const float up = std::nextafterf(thr, INFINITY);
-    const double next = std::isinf(up) ? std::ldexp(1.0, 128) : double(up);
-    const double mid = double(thr) + (next - double(thr)) * 0.5;
-    uint32_t bits;
-    std::memcpy(&bits, &thr, 4);
-    return bits & 1u ? std::nextafter(mid, -INFINITY) : mid;
 }
 
 struct WalkPlan

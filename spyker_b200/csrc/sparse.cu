@@ -881,6 +881,7 @@ __global__ void sparse_wta_kernel(const int64_t *__restrict__ offsets, const uin
         }
     }
     if (lane == 0) counts[s] = n;
+    for (int i = n * 5 + lane; i < count * 5; i += 32) winners[s * count * 5 + i] = 0;
 }
 
 // ---------------------------------------------------------------------------

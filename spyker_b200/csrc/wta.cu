@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(kWtaThreads)
         ++found;
     }
     if (threadIdx.x == 0) counts[b] = found;
+    for (int i = found * 5 + threadIdx.x; i < count * 5; i += blockDim.x) winners[b * count * 5 + i] = 0;
 }
 
 size_t keys_bytes(int64_t b, int64_t x) { return x <= kWtaSmemKeys ? 0 : (size_t(b) * size_t(x) * 4 + 7) / 8 * 8; }
