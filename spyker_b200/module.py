@@ -110,6 +110,15 @@ class Winners(Sequence):
         return Winners(torch.from_numpy(rec).to(dev), torch.from_numpy(cnt).to(dev))
 
 
+def _winner_buffers(batch: int, count: int, dev: torch.device):
+    """Records and counts of a selection (which writes all of them: a sample's
+    records past its count are zero)."""
+    if count <= 0:
+        return None, None
+    return (torch.empty((batch, count, 5), dtype=torch.int32, device=dev),
+            torch.empty((batch,), dtype=torch.int32, device=dev))
+
+
 class STDPConfig:
     """STDP configuration (utils.h:505-524)."""
 
@@ -563,8 +572,7 @@ def convwta(array, radius, count: int, threshold: float = 0.0) -> Winners:
         raise ValueError("Winners count can't be less than 1.")
     x = Bound(array).dev
     s = to5(list(x.shape))
-    rec = torch.zeros((s[0], count, 5), dtype=torch.int32, device=x.device) if count > 0 else None
-    cnt = torch.zeros((s[0],), dtype=torch.int32, device=x.device) if count > 0 else None
+    rec, cnt = _winner_buffers(s[0], count, x.device)
     ws, wsb = _workspace(_lib.lib.spk_rank_convwta_workspace(*s), x.device)
     call("spk_rank_convwta", ptr(x), type_code(x.dtype), *s, r2[0], r2[1], count, float(threshold), ptr(rec), ptr(cnt),
          ptr(ws), wsb, stream())
@@ -578,8 +586,7 @@ def fcwta(array, radius: int, count: int, threshold: float = 0.0) -> Winners:
         raise ValueError("Winners count can't be less than 1.")
     x = Bound(array).dev
     s = to3(list(x.shape))
-    rec = torch.zeros((s[0], count, 5), dtype=torch.int32, device=x.device) if count > 0 else None
-    cnt = torch.zeros((s[0],), dtype=torch.int32, device=x.device) if count > 0 else None
+    rec, cnt = _winner_buffers(s[0], count, x.device)
     ws, wsb = _workspace(_lib.lib.spk_rank_fcwta_workspace(*s), x.device)
     call("spk_rank_fcwta", ptr(x), type_code(x.dtype), *s, radius, count, float(threshold), ptr(rec), ptr(cnt), ptr(ws),
          wsb, stream())
@@ -752,8 +759,7 @@ def conv_fire_wta(array, conv: "Conv", threshold: float, radius, count: int, val
     pooled = None
     if p2 is not None:
         pooled = torch.empty(shape.pool(oshape, p2, p2, (0, 0, 0, 0)), dtype=torch.uint8, device=x.device)
-    rec = torch.zeros((s[0], count, 5), dtype=torch.int32, device=x.device) if count > 0 else None
-    cnt = torch.zeros((s[0],), dtype=torch.int32, device=x.device) if count > 0 else None
+    rec, cnt = _winner_buffers(s[0], count, x.device)
     ws, wsb = _workspace(nb, x.device)
     call("spk_conv_fire_wta", ptr(x), type_code(x.dtype), ptr(k), s[0], s[1], cin, s[3], s[4], cout, kh, kw,
          conv._stride[0], conv._stride[1], i64(*conv._pad), float(threshold), float(value), float(inhibit_threshold),

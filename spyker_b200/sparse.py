@@ -224,7 +224,7 @@ def inhibit(array) -> SparseTensor:
 
 def convwta(array, radius, count: int):
     """Winners in (step, list) order outside every accepted box (sparse/wta.cpp:44-95)."""
-    from .module import Winners
+    from .module import Winners, _winner_buffers
 
     a = _check(array)
     r2 = expand2(radius)
@@ -233,8 +233,7 @@ def convwta(array, radius, count: int):
     if count <= 0:
         raise ValueError("Winners count can't be less than 1.")
     u, t, c, h, w = a._shape
-    rec = torch.zeros((u, count, 5), dtype=torch.int32, device=a.device)
-    cnt = torch.zeros((u,), dtype=torch.int32, device=a.device)
+    rec, cnt = _winner_buffers(u, count, a.device)
     call("spk_sparse_convwta", ptr(a.offsets), ptr(a.events), u, t, c, h, w, i64(*r2), count, ptr(rec), ptr(cnt),
          stream())
     return Winners(rec, cnt)
