@@ -2989,7 +2989,7 @@ TcParams prepare(const Plan &pl, const void *in, const float *kernel, int64_t n,
         const int64_t cp = pl.nhwc ? pl.cpad : cin;
         negw = reinterpret_cast<int *>(ws + size_t(nnets) * align256(pl.wimg_bytes) +
                                        align256(size_t(n / t_fused) * h * w * cp) + 128);
-        SPK_CUDA(cudaMemsetAsync(negw - 32, 0, 256, s));  // the flag, this word and the search's largest weight
+        SPK_CUDA(cudaMemsetAsync(negw - 32, 0, 256, s));  // the flag, this word and the walk's two
     }
     const dim3 sgrid(grid_for(wthreads, 256), unsigned(nnets));
     split_weights_kernel<<<sgrid, 256, 0, s>>>(kernel, reinterpret_cast<uint4 *>(wimg), int(cout), int(cin),
@@ -3291,8 +3291,8 @@ struct Nets
 // Up to how many output pixels the walk (search_walk.cuh) is the faster
 // search: its time grows with the pixels from a few microseconds, the rounds
 // start near 100 us (some 20 dependent launches) and then spend less per
-// pixel.  2 -> 30 channels 5 x 5: 50k pixels 60 against 140 us, 363k 340
-// against 230; 30 -> 100 channels: 0.2k 17 against 120, 85k 515 against 233.
+// pixel.  2 -> 30 channels 5 x 5: 50k pixels 46 against 140 us, 363k 340
+// against 230; 30 -> 100 channels: 0.2k 14 against 120, 85k 515 against 233.
 bool walk_pays(int64_t npix, int groups, int cout)
 {
     const bool small = groups <= 32 && cout <= 32;  // one load and one channel per lane
@@ -3351,7 +3351,9 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
             search_init_kernel<<<grid_for(b, 256), 256, 0, s>>>(P.mins, P.maxs, b, P.negw, P.flag);
             SPK_LAUNCHED();
         }
-        launch_search_walk(P, WalkSearch{wd, kernel, wtop, nch, groups, rounding_bound(P.thr)}, s);
+        launch_search_walk(P, WalkSearch{wd, kernel, wtop, nch, groups, rounding_bound(P.thr), reinterpret_cast<int *>(la),
+                                        P.negw - 8},
+                           s);
         write();
         return;
     }

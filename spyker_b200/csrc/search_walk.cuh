@@ -16,17 +16,19 @@
 //
 // Bound by issue slots (the sort and the additions, some 1000 instructions a
 // pixel) and, for few pixels, by the latency of one pixel: 2 -> 30 channels 5 x
-// 5 on one image of 28 x 28 6.4 us, on 64 images 60 us; 30 -> 100 channels on
-// one image of 14 x 14 16 us.  The rounds took about 115 us for each of them
+// 5 on one image of 28 x 28 6.2 us, on 64 images 46 us; 30 -> 100 channels on
+// one image of 14 x 14 13.5 us.  The rounds took about 115 us for each of them
 // (64 images: 140 us) and win above some 100,000 pixels (walk_pays).
 //
 // Arithmetic: a channel's weights are the 32-bit integers floor(w 2^(32-e)) of
 // the digit split (the same 2^e, remainder bound and certification as the
 // tensor-core rounds), so a running sum is the exact term total R, in 64-bit
-// integers and in any order.  A decision that the remainders leave open is
-// made from the oracle's ordered FP64 sums; a winner's value that they leave
-// open from an FP64 sum in another order where its error bound rounds to one
-// float, else from the ordered one.
+// integers and in any order.  A winner's value that the remainders leave open
+// comes from an FP64 sum whose error bound rounds to one float; pixels with a
+// decision (or such a sum) left open go to a list, and walk_exact_kernel
+// bisects them with the oracle's ordered FP64 sums.  With that bisection inside
+// the walk the kernel kept a stack and spilled: 60 us instead of 46, and a
+// graph of the launches took 95 to 1300 ms to instantiate instead of 26.
 
 // wd[k][cz]: the integers of input k (channels-last order, `kreal` of them)
 // and channel n, echan / cscale as fixed_split_kernel's, the layer's largest
@@ -106,6 +108,7 @@ struct WalkSearch
     const unsigned *wmax;
     int cz, groups;  // channel stride of wd; 8-channel groups of a receptive field
     double bound;    // F32(S) > thr as S > bound
+    int *redo, *redo_count;  // pixels left to walk_exact_kernel
 };
 
 __device__ __forceinline__ float warp_max(float v)
@@ -157,18 +160,11 @@ __device__ __forceinline__ int walk_decide(const uint64_t (&acc)[NG], const floa
     return 2;
 }
 
-// The oracle's potential of channel o at step t.
-__device__ __noinline__ float walk_oracle(const TcParams &P, const uint8_t *fm, const float *kernel, int o, int iy0,
-                                          int ix0, int t)
-{
-    return float(oracle_sum(P, fm, kernel + int64_t(o) * P.cin * P.kh * P.kw, iy0, ix0, P.cpad, t));
-}
-
 template <int R, int NG>
 __global__ void __launch_bounds__(256, NG <= 4 ? 2 : 1)
     search_walk_kernel(const __grid_constant__ TcParams P, const __grid_constant__ WalkSearch A)
 {
-    constexpr int U = NG <= 4 ? 8 : 4;  // inputs in flight
+    constexpr int U = NG <= 4 && R * NG < 16 ? 8 : 4;  // inputs in flight
     extern __shared__ __align__(16) uint16_t walk_smem[];
     if (*P.negw || *P.flag) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -239,6 +235,7 @@ __global__ void __launch_bounds__(256, NG <= 4 ? 2 : 1)
         for (int r = 0; r < R; ++r) n += __popc(spike_bytes(f[r].x, fired)) + __popc(spike_bytes(f[r].y, fired));
         const int total = __reduce_add_sync(0xffffffffu, n);
         int t0 = T, w = 0;
+        bool redo = false;  // left to walk_exact_kernel
         float v = P.thv;
         // (the widening covers the sum's roundings: K < 2^13 terms)
         if (float(total) * wmax * 1.001f > thr)
@@ -296,11 +293,11 @@ __global__ void __launch_bounds__(256, NG <= 4 ? 2 : 1)
 #pragma unroll
             for (int g = 0; g < NG; ++g) acc[g] = 0;
             bool exact = true;
-            for (int base = 0; base < total && t0 == T; base += 32)
+            for (int base = 0; base < total && t0 == T && !redo; base += 32)
             {
                 const unsigned mine = base + lane < total ? list[base + lane] : 0u;
                 const unsigned ends = __ballot_sync(0xffffffffu, mine & 0x8000u);
-                for (int i0 = 0; i0 < 32 && base + i0 < total && t0 == T; i0 += U)
+                for (int i0 = 0; i0 < 32 && base + i0 < total && t0 == T && !redo; i0 += U)
                 {
                     const unsigned batch = ends >> i0;
                     uint32_t d[U][NG];
@@ -338,20 +335,8 @@ __global__ void __launch_bounds__(256, NG <= 4 ? 2 : 1)
                         int dec = walk_decide<NG>(acc, scale, err, thr, lane, P.cout, w, v, exact);
                         if (dec == 0)
                         {
-                            // the oracle's sums of all channels at this step
-                            float best = -INFINITY;
-                            unsigned bi = 0xFFFFFFFFu;
-                            for (int o = lane; o < P.cout; o += 32)
-                            {
-                                const float pv = walk_oracle(P, fm, A.kernel, o, iy0, ix0, t);
-                                if (pv > best) best = pv, bi = unsigned(o);
-                            }
-                            __syncwarp();
-                            const float top = warp_max(best);
-                            bi = __reduce_min_sync(0xffffffffu, best == top ? bi : 0xFFFFFFFFu);
-                            if (lane == 0) atomicAdd(&g_recomputes, 1ull);
-                            dec = top > thr ? 2 : 1;
-                            if (dec == 2) w = int(bi), v = top, exact = true;
+                            redo = true;
+                            break;
                         }
                         if (dec == 2)
                         {
@@ -361,7 +346,7 @@ __global__ void __launch_bounds__(256, NG <= 4 ? 2 : 1)
                     }
                 }
             }
-            if (t0 < T && P.wta)
+            if (t0 < T && P.wta && !redo)
             {
                 // the winner's total at T - 1: the lanes add the inputs left
                 float vt = v;
@@ -417,16 +402,18 @@ __global__ void __launch_bounds__(256, NG <= 4 ? 2 : 1)
                     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
                     float pv, lo, hi;
                     s_round(s, __double2float_ru(s * 0x1p-39), pv, lo, hi);
-                    if (lo != hi) pv = walk_oracle(P, fm, A.kernel, w, iy0, ix0, t);
+                    redo |= lo != hi;
                     if (lane == 0) atomicAdd(&g_recomputes, 1ull);
                     (pass == 0 ? v : vt) = pv;
                     if (pass == 0 && t0 == T - 1) vt = pv, texact = true;
                 }
-                if (lane == 0) atomicMax(P.maxs + smp, order_enc(vt));
+                if (lane == 0 && !redo) atomicMax(P.maxs + smp, order_enc(vt));
             }
             __syncwarp();
         }
-        if (lane == 0)
+        if (lane == 0 && redo)
+            A.redo[atomicAdd(A.redo_count, 1)] = int(pix);
+        else if (lane == 0)
         {
             P.records[pix] = t0 < T ? make_int4(w, t0, __float_as_int(v), 0) : make_int4(0, T, __float_as_int(P.thv), 0);
             // a step below the threshold leaves its value in the sample
@@ -435,6 +422,70 @@ __global__ void __launch_bounds__(256, NG <= 4 ? 2 : 1)
                 atomicMin(P.mins + smp, order_enc(P.thv));
                 atomicMax(P.maxs + smp, order_enc(P.thv));
             }
+        }
+    }
+}
+
+// The pixels the walk left open, a warp each, from the oracle's sums: the first
+// step at which some channel is above the threshold by bisection (potentials
+// only grow), the first channel of the largest potential there, and with WTA
+// its potential at T - 1.
+__global__ void __launch_bounds__(128) walk_exact_kernel(TcParams P, WalkSearch A)
+{
+    if (*P.negw || *P.flag) return;
+    const int lane = threadIdx.x & 31, T = P.T, n = *A.redo_count;
+    for (int i = blockIdx.x * 4 + (threadIdx.x >> 5); i < n; i += gridDim.x * 4)
+    {
+        const int pix = A.redo[i], smp = pix / int(P.ohw), pp = pix - smp * int(P.ohw);
+        const int oy = pp / P.ow, ox = pp - oy * P.ow, iy0 = oy * P.sy - P.top, ix0 = ox * P.sx - P.left;
+        const uint8_t *fm = P.in + int64_t(smp) * P.img_stride;
+        int lo = -1, hi = T - 1, t = T - 1, w = 0;
+        float v = P.thv, vt = 0.f;
+        bool fires = true, last = false;
+        while (true)
+        {
+            // all channels at step t (the last round: the winner at T - 1)
+            float best = -INFINITY;
+            unsigned bi = 0xFFFFFFFFu;
+            for (int o = lane; o < P.cout; o += 32)
+            {
+                if (last && o != w) continue;
+                const float pv = float(oracle_sum(P, fm, A.kernel + int64_t(o) * P.cin * P.kh * P.kw, iy0, ix0, P.cpad, t));
+                if (pv > best) best = pv, bi = unsigned(o);
+            }
+            __syncwarp();
+            const float top = warp_max(best);
+            bi = __reduce_min_sync(0xffffffffu, best == top ? bi : 0xFFFFFFFFu);
+            if (last)
+            {
+                vt = top;
+                break;
+            }
+            if (top > P.thr)
+                hi = t, w = int(bi), v = top;
+            else if (t == T - 1)
+            {
+                fires = false;
+                break;
+            }
+            else
+                lo = t;
+            if (hi - lo > 1)
+                t = (lo + hi) >> 1;
+            else if (P.wta)
+                last = true, t = T - 1;
+            else
+                break;
+        }
+        if (lane != 0) continue;
+        atomicAdd(&g_recomputes, 1ull);
+        P.records[pix] = fires ? make_int4(w, hi, __float_as_int(v), 0) : make_int4(0, T, __float_as_int(P.thv), 0);
+        if (!P.wta) continue;
+        if (fires) atomicMax(P.maxs + smp, order_enc(vt));
+        if ((!fires || hi > 0) && P.thv != 0.f)
+        {
+            atomicMin(P.mins + smp, order_enc(P.thv));
+            atomicMax(P.maxs + smp, order_enc(P.thv));
         }
     }
 }
@@ -462,4 +513,7 @@ void launch_search_walk(const TcParams &P, const WalkSearch &A, cudaStream_t s)
     else if (P.cout <= 64) by_groups(std::integral_constant<int, 2>());
     else if (P.cout <= 128) by_groups(std::integral_constant<int, 4>());
     else by_groups(std::integral_constant<int, 8>());
+    // (the list of open pixels is almost always empty: a small grid)
+    walk_exact_kernel<<<unsigned(std::min<int64_t>(ceil_div(P.npix, 4), 2 * sm_count())), 128, 0, s>>>(P, A);
+    SPK_LAUNCHED();
 }
