@@ -287,15 +287,6 @@ __device__ __forceinline__ void arrive_expect_tx(uint64_t *bar, uint32_t bytes)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
-// 8-byte asynchronous global -> shared copy (both addresses 8-byte aligned),
-// completed for the issuing thread by cp_async_wait_all.
-__device__ __forceinline__ void cp_async8(void *dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // Bulk (non-tensor) global -> shared copy completing on `bar`; both addresses
 // 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
@@ -1179,12 +1170,11 @@ __device__ __forceinline__ void s_tier2(const TcParams &P, uint32_t lane_base, f
         dec = 1;
 }
 
-// The largest float any channel of value P (its exact total within the
-// rounding cell of P) can round to when the oracle's sum is within E of it.
-__device__ __forceinline__ float s_upper(float P, float E)
+// The largest float a channel of key `m` (units of `unit`, a power of two) can
+// have when the oracle's sum is within E of its exact total.
+__device__ __forceinline__ float s_upper(int m, double unit, float E)
 {
-    const double up = double(P) + 0.5 * (double(nextafterf(P, INFINITY)) - double(P));
-    return float(__dadd_ru(up, double(E)));
+    return float(__dadd_ru((double(m) + 1.0) * unit, double(E)));
 }
 
 // What a decided row does to its pixel (shared by the epilogue and the exact
@@ -1274,26 +1264,32 @@ __device__ __forceinline__ void s_extremes(const TcParams &P, int pix, const Sea
 }
 
 // Search epilogue of one row per thread (warps 0-3).  `emax` is the largest
-// channel bound.  Tier 1 scans the row: each channel's exact total R, its
-// float P = RN(R) * 2^(e - 32) (exact scaling by the channel's power of two),
-// the three largest (first index first).  The winner's value and, when the
-// runner-up is within two ulps, the runner-up's, are certified against their
-// channel bounds; nothing else can change a decision unless the third value
+// channel bound.  Tier 1 scans the row with 31-bit integer keys: a channel's
+// exact total R (u = q0 256 + q1, v = q2 256 + q3, R = u 2^16 + v) without its
+// lowest `drop` bits, shifted to the grid of the channel with the largest
+// weights, so a channel of key m is below (m + 1) `unit`.  The three largest
+// are kept (first index first).  The winner's value and, when the runner-up's
+// upper bound reaches it, the runner-up's, are certified against their channel
+// bounds from their totals; nothing else can change a decision unless the third
 // comes that close too.
+//
+// The keys cost about 20 integer instructions a channel; the 64-bit total of
+// every channel, its conversion to float and the float comparisons took some
+// 100 cycles a channel and warp (10,000 of the 22,000 cycles of a tile of 100
+// channels).
 // Running state of a row's scan over the channel parts of a tile: the three
-// largest potentials, the channels of the first two and their term totals
-// (r1 also carries the winner's total in the last round).
+// largest keys, the channels and totals of the first two (u1, v1 also carry
+// the winner's total in the last round).
 struct SearchScan
 {
-    float p1 = -INFINITY, p2 = -INFINITY, p3 = -INFINITY;
-    int a1 = -1, a2 = -1;
-    uint64_t r1 = 0, r2 = 0;
+    int m1 = -1, m2 = -1, m3 = -1, a1 = -1, a2 = -1;
+    uint32_t u1 = 0, v1 = 0, u2 = 0, v2 = 0;
 };
 
 template <int NS>
 __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pix, int t, int aux, int4 pstate,
-                                uint64_t *release, float emax, const float *scale, const float *bound, int idx,
-                                int part, SearchScan &sc)
+                                uint64_t *release, float emax, double unit, int drop, const float *scale,
+                                const float *bound, const int *shift, int idx, int part, SearchScan &sc)
 {
     const int warp = threadIdx.x >> 5;
     const uint32_t lane_base = acc + (uint32_t((warp & 3) * 32) << 16);
@@ -1306,44 +1302,56 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
     {
         const int col = (ok && aux >= cg && aux < cg + P.n_tile) ? aux - cg : -1;
         const uint64_t R = s_reload<NS>(lane_base, P.n_tile, col);
-        if (col >= 0) sc.r1 = R;
+        if (col >= 0) sc.u1 = uint32_t(R >> 16), sc.v1 = uint32_t(R & 0xFFFFu);
         tc_fence_before();
         mbar_arrive(release);
         if (!last) return;
         if (ok)
         {
             float lo, hi;
-            s_round(double(sc.r1) * double(scale[aux]), bound[aux], v, lo, hi);
+            s_round(double((uint64_t(sc.u1) << 16) + sc.v1) * double(scale[aux]), bound[aux], v, lo, hi);
             dec = lo == hi ? 2 : 3;
             a = aux;
         }
     }
     else
     {
-        float &p1 = sc.p1, &p2 = sc.p2, &p3 = sc.p3;
-        int &a1 = sc.a1, &a2 = sc.a2;
-        uint64_t &r1 = sc.r1, &r2 = sc.r2;
-        for (int cb = 0; cb < P.n_tile; cb += kEpiChunk)
-        {
-            uint32_t q[NS][kEpiChunk];
-            s_chunk<NS>(lane_base, cb, P.n_tile, q);
-            s_chunk_wait<NS>(q);
-            const int lim = P.cout - cg - cb;
+        const int up = 16 - drop;
+        auto scan = [&](const uint32_t(&q)[NS][kEpiChunk], int cb) {
+            const int4 sa = *reinterpret_cast<const int4 *>(shift + cg + cb);
+            const int4 sb = *reinterpret_cast<const int4 *>(shift + cg + cb + 4);
+            const int sh[kEpiChunk] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
 #pragma unroll
             for (int j = 0; j < kEpiChunk; ++j)
             {
-                const uint64_t R = s_total<NS>(q, j);
-                const int c = cg + cb + j;
-                const float pv = j < lim ? __ll2float_rn((long long)R) * scale[c] : -INFINITY;
-                const bool g1 = pv > p1, g2 = !g1 && pv > p2, g3 = !g1 && !g2 && pv > p3;
-                p3 = g1 || g2 ? p2 : (g3 ? pv : p3);
-                p2 = g1 ? p1 : (g2 ? pv : p2);
-                a2 = g1 ? a1 : (g2 ? c : a2);
-                r2 = g1 ? r1 : (g2 ? R : r2);
-                p1 = g1 ? pv : p1;
-                a1 = g1 ? c : a1;
-                r1 = g1 ? R : r1;
+                const uint32_t u = q[0][j] * 256u + q[1][j], v = q[2][j] * 256u + q[3][j];
+                const int key = int(((u << up) + (v >> drop)) >> sh[j]);
+                const bool g1 = key > sc.m1, g2 = key > sc.m2;
+                sc.m3 = max(sc.m3, min(sc.m2, key));
+                sc.m2 = max(sc.m2, min(sc.m1, key));
+                sc.m1 = max(sc.m1, key);
+                sc.a2 = g1 ? sc.a1 : (g2 ? cg + cb + j : sc.a2);
+                sc.u2 = g1 ? sc.u1 : (g2 ? u : sc.u2);
+                sc.v2 = g1 ? sc.v1 : (g2 ? v : sc.v2);
+                sc.a1 = g1 ? cg + cb + j : sc.a1;
+                sc.u1 = g1 ? u : sc.u1;
+                sc.v1 = g1 ? v : sc.v1;
             }
+        };
+        // (two chunks in flight; n_tile is a multiple of 16.  A padding
+        // channel's key is 0 and comes after the layer's two or more channels,
+        // so it is never the first or second)
+        static_assert(NS == 4, "keys of four digits");
+        uint32_t qa[NS][kEpiChunk], qb[NS][kEpiChunk];
+        s_chunk<NS>(lane_base, 0, P.n_tile, qa);
+        for (int cb = 0; cb < P.n_tile; cb += 2 * kEpiChunk)
+        {
+            s_chunk_wait<NS>(qa);
+            s_chunk<NS>(lane_base, cb + kEpiChunk, P.n_tile, qb);
+            scan(qa, cb);
+            s_chunk_wait<NS>(qb);
+            if (cb + 2 * kEpiChunk < P.n_tile) s_chunk<NS>(lane_base, cb + 2 * kEpiChunk, P.n_tile, qa);
+            scan(qb, cb + kEpiChunk);
         }
         if (!last)
         {
@@ -1355,22 +1363,22 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
         bool vexact = false;
         if (ok)
         {
-            if (s_upper(p1, emax) <= thr)
+            const int a1 = sc.a1, a2 = sc.a2;
+            if (s_upper(sc.m1, unit, emax) <= thr)
                 d1 = 1;  // no channel's value can round above the threshold
             else
             {
                 float pa, lo1, hi1;
-                s_round(double(r1) * double(scale[a1]), bound[a1], pa, lo1, hi1);
-                const float near = nextafterf(nextafterf(p1, -INFINITY), -INFINITY);
-                if (lo1 > thr && !(p3 >= near && s_upper(p3, emax) >= lo1))
+                s_round(double((uint64_t(sc.u1) << 16) + sc.v1) * double(scale[a1]), bound[a1], pa, lo1, hi1);
+                if (lo1 > thr && s_upper(sc.m3, unit, emax) < lo1)
                 {
                     bool win = true;
-                    if (p2 >= near && s_upper(p2, emax) >= lo1)
+                    if (s_upper(sc.m2, unit, emax) >= lo1)
                     {
                         float pb, lo2, hi2;
-                        s_round(double(r2) * double(scale[a2]), bound[a2], pb, lo2, hi2);
-                        // both exact: the larger wins, ties to the lower index (a1)
-                        win = lo1 > hi2 || (lo1 == hi1 && lo2 == hi2 && pa >= pb);
+                        s_round(double((uint64_t(sc.u2) << 16) + sc.v2) * double(scale[a2]), bound[a2], pb, lo2, hi2);
+                        // both exact: the larger wins, ties to the lower index
+                        win = lo1 > hi2 || (lo1 == hi1 && lo2 == hi2 && (pa > pb || (pa == pb && a1 < a2)));
                     }
                     if (win) d1 = 2, vexact = lo1 == hi1, v = pa;
                 }
@@ -1393,7 +1401,7 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
             if (d1 == 1)
                 dec = 1;
             else if (d1 == 2)
-                a = a1, dec = vexact ? 2 : 3;
+                a = sc.a1, dec = vexact ? 2 : 3;
             else
                 dec = d2, a = a2t, v = v2;
         }
@@ -1407,29 +1415,38 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
     // exact recompute.  The rarer lists take one atomic per warp each, all
     // in flight at once.
     if (ok && P.round != 2 && (dec == 1 || dec == 2)) P.list_out[idx] = r.next ? r.next_e : make_int2(pix, -1);
-    if (P.round != 2) list_count_warp(P.list_bc, idx, ok && (dec == 1 || dec == 2) && r.next);
     const int lane = threadIdx.x & 31;
+    if (P.round != 2)
+    {
+        // (the warp's 32 rows lie in one compaction block)
+        static_assert(kCompactShift >= 5, "32 rows in a block");
+        const unsigned nx = __ballot_sync(0xffffffffu, ok && (dec == 1 || dec == 2) && r.next);
+        if (nx && lane == 0) atomicAdd(P.list_bc + (idx >> kCompactShift), __popc(nx));
+    }
     const unsigned below = (1u << lane) - 1u;
     const bool wf = ok && dec == 0, wv = ok && dec == 3;
     const unsigned mf = __ballot_sync(0xffffffffu, wf), mv = __ballot_sync(0xffffffffu, wv);
     const unsigned mi = __ballot_sync(0xffffffffu, r.fin);
-    int bf = 0, bv = 0, bi = 0;
-    if (lane == 0)
+    if (mf | mv | mi)
     {
-        if (mf) bf = atomicAdd(P.fix_count, __popc(mf));
-        if (mv) bv = atomicAdd(P.val_count, __popc(mv));
-        if (mi) bi = atomicAdd(P.final_count, __popc(mi));
+        int bf = 0, bv = 0, bi = 0;
+        if (lane == 0)
+        {
+            if (mf) bf = atomicAdd(P.fix_count, __popc(mf));
+            if (mv) bv = atomicAdd(P.val_count, __popc(mv));
+            if (mi) bi = atomicAdd(P.final_count, __popc(mi));
+        }
+        bf = __shfl_sync(0xffffffffu, bf, 0) + __popc(mf & below);
+        bv = __shfl_sync(0xffffffffu, bv, 0) + __popc(mv & below);
+        bi = __shfl_sync(0xffffffffu, bi, 0) + __popc(mi & below);
+        if (wf) P.fix_list[bf] = make_int4(pix, t, idx, aux);
+        if (wv) P.val_list[bv] = make_int4(pix, t, idx, a);
+        if (r.fin) P.final_list[bi] = r.fin_e;
     }
-    bf = __shfl_sync(0xffffffffu, bf, 0) + __popc(mf & below);
-    bv = __shfl_sync(0xffffffffu, bv, 0) + __popc(mv & below);
-    bi = __shfl_sync(0xffffffffu, bi, 0) + __popc(mi & below);
-    if (wf) P.fix_list[bf] = make_int4(pix, t, idx, aux);
-    if (wv) P.val_list[bv] = make_int4(pix, t, idx, a);
-    if (r.fin) P.final_list[bi] = r.fin_e;
     if (P.wta)
     {
         // the sample maxima: one atomic per sample among the warp's lanes
-        const int smp = ok ? pix / int(P.ohw) : -1;
+        const int smp = ok ? int(div_by(uint32_t(pix), P.ohw_m, P.ohw_sh)) : -1;
         const bool has = ok && r.max;
         const unsigned key = has ? unsigned(smp) : 0xFFFFFFFFu;
         const unsigned peers = __match_any_sync(0xffffffffu, key);
@@ -1444,11 +1461,9 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
     }
 }
 
-// A search row's pixel in three words: byte offset of its sample's
-// first-spike map (-1: no row), receptive-field origin (iy0, ix0) packed as
-// two 16-bit fields, and its step.  The search operands are 8-bit and
-// channels-last: a 16-byte chunk of a row is two 8-channel groups, each 8
-// bytes of the first-spike map (0xFF: outside the input).
+// The search operands are 8-bit and channels-last: a 16-byte chunk of a row is
+// two 8-channel groups, each 8 bytes of the first-spike map (0xFF: outside the
+// input).
 
 // Bytes 1 where the first-spike byte f <= t, else 0; tt = (t + 1) * 0x01010101
 // ((f | 0x80) - (t + 1) keeps bit 7 iff f > t, no borrow between bytes).
@@ -1457,140 +1472,181 @@ __device__ __forceinline__ uint32_t spike_bytes(uint32_t f, uint32_t tt)
     return (~((f | 0x80808080u) - tt) >> 7) & 0x01010101u;
 }
 
-// 8-channel group g of a search row (tab entry: first channel, ky, kx,
-// valid); 0xFF bytes outside the input.
-__device__ __forceinline__ uint2 fst_group(const TcParams &P, const int4 *tab, int base, int yx, int g)
+// 8 or 16 bytes of a first-spike map, 0xFF where !ok (a predicated load: no
+// branch, so the loads of all units of a step are in flight together).
+__device__ __forceinline__ uint2 fst_ldg8(const uint8_t *p, bool ok)
 {
-    if (base < 0) return make_uint2(~0u, ~0u);
-    const int iy0 = int(uint32_t(yx) >> 16) - 32768, ix0 = int(uint32_t(yx) & 0xFFFFu) - 32768;
-    const int4 e = tab[g];
-    const int iy = iy0 + e.y, ix = ix0 + e.z;
-    if (e.w && iy >= 0 && iy < P.h && ix >= 0 && ix < P.w)
-        return __ldg(reinterpret_cast<const uint2 *>(P.in + base + (iy * P.w + ix) * P.cpad + e.x));
-    return make_uint2(~0u, ~0u);
+    uint2 r;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.b32 %0, -1;\n\tmov.b32 %1, -1;\n\t"
+        "@p ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t}"
+        : "=&r"(r.x), "=&r"(r.y)
+        : "l"(p), "r"(uint32_t(ok)));
+    return r;
 }
-
-// The list entries of the rows a thread with kc == 0 covers in `tile`, copied
-// into `buf` (128 entries, by row) asynchronously.
-template <int NU>
-__device__ __forceinline__ void entry_prefetch(const TcParams &P, int2 *buf, int64_t tile, int row0, int rs,
-                                               int64_t nrows)
+__device__ __forceinline__ uint4 fst_ldg16(const uint8_t *p, bool ok)
 {
-#pragma unroll
-    for (int i = 0; i < NU; ++i)
-    {
-        const int64_t idx = tile * BM + row0 + rs * i;
-        if (idx < nrows) cp_async8(buf + row0 + rs * i, P.list_in + idx);
-    }
-    cp_async_commit();
+    uint4 r;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.b32 %0, -1;\n\tmov.b32 %1, -1;\n\tmov.b32 %2, -1;\n\t"
+        "mov.b32 %3, -1;\n\t@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w)
+        : "l"(p), "r"(uint32_t(ok)));
+    return r;
 }
 
 // Search producers: a thread builds NU (row, 16-byte chunk) units of every K
 // block (128 U8 elements), one row each at that row's own step.  Unit i of
 // thread p is row (p & 7) + 8 (p >> 6) + (1024 / NU / 8) i and chunk
 // (p >> 3) & 7, so the 8 lanes of a quarter warp take 8 consecutive rows of
-// one chunk (distinct 16-byte bank groups).  The gathers of a step are issued
-// before the wait for its stage, all in flight together.  (Copying them into
-// the stage with 8-byte cp.async and converting in place one step later
-// measured slower: the per-copy issue cost outweighed the deeper pipeline.)
-// In rounds with a row list the threads with kc == 0
-// (together one per row) fetch the next tile's list entries into shared
-// memory (cp.async) while the current tile is built, so their latency leaves
-// the per-tile chain; every producer thread reads them after an mbarrier of
-// the NT producers (two buffers, by tile parity).
-template <int NU>
+// one chunk (distinct 16-byte bank groups).  A unit's bytes are loaded one K
+// block ahead, right after the unit's block before it is stored, so the loads'
+// latency runs beside the stores, the fence and the wait for the next stage.
+// The rows' places (byte offset of the receptive field's origin, its
+// coordinates, the step) are worked out once per row by the first 128 threads,
+// which also hold the next tile's list entries in registers, and handed over
+// in shared memory (two buffers by tile parity, an mbarrier of the NT
+// producers).  WIDE: 16 channels of a chunk in one load (cpad a multiple of
+// 16).  A tile of 100 channels and 7 K blocks took the producers 18,000 cycles
+// with branches around each load, which kept two of them in flight.
+constexpr int kNoRow = 1 << 28;  // a row coordinate outside every input
+template <int NU, bool WIDE>
 __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *tab, unsigned char *smem,
                                                 uint64_t *full_bar, uint64_t *empty_bar, int S, int stage_bytes,
                                                 int a_bytes, int b_bytes, int p, int64_t nrows, int64_t ntiles,
-                                                int2 *s_ent, uint64_t *ent_bar, int *s_tiles, uint64_t *tq_bar)
+                                                int2 *s_row, uint8_t *s_step, uint64_t *ent_bar, int *s_tiles,
+                                                uint64_t *tq_bar)
 {
     constexpr int NT = 1024 / NU, RS = NT / 8;  // producer threads; row step between a thread's units
+    static_assert(NT >= BM, "a thread per row");
     const int row0 = (p & 7) + 8 * (p >> 6), kc = (p >> 3) & 7;
     if (int64_t(blockIdx.x) >= ntiles) return;
     const bool listed = !(P.round == 0 && !P.r0_list);
     const bool dyn = P.tile_ctr != nullptr;
     int ticket = 0;  // (thread 0) the claimed ticket of the tile after the next one
+    int2 ent = make_int2(-1, 0);
+    auto entry = [&](int64_t tile) {  // row p's entry of `tile`
+        const int64_t idx = tile * BM + p;
+        ent = make_int2(-1, 0);
+        if (p < BM && idx < nrows) ent = listed ? P.list_in[idx] : make_int2(int(idx), 0);
+    };
     if (p == 0)
     {
         s_tiles[0] = int(blockIdx.x);
         mbar_arrive(&tq_bar[0]);
         if (dyn) ticket = atomicAdd(P.tile_ctr, 1);
     }
-    if (listed && kc == 0) entry_prefetch<NU>(P, s_ent, blockIdx.x, row0, RS, nrows);
-    int ss = 0;  // the stage ring: slot and pass of the next K block
-    uint32_t su = 0;
-    int64_t tile = blockIdx.x;
-    for (uint32_t k = 0;; ++k)
-    {
+    entry(blockIdx.x);
+    // The rows of the CTA's k-th tile into the buffers; returns the tile after
+    // it (-1: none, -2: gave up).
+    auto setup = [&](uint32_t k, int64_t tile) -> int {
         const int cb = int(k & 1);
-        // thread 0 publishes the tile after this one in the ring (-1: none)
+        // thread 0 publishes the tile after this one in the ring
         if (p == 0)
         {
             const int64_t nt = dyn ? int64_t(gridDim.x) + ticket : tile + gridDim.x;
             s_tiles[(k + 1) & 15] = nt < ntiles ? int(nt) : -1;
             mbar_arrive(&tq_bar[(k + 1) & 15]);
         }
-        if (listed && kc == 0) cp_async_wait_all();
+        if (p < BM)
+        {
+            int2 r = make_int2(0, -1);  // no row
+            if (ent.x >= 0)
+            {
+                const uint32_t smp = div_by(uint32_t(ent.x), P.ohw_m, P.ohw_sh);
+                const uint32_t pix = uint32_t(ent.x) - smp * uint32_t(P.ohw);
+                const int oy = int(div_by(pix, P.ow_m, P.ow_sh)), ox = int(pix) - oy * P.ow;
+                const int iy = oy * P.sy - P.top, ix = ox * P.sx - P.left;
+                r.x = int(int64_t(smp) * P.img_stride) + (iy * P.w + ix) * P.cpad;
+                r.y = int((uint32_t(iy + 32768) << 16) | uint32_t(ix + 32768));
+            }
+            s_row[cb * BM + p] = r;
+            s_step[cb * BM + p] = uint8_t(P.round == 1 ? ent.y : P.T - 1);
+        }
         mbar_arrive(&ent_bar[cb]);
-        if (!wait_bounded(&ent_bar[cb], (k >> 1) & 1)) return;
-        // every thread has read the other entry buffer (the previous tile's)
-        // and sees the next tile
+        if (!wait_bounded(&ent_bar[cb], (k >> 1) & 1)) return -2;
+        // every thread has left the other buffers (the previous tile's) and
+        // sees the next tile
         const int next = s_tiles[(k + 1) & 15];
         if (p == 0 && dyn && next >= 0) ticket = atomicAdd(P.tile_ctr, 1);
-        if (listed && kc == 0 && next >= 0) entry_prefetch<NU>(P, s_ent + (cb ^ 1) * BM, next, row0, RS, nrows);
-        int ubase[NU], uyx[NU];
-        uint32_t utt[NU];
-#pragma unroll
-        for (int i = 0; i < NU; ++i)
+        if (next >= 0) entry(next);
+        return next;
+    };
+    int ubase[NU], uy[NU], ux[NU];
+    uint32_t utt[NU];
+    uint4 f[NU];
+    auto place = [&](uint32_t k, int i) {
+        const int r = int(k & 1) * BM + row0 + RS * i;
+        const int2 e = s_row[r];
+        ubase[i] = e.x;
+        uy[i] = e.y == -1 ? kNoRow : int(uint32_t(e.y) >> 16) - 32768, ux[i] = int(uint32_t(e.y) & 0xFFFFu) - 32768;
+        utt[i] = (uint32_t(s_step[r]) + 1u) * 0x01010101u;
+    };
+    // the chunk's bytes of unit i; ea, eb: its two groups' table entries
+    // (byte offset from the origin, ky, kx)
+    auto load = [&](int i, const int4 &ea, const int4 &eb) {
+        const bool oka = uint32_t(uy[i] + ea.y) < uint32_t(P.h) && uint32_t(ux[i] + ea.z) < uint32_t(P.w);
+        if constexpr (WIDE)
+            f[i] = fst_ldg16(P.in + int64_t(ubase[i] + ea.x), oka);
+        else
         {
-            const int64_t idx = tile * BM + row0 + RS * i;
-            ubase[i] = -1, uyx[i] = 0, utt[i] = 0x01010101u;
-            if (idx < nrows)
+            const bool okb = uint32_t(uy[i] + eb.y) < uint32_t(P.h) && uint32_t(ux[i] + eb.z) < uint32_t(P.w);
+            const uint2 a = fst_ldg8(P.in + int64_t(ubase[i] + ea.x), oka);
+            const uint2 b = fst_ldg8(P.in + int64_t(ubase[i] + eb.x), okb);
+            f[i] = make_uint4(a.x, a.y, b.x, b.y);
+        }
+    };
+    uint32_t k = 0;
+    int next = setup(0, blockIdx.x);
+    if (next == -2) return;
+    {
+        const int4 ea = tab[2 * kc], eb = tab[2 * kc + 1];
+#pragma unroll
+        for (int i = 0; i < NU; ++i) place(0, i), load(i, ea, eb);
+    }
+    int ss = 0;  // the stage ring: slot and pass of the next K block
+    uint32_t su = 0;
+    const int steps = P.nparts * P.kblocks;  // K blocks of a tile
+    for (int step = 0, kb = 0;;)
+    {
+        const bool last = step == steps - 1, more = !last || next >= 0;
+        if (last && more)
+        {
+            ++k;
+            next = setup(k, next);
+            if (next == -2) return;
+        }
+        if (su > 0 && !wait_bounded(&empty_bar[ss], (su - 1) & 1)) return;
+        unsigned char *sA = smem + ss * stage_bytes;
+        if (p == 0)
+        {
+            arrive_expect_tx(&full_bar[ss], uint32_t(b_bytes));
+            bulk_g2s(sA + a_bytes, P.wimg + int64_t(step) * b_bytes, uint32_t(b_bytes), &full_bar[ss]);
+        }
+        auto store = [&](int i) {
+            *reinterpret_cast<uint4 *>(a_row_chunk(sA, row0 + RS * i, kc)) =
+                make_uint4(spike_bytes(f[i].x, utt[i]), spike_bytes(f[i].y, utt[i]), spike_bytes(f[i].z, utt[i]),
+                           spike_bytes(f[i].w, utt[i]));
+        };
+        if (++kb == P.kblocks) kb = 0;
+        const int4 ea = tab[kb * 16 + 2 * kc], eb = tab[kb * 16 + 2 * kc + 1];
+        if (!last)
+        {
+#pragma unroll
+            for (int i = 0; i < NU; ++i) store(i), load(i, ea, eb);
+        }
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < NU; ++i)
             {
-                int2 e = make_int2(int(idx), P.T - 1);
-                if (listed)
-                {
-                    e = s_ent[cb * BM + row0 + RS * i];
-                    if (P.round != 1) e.y = P.T - 1;
-                }
-                const uint32_t smp = div_by(uint32_t(e.x), P.ohw_m, P.ohw_sh);
-                const uint32_t pix = uint32_t(e.x) - smp * uint32_t(P.ohw);
-                const int oy = int(div_by(pix, P.ow_m, P.ow_sh)), ox = int(pix) - oy * P.ow;
-                ubase[i] = int(int64_t(smp) * P.img_stride);
-                uyx[i] = int((uint32_t(oy * P.sy - P.top + 32768) << 16) | uint32_t(ox * P.sx - P.left + 32768));
-                utt[i] = uint32_t(e.y + 1) * 0x01010101u;
+                store(i);
+                if (more) place(k, i), load(i, ea, eb);
             }
         }
-        for (int part = 0; part < P.nparts; ++part)
-            for (int kb = 0; kb < P.kblocks; ++kb)
-            {
-                uint2 fa[NU], fb[NU];
-#pragma unroll
-                for (int i = 0; i < NU; ++i)
-                {
-                    fa[i] = fst_group(P, tab, ubase[i], uyx[i], kb * 16 + 2 * kc);
-                    fb[i] = fst_group(P, tab, ubase[i], uyx[i], kb * 16 + 2 * kc + 1);
-                }
-                const int s = ss;
-                if (su > 0 && !wait_bounded(&empty_bar[s], (su - 1) & 1)) return;
-                unsigned char *sA = smem + s * stage_bytes;
-                if (p == 0)
-                {
-                    arrive_expect_tx(&full_bar[s], uint32_t(b_bytes));
-                    bulk_g2s(sA + a_bytes, P.wimg + (int64_t(part) * P.kblocks + kb) * b_bytes, uint32_t(b_bytes),
-                             &full_bar[s]);
-                }
-#pragma unroll
-                for (int i = 0; i < NU; ++i)
-                    *reinterpret_cast<uint4 *>(a_row_chunk(sA, row0 + RS * i, kc)) =
-                        make_uint4(spike_bytes(fa[i].x, utt[i]), spike_bytes(fa[i].y, utt[i]),
-                                   spike_bytes(fb[i].x, utt[i]), spike_bytes(fb[i].y, utt[i]));
-                fence_proxy_async_smem();
-                mbar_arrive(&full_bar[s]);
-                if (++ss == S) ss = 0, ++su;
-            }
-        if (next < 0) break;
-        tile = next;
+        fence_proxy_async_smem();
+        mbar_arrive(&full_bar[ss]);
+        if (++ss == S) ss = 0, ++su;
+        step = last ? 0 : step + 1;
+        if (!more) break;
     }
 }
 
@@ -1648,18 +1704,29 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     // search: the channels' scales and bounds, staged after the table
     const int nch = MODE == kSearch ? P.nparts * P.n_tile : P.n_tile;  // channels of the tables
     float *s_scale = reinterpret_cast<float *>(tab + P.kblocks * 16), *s_bound = s_scale + nch;
-    // search: two buffers of the next tile's list entries (128 each)
-    int2 *s_ent = reinterpret_cast<int2 *>(s_bound + nch + ((16 - ((2 * nch) & 15)) & 15));
+    // search: the channels' shifts to the common grid of the keys (nch is a
+    // multiple of 16), two buffers of the tile's rows (128 each): places, steps
+    int *s_shift = reinterpret_cast<int *>(s_bound + nch);
+    int2 *s_row = reinterpret_cast<int2 *>(s_shift + nch);
+    uint8_t *s_step = reinterpret_cast<uint8_t *>(s_row + 2 * BM);
     if constexpr (MODE == kSearch)
     {
         // per 8-element group of a 128-element K block (channels-last, 8-bit
-        // operands): (first channel, ky, kx, valid)
+        // operands): (byte offset from the receptive field's origin, ky, kx)
         for (int g = tid; g < P.kblocks * 16; g += blockDim.x)
         {
-            const int k = g * 8, tap = k / P.cpad, c = k % P.cpad;
-            tab[g] = make_int4(c, tap / P.kw, tap % P.kw, (tap < taps && c < P.cin) ? 1 : 0);
+            const int k = g * 8, tap = k / P.cpad, c = k % P.cpad, ky = tap / P.kw, kx = tap % P.kw;
+            tab[g] = (tap < taps && c < P.cin) ? make_int4((ky * P.w + kx) * P.cpad + c, ky, kx, 0)
+                                               : make_int4(0, kNoRow, 0, 0);
         }
-        for (int c = tid; c < nch; c += blockDim.x) s_scale[c] = P.cscale[c], s_bound[c] = P.echan[c];
+        // cscale = 2^(e - 32), e the channel's exponent; sinfo[1] the largest e + 128
+        for (int c = tid; c < nch; c += blockDim.x)
+        {
+            const float sc = P.cscale[c];
+            s_scale[c] = sc, s_bound[c] = P.echan[c];
+            const int e = int(__float_as_uint(sc) >> 23) - 127 + 8 * kSearchTerms;
+            s_shift[c] = min(max(int(P.sinfo[1]) - 128 - e, 0), 31);
+        }
     }
     else if constexpr (MODE != kPotentials)
     {
@@ -1715,8 +1782,15 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
 
     constexpr int kMmaWarp = 4 + NPW;
     if (MODE == kSearch && warp >= 4 && warp < kMmaWarp)
-        search_producer<1024 / (32 * NPW)>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes,
-                                           tid - 128, nrows, ntiles, s_ent, ent_bar, s_tiles, tq_bar);
+    {
+        constexpr int NU = 1024 / (32 * NPW);
+        if (P.cpad % 16 == 0 && (reinterpret_cast<uintptr_t>(P.in) & 15) == 0 && (P.img_stride & 15) == 0)
+            search_producer<NU, true>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128,
+                                      nrows, ntiles, s_row, s_step, ent_bar, s_tiles, tq_bar);
+        else
+            search_producer<NU, false>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128,
+                                       nrows, ntiles, s_row, s_step, ent_bar, s_tiles, tq_bar);
+    }
     else if (MODE != kPotentials && MODE != kSearch && warp >= 4 && warp < kMmaWarp)
     {
         // ---------------- fused producers (8 warps) ----------------
@@ -1864,8 +1938,17 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
         // warp w reads tensor-memory lanes 32 w .. 32 w + 31 (rows of the tile)
         const int row = (warp & 3) * 32 + lane;
         // the largest channel bound (search)
+        // and the grid of its keys: R < inputs 2^32, so `drop` bits fewer
+        // leave 31
         float emax = 0.f;
-        if constexpr (MODE == kSearch) emax = __uint_as_float(P.sinfo[0]);
+        double unit = 0.0;
+        int drop = 1;
+        if constexpr (MODE == kSearch)
+        {
+            emax = __uint_as_float(P.sinfo[0]);
+            while ((1 << (drop - 1)) < P.cin * taps) ++drop;
+            unit = ldexp(1.0, drop + int(P.sinfo[1]) - 128 - 8 * kSearchTerms);
+        }
         uint32_t j = 0, k = 0;
         const int parts = MODE == kSearch ? P.nparts : 1;
         SearchScan scan;
@@ -1945,7 +2028,8 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
             {
                 if (part == 0) scan = SearchScan{};
                 search_epilogue<kSearchTerms>(P, acc, s_ok, s_e.x, s_e.y, P.round == 2 ? s_aux : 0, s_st,
-                                              &acce_bar[a], emax, s_scale, s_bound, int(tile * BM + row), part, scan);
+                                              &acce_bar[a], emax, unit, drop, s_scale, s_bound, s_shift, int(tile * BM + row),
+                                              part, scan);
             }
             else if constexpr (MODE == kFused)
             {
@@ -2196,7 +2280,7 @@ __global__ void __launch_bounds__(256) fixed_split_kernel(const float *__restric
     __syncthreads();
     mx = s_mx[0], lsb = s_lsb[0];
     for (int i = 1; i < int(blockDim.x >> 5); ++i) mx = fmaxf(mx, s_mx[i]), lsb = min(lsb, s_lsb[i]);
-    int e = 0;
+    int e = -94;  // (a channel without a positive weight: the smallest grid, so that it never sets the largest)
     if (mx > 0.f)
     {
         int ex;
@@ -2761,9 +2845,9 @@ Plan make_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64
         pl.xt_bytes = pl.nhwc ? size_t(n) * h * w * pl.cpad : 0;
     // (kTimes: the table is followed by the per-warp first-step candidates,
     // two buffers of 4 warps x n_tile ints)
-    // (search: 16 group entries per K block, the channels' scales and bounds
-    // and two buffers of tile entries)
-    const size_t tab = nsplit > 0   ? size_t(pl.kblocks) * 256 + size_t(pl.parts) * pl.n_tile * 8 + 64 + 2 * BM * 8
+    // (search: 16 group entries per K block, the channels' scales, bounds and
+    // shifts and two buffers of tile rows)
+    const size_t tab = nsplit > 0   ? size_t(pl.kblocks) * 256 + size_t(pl.parts) * pl.n_tile * 12 + 2 * BM * 9
                        : t_fused > 0 ? (size_t(pl.kblocks) * BK + 8) * 16 + (times ? size_t(pl.n_tile) * 32 : 0)
                        : !pl.nhwc   ? size_t(pl.kblocks) * BK * 16
                                     : size_t(pl.kblocks) * 8 * 16;
