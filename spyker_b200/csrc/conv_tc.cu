@@ -137,7 +137,8 @@ struct TcParams
     int *val_count;
     int4 *state;     // per pixel: (lo | hi << 8 | winner << 16, value, winner at T-1, value at T-1)
     const float *echan;     // per channel bound of |oracle potential - exact term sum|
-    const float *cscale;    // per channel 2^(e - 32): the value of one unit of the term total
+    const float *cscale;    // per channel, the value of one unit of the term total (2^(e - 31); the walk 2^(e - 32))
+    const float *ccent;     // per channel, the middle of what the split left out
     const unsigned *sinfo;  // [0] largest echan (bits), [1] largest channel exponent + 128
     int kreal;              // real K (taps x input channels)
     int r0_list;            // round 0 takes the (pixel, T - 1) entries of list_in (bound pre-filter ran)
@@ -151,8 +152,9 @@ struct TcParams
 // kTimes: the fused (pixel, time) rows with an epilogue that writes each
 // neuron's first step above threshold (F32 time, T = never).
 constexpr int kPotentials = 0, kFused = 1, kTimes = 2, kSearch = 3;
-// Base-256 digits per weight of the search kernels' 8-bit split.
-constexpr int kSearchTerms = 4;
+// Accumulator columns per channel of the search kernels (fixed_split_kernel):
+// the upper 16 and the lower 15 bits of a weight's 31-bit integer.
+constexpr int kSearchTerms = 2, kLowBits = 15, kSearchBits = 31;
 
 __device__ __forceinline__ unsigned order_enc(float f)
 {
@@ -1080,18 +1082,18 @@ __device__ __forceinline__ void s_chunk_wait(uint32_t (&q)[NS][kEpiChunk])
     for (int j = 0; j < NS; ++j) tmem_ld_wait8(q[j]);
 }
 
-// Exact term total of a column: the NS 32-bit accumulators hold sums of
-// base-256 digit products, so the total is an integer below 2^46.
-template <int NS>
-__device__ __forceinline__ uint64_t s_total(const uint32_t (&q)[NS][kEpiChunk], int j)
+// Exact term total: the two accumulators hold the sums of the upper and lower
+// bits, so the total is an integer below 2^45.
+__device__ __forceinline__ uint64_t s_total(uint32_t u, uint32_t v) { return (uint64_t(u) << kLowBits) + v; }
+
+// The middle of what a channel's potential can be: its total's value plus the
+// middle of the remainders (exact but for one rounding that the bound covers).
+__device__ __forceinline__ double s_value(uint64_t R, float scale, float cent)
 {
-    uint64_t r = 0;
-#pragma unroll
-    for (int i = 0; i < NS; ++i) r = (r << 8) + uint64_t(q[i][j]);
-    return r;
+    return double(R) * double(scale) + double(cent);
 }
 
-// The floats a potential within E of the exact S (= R * scale) can round to:
+// The floats a potential within E of S can round to:
 // [lo, hi] = [RN(S - E), RN(S + E)] (RN is monotone); lo == hi: P is the
 // oracle's value.  E == 0: the term total is the oracle's FP64 sum itself.
 __device__ __forceinline__ void s_round(double S, float E, float &P, float &lo, float &hi)
@@ -1122,7 +1124,7 @@ __device__ __forceinline__ uint64_t s_reload(uint32_t lane_base, int n_tile, int
         const bool mine = col >= 0 && (col >> 3) == (c0 >> 3);
         const int jj = col - c0;
 #pragma unroll
-        for (int j = 0; j < kEpiChunk; ++j) R = (mine && jj == j) ? s_total<NS>(q, j) : R;
+        for (int j = 0; j < kEpiChunk; ++j) R = (mine && jj == j) ? s_total(q[0][j], q[1][j]) : R;
         pending &= ~__ballot_sync(0xffffffffu, mine);
     }
     return R;
@@ -1132,7 +1134,7 @@ __device__ __forceinline__ uint64_t s_reload(uint32_t lane_base, int n_tile, int
 // channel above thr, 2 crossing with winner a (first of the largest) of value v.
 template <int NS>
 __device__ __forceinline__ void s_tier2(const TcParams &P, uint32_t lane_base, float thr, int &dec, int &a, float &v,
-                                        const float *scale, const float *bound)
+                                        const float *scale, const float *bound, const float *cent)
 {
     float mlo = -INFINITY, hmax = -INFINITY, hun = -INFINITY, vs = -INFINITY;
     int as = -1;
@@ -1147,7 +1149,7 @@ __device__ __forceinline__ void s_tier2(const TcParams &P, uint32_t lane_base, f
             const int c = c0 + j;
             const bool real = c < P.cout;
             float pc, lo, hi;
-            const double S = double(s_total<NS>(q, j)) * double(real ? scale[c] : 0.f);
+            const double S = real ? s_value(s_total(q[0][j], q[1][j]), scale[c], cent[c]) : 0.0;
             s_round(S, real ? bound[c] : 0.f, pc, lo, hi);
             if (!real) lo = hi = pc = -INFINITY;
             mlo = fmaxf(mlo, lo);
@@ -1265,31 +1267,32 @@ __device__ __forceinline__ void s_extremes(const TcParams &P, int pix, const Sea
 
 // Search epilogue of one row per thread (warps 0-3).  `emax` is the largest
 // channel bound.  Tier 1 scans the row with 31-bit integer keys: a channel's
-// exact total R (u = q0 256 + q1, v = q2 256 + q3, R = u 2^16 + v) without its
-// lowest `drop` bits, shifted to the grid of the channel with the largest
-// weights, so a channel of key m is below (m + 1) `unit`.  The three largest
-// are kept (first index first).  The winner's value and, when the runner-up's
-// upper bound reaches it, the runner-up's, are certified against their channel
-// bounds from their totals; nothing else can change a decision unless the third
-// comes that close too.
+// exact total R (R = u 2^15 + v from its two columns) without its lowest `drop`
+// bits, shifted to the grid of the channel with the largest weights, so a
+// channel of key m is below (m + 1) `unit`.  The three largest are kept (first
+// index first).  The winner's value and, when the runner-up's upper bound
+// reaches it, the runner-up's, are certified against their channel bounds from
+// their totals; nothing else can change a decision unless the third comes that
+// close too.
 //
-// The keys cost about 20 integer instructions a channel; the 64-bit total of
-// every channel, its conversion to float and the float comparisons took some
-// 100 cycles a channel and warp (10,000 of the 22,000 cycles of a tile of 100
-// channels).
+// Bound by the integer pipe (half rate, which the producers share).  64-bit
+// totals of every channel, their conversion to float and float comparisons
+// took some 100 cycles a channel and warp, keys of four digit columns 60.
 // Running state of a row's scan over the channel parts of a tile: the three
-// largest keys, the channels and totals of the first two (u1, v1 also carry
-// the winner's total in the last round).
+// largest keys, the channels of the first two and the total of the first (u1,
+// v1 also carry the winner's total in the last round).  MULTI (several parts):
+// also the second's total; with one part it is read again when it is needed.
 struct SearchScan
 {
     int m1 = -1, m2 = -1, m3 = -1, a1 = -1, a2 = -1;
     uint32_t u1 = 0, v1 = 0, u2 = 0, v2 = 0;
 };
 
-template <int NS>
+template <int NS, bool MULTI>
 __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pix, int t, int aux, int4 pstate,
                                 uint64_t *release, float emax, double unit, int drop, const float *scale,
-                                const float *bound, const int *shift, int idx, int part, SearchScan &sc)
+                                const float *bound, const float *cent, const int *shift, int idx, int part,
+                                SearchScan &sc)
 {
     const int warp = threadIdx.x >> 5;
     const uint32_t lane_base = acc + (uint32_t((warp & 3) * 32) << 16);
@@ -1302,21 +1305,21 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
     {
         const int col = (ok && aux >= cg && aux < cg + P.n_tile) ? aux - cg : -1;
         const uint64_t R = s_reload<NS>(lane_base, P.n_tile, col);
-        if (col >= 0) sc.u1 = uint32_t(R >> 16), sc.v1 = uint32_t(R & 0xFFFFu);
+        if (col >= 0) sc.u1 = uint32_t(R >> kLowBits), sc.v1 = uint32_t(R) & ((1u << kLowBits) - 1u);
         tc_fence_before();
         mbar_arrive(release);
         if (!last) return;
         if (ok)
         {
             float lo, hi;
-            s_round(double((uint64_t(sc.u1) << 16) + sc.v1) * double(scale[aux]), bound[aux], v, lo, hi);
+            s_round(s_value(s_total(sc.u1, sc.v1), scale[aux], cent[aux]), bound[aux], v, lo, hi);
             dec = lo == hi ? 2 : 3;
             a = aux;
         }
     }
     else
     {
-        const int up = 16 - drop;
+        const uint32_t up = 1u << (kLowBits - drop);
         auto scan = [&](const uint32_t(&q)[NS][kEpiChunk], int cb) {
             const int4 sa = *reinterpret_cast<const int4 *>(shift + cg + cb);
             const int4 sb = *reinterpret_cast<const int4 *>(shift + cg + cb + 4);
@@ -1324,15 +1327,18 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
 #pragma unroll
             for (int j = 0; j < kEpiChunk; ++j)
             {
-                const uint32_t u = q[0][j] * 256u + q[1][j], v = q[2][j] * 256u + q[3][j];
-                const int key = int(((u << up) + (v >> drop)) >> sh[j]);
+                const uint32_t u = q[0][j], v = q[1][j];
+                const int key = int((u * up + (v >> drop)) >> sh[j]);
                 const bool g1 = key > sc.m1, g2 = key > sc.m2;
                 sc.m3 = max(sc.m3, min(sc.m2, key));
                 sc.m2 = max(sc.m2, min(sc.m1, key));
                 sc.m1 = max(sc.m1, key);
                 sc.a2 = g1 ? sc.a1 : (g2 ? cg + cb + j : sc.a2);
-                sc.u2 = g1 ? sc.u1 : (g2 ? u : sc.u2);
-                sc.v2 = g1 ? sc.v1 : (g2 ? v : sc.v2);
+                if constexpr (MULTI)
+                {
+                    sc.u2 = g1 ? sc.u1 : (g2 ? u : sc.u2);
+                    sc.v2 = g1 ? sc.v1 : (g2 ? v : sc.v2);
+                }
                 sc.a1 = g1 ? cg + cb + j : sc.a1;
                 sc.u1 = g1 ? u : sc.u1;
                 sc.v1 = g1 ? v : sc.v1;
@@ -1341,7 +1347,7 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
         // (two chunks in flight; n_tile is a multiple of 16.  A padding
         // channel's key is 0 and comes after the layer's two or more channels,
         // so it is never the first or second)
-        static_assert(NS == 4, "keys of four digits");
+        static_assert(NS == 2, "keys of two columns");
         uint32_t qa[NS][kEpiChunk], qb[NS][kEpiChunk];
         s_chunk<NS>(lane_base, 0, P.n_tile, qa);
         for (int cb = 0; cb < P.n_tile; cb += 2 * kEpiChunk)
@@ -1360,28 +1366,32 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
             return;
         }
         int d1 = 0;  // tier-1 decision: 0 open, 1 below, 2 winner decided (value certified or not)
-        bool vexact = false;
+        bool vexact = false, near2 = false;
+        float pa = 0.f, lo1 = 0.f, hi1 = 0.f;
         if (ok)
         {
-            const int a1 = sc.a1, a2 = sc.a2;
             if (s_upper(sc.m1, unit, emax) <= thr)
                 d1 = 1;  // no channel's value can round above the threshold
             else
             {
-                float pa, lo1, hi1;
-                s_round(double((uint64_t(sc.u1) << 16) + sc.v1) * double(scale[a1]), bound[a1], pa, lo1, hi1);
+                s_round(s_value(s_total(sc.u1, sc.v1), scale[sc.a1], cent[sc.a1]), bound[sc.a1], pa, lo1, hi1);
                 if (lo1 > thr && s_upper(sc.m3, unit, emax) < lo1)
                 {
-                    bool win = true;
-                    if (s_upper(sc.m2, unit, emax) >= lo1)
-                    {
-                        float pb, lo2, hi2;
-                        s_round(double((uint64_t(sc.u2) << 16) + sc.v2) * double(scale[a2]), bound[a2], pb, lo2, hi2);
-                        // both exact: the larger wins, ties to the lower index
-                        win = lo1 > hi2 || (lo1 == hi1 && lo2 == hi2 && (pa > pb || (pa == pb && a1 < a2)));
-                    }
-                    if (win) d1 = 2, vexact = lo1 == hi1, v = pa;
+                    near2 = s_upper(sc.m2, unit, emax) >= lo1;
+                    if (!near2) d1 = 2, vexact = lo1 == hi1, v = pa;
                 }
+            }
+        }
+        if (__any_sync(0xffffffffu, near2))
+        {
+            const uint64_t R2 = MULTI ? s_total(sc.u2, sc.v2) : s_reload<NS>(lane_base, P.n_tile, near2 ? sc.a2 : -1);
+            if (near2)
+            {
+                float pb, lo2, hi2;
+                s_round(s_value(R2, scale[sc.a2], cent[sc.a2]), bound[sc.a2], pb, lo2, hi2);
+                // both exact: the larger wins, ties to the lower index
+                if (lo1 > hi2 || (lo1 == hi1 && lo2 == hi2 && (pa > pb || (pa == pb && sc.a1 < sc.a2))))
+                    d1 = 2, vexact = lo1 == hi1, v = pa;
             }
         }
         int d2 = 0, a2t = -1;
@@ -1392,7 +1402,7 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
         if (open1 && P.nparts == 1)
         {
             if ((threadIdx.x & 31) == 0) atomicAdd(&g_rechecks, (unsigned long long)__popc(open1));
-            s_tier2<NS>(P, lane_base, thr, d2, a2t, v2, scale, bound);
+            s_tier2<NS>(P, lane_base, thr, d2, a2t, v2, scale, bound, cent);
         }
         tc_fence_before();
         mbar_arrive(release);
@@ -1465,11 +1475,14 @@ __device__ void search_epilogue(const TcParams &P, uint32_t acc, bool ok, int pi
 // two 8-channel groups, each 8 bytes of the first-spike map (0xFF: outside the
 // input).
 
-// Bytes 1 where the first-spike byte f <= t, else 0; tt = (t + 1) * 0x01010101
-// ((f | 0x80) - (t + 1) keeps bit 7 iff f > t, no borrow between bytes).
-__device__ __forceinline__ uint32_t spike_bytes(uint32_t f, uint32_t tt)
+// Bytes 0xFF where the first-spike byte f <= t, else 0; tt = 0x80808080 + t *
+// 0x01010101 (f is 0 .. 127 or 0xFF, t <= 126: the difference keeps bit 7 iff
+// f <= t, no borrow between bytes; prmt then copies each byte's sign).
+__device__ __forceinline__ uint32_t spike_mask(uint32_t f, uint32_t tt)
 {
-    return (~((f | 0x80808080u) - tt) >> 7) & 0x01010101u;
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(r) : "r"(tt - (f & 0x7F7F7F7Fu)));
+    return r;
 }
 
 // 8 or 16 bytes of a first-spike map, 0xFF where !ok (a predicated load: no
@@ -1493,31 +1506,35 @@ __device__ __forceinline__ uint4 fst_ldg16(const uint8_t *p, bool ok)
     return r;
 }
 
-// Search producers: a thread builds NU (row, 16-byte chunk) units of every K
-// block (128 U8 elements), one row each at that row's own step.  Unit i of
-// thread p is row (p & 7) + 8 (p >> 6) + (1024 / NU / 8) i and chunk
-// (p >> 3) & 7, so the 8 lanes of a quarter warp take 8 consecutive rows of
-// one chunk (distinct 16-byte bank groups).  A unit's bytes are loaded one K
-// block ahead, right after the unit's block before it is stored, so the loads'
-// latency runs beside the stores, the fence and the wait for the next stage.
+// Search producers.  A K block is 64 inputs, each twice in a row's 128 bytes:
+// chunks 0 .. 3 hold 255 where the input has fired by the row's step (they
+// meet the multiples of 255 of the weights' fields, fixed_split_kernel),
+// chunks 4 .. 7 hold 1.  The warps form groups of four that take the K blocks
+// in turn; a thread builds four (row, 16-input chunk) units of its group's
+// block: rows (p & 7) + 8 (p >> 5) + 32 i of chunk (p >> 3) & 3, so the 8 lanes
+// of a quarter warp take 8 consecutive rows of one chunk (distinct 16-byte bank
+// groups).  A unit's bytes are loaded one block of the group ahead, right after
+// the unit's block before it is stored, so the loads' latency runs beside the
+// stores, the fence and the wait for the next stage.
 // The rows' places (byte offset of the receptive field's origin, its
 // coordinates, the step) are worked out once per row by the first 128 threads,
 // which also hold the next tile's list entries in registers, and handed over
-// in shared memory (two buffers by tile parity, an mbarrier of the NT
-// producers).  WIDE: 16 channels of a chunk in one load (cpad a multiple of
-// 16).  A tile of 100 channels and 7 K blocks took the producers 18,000 cycles
-// with branches around each load, which kept two of them in flight.
+// in shared memory (two buffers by tile parity, an mbarrier of all producers).
+// WIDE: 16 channels of a chunk in one load (cpad a multiple of 16).  With
+// branches around each load, which kept two of them in flight, the producers
+// of a tile of 100 channels and 800 inputs took 18,000 cycles.
 constexpr int kNoRow = 1 << 28;  // a row coordinate outside every input
-template <int NU, bool WIDE>
+template <int NPW, bool WIDE>
 __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *tab, unsigned char *smem,
                                                 uint64_t *full_bar, uint64_t *empty_bar, int S, int stage_bytes,
-                                                int a_bytes, int b_bytes, int p, int64_t nrows, int64_t ntiles,
+                                                int a_bytes, int b_bytes, int tid, int64_t nrows, int64_t ntiles,
                                                 int2 *s_row, uint8_t *s_step, uint64_t *ent_bar, int *s_tiles,
                                                 uint64_t *tq_bar)
 {
-    constexpr int NT = 1024 / NU, RS = NT / 8;  // producer threads; row step between a thread's units
-    static_assert(NT >= BM, "a thread per row");
-    const int row0 = (p & 7) + 8 * (p >> 6), kc = (p >> 3) & 7;
+    constexpr int G = NPW / 4, NU = 4;
+    static_assert(NPW % 4 == 0 && BM == 128, "a thread per row");
+    const int p = tid & 127, grp = tid >> 7;
+    const int row0 = (p & 7) + 8 * (p >> 5), kc = (p >> 3) & 3;
     if (int64_t(blockIdx.x) >= ntiles) return;
     const bool listed = !(P.round == 0 && !P.r0_list);
     const bool dyn = P.tile_ctr != nullptr;
@@ -1526,9 +1543,9 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
     auto entry = [&](int64_t tile) {  // row p's entry of `tile`
         const int64_t idx = tile * BM + p;
         ent = make_int2(-1, 0);
-        if (p < BM && idx < nrows) ent = listed ? P.list_in[idx] : make_int2(int(idx), 0);
+        if (grp == 0 && idx < nrows) ent = listed ? P.list_in[idx] : make_int2(int(idx), 0);
     };
-    if (p == 0)
+    if (tid == 0)
     {
         s_tiles[0] = int(blockIdx.x);
         mbar_arrive(&tq_bar[0]);
@@ -1540,13 +1557,13 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
     auto setup = [&](uint32_t k, int64_t tile) -> int {
         const int cb = int(k & 1);
         // thread 0 publishes the tile after this one in the ring
-        if (p == 0)
+        if (tid == 0)
         {
             const int64_t nt = dyn ? int64_t(gridDim.x) + ticket : tile + gridDim.x;
             s_tiles[(k + 1) & 15] = nt < ntiles ? int(nt) : -1;
             mbar_arrive(&tq_bar[(k + 1) & 15]);
         }
-        if (p < BM)
+        if (grp == 0)
         {
             int2 r = make_int2(0, -1);  // no row
             if (ent.x >= 0)
@@ -1566,7 +1583,7 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
         // every thread has left the other buffers (the previous tile's) and
         // sees the next tile
         const int next = s_tiles[(k + 1) & 15];
-        if (p == 0 && dyn && next >= 0) ticket = atomicAdd(P.tile_ctr, 1);
+        if (tid == 0 && dyn && next >= 0) ticket = atomicAdd(P.tile_ctr, 1);
         if (next >= 0) entry(next);
         return next;
     };
@@ -1574,11 +1591,11 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
     uint32_t utt[NU];
     uint4 f[NU];
     auto place = [&](uint32_t k, int i) {
-        const int r = int(k & 1) * BM + row0 + RS * i;
+        const int r = int(k & 1) * BM + row0 + 32 * i;
         const int2 e = s_row[r];
         ubase[i] = e.x;
         uy[i] = e.y == -1 ? kNoRow : int(uint32_t(e.y) >> 16) - 32768, ux[i] = int(uint32_t(e.y) & 0xFFFFu) - 32768;
-        utt[i] = (uint32_t(s_step[r]) + 1u) * 0x01010101u;
+        utt[i] = 0x80808080u + uint32_t(s_step[r]) * 0x01010101u;
     };
     // the chunk's bytes of unit i; ea, eb: its two groups' table entries
     // (byte offset from the origin, ky, kx)
@@ -1594,41 +1611,62 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
             f[i] = make_uint4(a.x, a.y, b.x, b.y);
         }
     };
+    // K blocks of a tile (part-major), the group's current one and its tile
+    const int steps = P.nparts * P.kblocks;
     uint32_t k = 0;
-    int next = setup(0, blockIdx.x);
+    int next = setup(0, blockIdx.x), step = grp;
     if (next == -2) return;
-    {
-        const int4 ea = tab[2 * kc], eb = tab[2 * kc + 1];
-#pragma unroll
-        for (int i = 0; i < NU; ++i) place(0, i), load(i, ea, eb);
-    }
-    int ss = 0;  // the stage ring: slot and pass of the next K block
-    uint32_t su = 0;
-    const int steps = P.nparts * P.kblocks;  // K blocks of a tile
-    for (int step = 0, kb = 0;;)
-    {
-        const bool last = step == steps - 1, more = !last || next >= 0;
-        if (last && more)
+    // to the group's next block: 1 same tile, 2 a later one, 0 none left, -1 gave up
+    auto settle = [&]() -> int {
+        int moved = 1;
+        while (step >= steps)
         {
-            ++k;
-            next = setup(k, next);
-            if (next == -2) return;
+            if (next < 0) return 0;
+            step -= steps, moved = 2;
+            next = setup(++k, next);
+            if (next == -2) return -1;
         }
+        return moved;
+    };
+    if (settle() <= 0) return;
+    auto chunk = [&](int4 &ea, int4 &eb) {
+        int kb = step;
+        while (kb >= P.kblocks) kb -= P.kblocks;
+        ea = tab[kb * 8 + 2 * kc], eb = tab[kb * 8 + 2 * kc + 1];
+    };
+    {
+        int4 ea, eb;
+        chunk(ea, eb);
+#pragma unroll
+        for (int i = 0; i < NU; ++i) place(k, i), load(i, ea, eb);
+    }
+    int ss = grp;  // the stage ring: slot and pass of the group's block
+    uint32_t su = 0;
+    while (ss >= S) ss -= S, ++su;
+    for (;;)
+    {
+        const int now = step;
+        step += G;
+        const int moved = settle();
+        if (moved < 0) return;
         if (su > 0 && !wait_bounded(&empty_bar[ss], (su - 1) & 1)) return;
         unsigned char *sA = smem + ss * stage_bytes;
         if (p == 0)
         {
             arrive_expect_tx(&full_bar[ss], uint32_t(b_bytes));
-            bulk_g2s(sA + a_bytes, P.wimg + int64_t(step) * b_bytes, uint32_t(b_bytes), &full_bar[ss]);
+            bulk_g2s(sA + a_bytes, P.wimg + int64_t(now) * b_bytes, uint32_t(b_bytes), &full_bar[ss]);
         }
         auto store = [&](int i) {
-            *reinterpret_cast<uint4 *>(a_row_chunk(sA, row0 + RS * i, kc)) =
-                make_uint4(spike_bytes(f[i].x, utt[i]), spike_bytes(f[i].y, utt[i]), spike_bytes(f[i].z, utt[i]),
-                           spike_bytes(f[i].w, utt[i]));
+            const uint4 m = make_uint4(spike_mask(f[i].x, utt[i]), spike_mask(f[i].y, utt[i]),
+                                       spike_mask(f[i].z, utt[i]), spike_mask(f[i].w, utt[i]));
+            unsigned char *c = a_row_chunk(sA, row0 + 32 * i, kc);
+            *reinterpret_cast<uint4 *>(c) = m;
+            *reinterpret_cast<uint4 *>(c + 4 * 128) =
+                make_uint4(m.x & 0x01010101u, m.y & 0x01010101u, m.z & 0x01010101u, m.w & 0x01010101u);
         };
-        if (++kb == P.kblocks) kb = 0;
-        const int4 ea = tab[kb * 16 + 2 * kc], eb = tab[kb * 16 + 2 * kc + 1];
-        if (!last)
+        int4 ea = make_int4(0, 0, 0, 0), eb = ea;
+        if (moved) chunk(ea, eb);
+        if (moved == 1)
         {
 #pragma unroll
             for (int i = 0; i < NU; ++i) store(i), load(i, ea, eb);
@@ -1639,14 +1677,14 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
             for (int i = 0; i < NU; ++i)
             {
                 store(i);
-                if (more) place(k, i), load(i, ea, eb);
+                if (moved) place(k, i), load(i, ea, eb);
             }
         }
         fence_proxy_async_smem();
         mbar_arrive(&full_bar[ss]);
-        if (++ss == S) ss = 0, ++su;
-        step = last ? 0 : step + 1;
-        if (!more) break;
+        if (!moved) break;
+        ss += G;
+        while (ss >= S) ss -= S, ++su;
     }
 }
 
@@ -1694,7 +1732,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
         nrows = (P.round == 0 && !P.r0_list) ? P.npix : int64_t(*P.count_in);
         ntiles = ceil_div(nrows, BM);
     }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int S = P.stages, nacc = P.nacc;
     const int a_bytes = BM * BK * 2;
     const int b_bytes = P.nsplit * P.n_tile * BK * 2;
@@ -1703,28 +1741,28 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     const int taps = P.kh * P.kw;
     // search: the channels' scales and bounds, staged after the table
     const int nch = MODE == kSearch ? P.nparts * P.n_tile : P.n_tile;  // channels of the tables
-    float *s_scale = reinterpret_cast<float *>(tab + P.kblocks * 16), *s_bound = s_scale + nch;
+    float *s_scale = reinterpret_cast<float *>(tab + P.kblocks * 8), *s_bound = s_scale + nch;
     // search: the channels' shifts to the common grid of the keys (nch is a
     // multiple of 16), two buffers of the tile's rows (128 each): places, steps
-    int *s_shift = reinterpret_cast<int *>(s_bound + nch);
+    float *s_cent = s_bound + nch;
+    int *s_shift = reinterpret_cast<int *>(s_cent + nch);
     int2 *s_row = reinterpret_cast<int2 *>(s_shift + nch);
     uint8_t *s_step = reinterpret_cast<uint8_t *>(s_row + 2 * BM);
     if constexpr (MODE == kSearch)
     {
-        // per 8-element group of a 128-element K block (channels-last, 8-bit
-        // operands): (byte offset from the receptive field's origin, ky, kx)
-        for (int g = tid; g < P.kblocks * 16; g += blockDim.x)
+        // per 8-input group of a 64-input K block (channels-last): (byte offset from the receptive field's origin, ky, kx)
+        for (int g = tid; g < P.kblocks * 8; g += blockDim.x)
         {
             const int k = g * 8, tap = k / P.cpad, c = k % P.cpad, ky = tap / P.kw, kx = tap % P.kw;
             tab[g] = (tap < taps && c < P.cin) ? make_int4((ky * P.w + kx) * P.cpad + c, ky, kx, 0)
                                                : make_int4(0, kNoRow, 0, 0);
         }
-        // cscale = 2^(e - 32), e the channel's exponent; sinfo[1] the largest e + 128
+        // cscale = 2^(e - 31), e the channel's exponent; sinfo[1] the largest e + 128
         for (int c = tid; c < nch; c += blockDim.x)
         {
             const float sc = P.cscale[c];
-            s_scale[c] = sc, s_bound[c] = P.echan[c];
-            const int e = int(__float_as_uint(sc) >> 23) - 127 + 8 * kSearchTerms;
+            s_scale[c] = sc, s_bound[c] = P.echan[c], s_cent[c] = P.ccent[c];
+            const int e = int(__float_as_uint(sc) >> 23) - 127 + kSearchBits;
             s_shift[c] = min(max(int(P.sinfo[1]) - 128 - e, 0), 31);
         }
     }
@@ -1762,7 +1800,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     if (tid == 0)
     {
         for (int s = 0; s < S; ++s)
-            mbar_init(&full_bar[s], 1 + 32 * NPW), mbar_init(&empty_bar[s], 1);
+            mbar_init(&full_bar[s], 1 + (MODE == kSearch ? 128 : 32 * NPW)), mbar_init(&empty_bar[s], 1);
         for (int a = 0; a < 2; ++a) mbar_init(&accf_bar[a], 1), mbar_init(&acce_bar[a], 128);
         mbar_init(&tim_bar, 128);
         for (int b = 0; b < 2; ++b) mbar_init(&ent_bar[b], 32 * NPW);
@@ -1783,13 +1821,12 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     constexpr int kMmaWarp = 4 + NPW;
     if (MODE == kSearch && warp >= 4 && warp < kMmaWarp)
     {
-        constexpr int NU = 1024 / (32 * NPW);
         if (P.cpad % 16 == 0 && (reinterpret_cast<uintptr_t>(P.in) & 15) == 0 && (P.img_stride & 15) == 0)
-            search_producer<NU, true>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128,
-                                      nrows, ntiles, s_row, s_step, ent_bar, s_tiles, tq_bar);
-        else
-            search_producer<NU, false>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128,
+            search_producer<NPW, true>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128,
                                        nrows, ntiles, s_row, s_step, ent_bar, s_tiles, tq_bar);
+        else
+            search_producer<NPW, false>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128,
+                                        nrows, ntiles, s_row, s_step, ent_bar, s_tiles, tq_bar);
     }
     else if (MODE != kPotentials && MODE != kSearch && warp >= 4 && warp < kMmaWarp)
     {
@@ -1860,11 +1897,34 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     else if (warp == kMmaWarp)
     {
         // ---------------- MMA issuer ----------------
-        if (lane == 0)
         {
-            uint32_t it = 0, j = 0, k = 0;
+            // The whole warp runs the loops, on values that are the same in
+            // every lane (votes and shuffles where the compiler cannot see
+            // it), and one elected lane issues: the instructions take their
+            // descriptors from uniform registers, and in a branch of one
+            // lane each of them was preceded by moves that cost more than the
+            // multiplication (K block of four MMAs of 64 columns: 830 cycles).
+            // Descriptors are offsets (in 16-byte units) from the first
+            // stage's; the rings' slots and passes count up.
+            const uint32_t utmem = __shfl_sync(0xffffffffu, tmem, 0);
+            const bool leader = elect_one();  // (the thread that issues also commits)
+            uint32_t j = 0, k = 0;
             bool failed = false;
             const int parts = MODE == kSearch ? P.nparts : 1;
+            const uint64_t desc0 = smem_desc(smem_u32(smem), 128, 1024);
+            const uint32_t stage16 = uint32_t(stage_bytes) >> 4, a16 = uint32_t(a_bytes) >> 4;
+            // The split terms' weight rows are stacked in one K-major B of
+            // nsplit * n_tile rows whose accumulators are adjacent: one MMA
+            // covers up to 256 of them, so the A tile is read once per 256
+            // columns, not once per term.
+            const int ncols = P.nsplit * P.n_tile, nlast = ncols - ((ncols - 1) & ~255);
+            const uint32_t ifull = MODE == kSearch ? idesc_u8_s32(BM, 256) : idesc_bf16_f32(BM, 256);
+            const uint32_t ilast = MODE == kSearch ? idesc_u8_s32(BM, nlast) : idesc_bf16_f32(BM, nlast);
+            // (search: steps 0, 1 are the inputs' 255s, 2, 3 their 1s; a last
+            // block of 32 inputs or fewer has the even ones only)
+            const int half = MODE == kSearch && P.kreal - (P.kblocks - 1) * BK <= 32 ? P.kblocks - 1 : -1;
+            int s = 0, a = 0;
+            uint32_t u = 0, ua = 0;  // passes of the stage and accumulator rings
             int64_t tile = blockIdx.x;
             // units (tile, part) in the CTA's order: the tiles stride by the
             // grid, or (search) come from the producers' ring
@@ -1875,8 +1935,8 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
                     // (after the last part of a tile) the next tile
                     if constexpr (MODE == kSearch)
                     {
-                        if (!wait_bounded(&tq_bar[k & 15], (k >> 4) & 1)) break;
-                        tile = s_tiles[k & 15];
+                        if (!__all_sync(0xffffffffu, wait_bounded(&tq_bar[k & 15], (k >> 4) & 1))) break;
+                        tile = __shfl_sync(0xffffffffu, s_tiles[k & 15], 0);
                         if (tile < 0) break;
                     }
                     else
@@ -1886,48 +1946,44 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
                     }
                 }
                 if (++part == parts) part = 0, ++k;
-                const int a = int(j % uint32_t(nacc));
-                const uint32_t ua = j / uint32_t(nacc);
-                if (ua > 0 && !wait_bounded(&acce_bar[a], (ua - 1) & 1)) break;
+                if (ua > 0 && !__all_sync(0xffffffffu, wait_bounded(&acce_bar[a], (ua - 1) & 1))) break;
                 tc_fence_after();
-                const uint32_t d = tmem + uint32_t(a * acc_cols);
-                for (int kb = 0; kb < P.kblocks; ++kb, ++it)
+                const uint32_t d = utmem + uint32_t(a * acc_cols);
+                for (int kb = 0; kb < P.kblocks; ++kb)
                 {
-                    const int s = int(it % uint32_t(S));
-                    const uint32_t u = it / uint32_t(S);
-                    if (!wait_bounded(&full_bar[s], u & 1))
+                    if (!__all_sync(0xffffffffu, wait_bounded(&full_bar[s], u & 1)))
                     {
                         failed = true;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t a_base = smem_u32(smem + s * stage_bytes);
-                    const uint32_t b_base = a_base + uint32_t(a_bytes);
-                    // The split terms' weight rows are stacked in one K-major
-                    // B of nsplit * n_tile rows whose accumulators are
-                    // adjacent: one MMA covers up to 256 of them, so the A
-                    // tile is read once per 256 columns, not once per term.
-                    const int ncols = P.nsplit * P.n_tile;
-                    for (int c = 0; c < ncols; c += 256)
+                    const uint64_t ad = desc0 + uint64_t(uint32_t(s) * stage16), bd = ad + a16;
+                    if (leader)
                     {
-                        const int n = ncols - c < 256 ? ncols - c : 256;
-                        // the same 32-byte steps of each 128-byte row: 16
-                        // BF16 or (search) 32 U8 elements per instruction
-                        const uint32_t idesc = MODE == kSearch ? idesc_u8_s32(BM, n) : idesc_bf16_f32(BM, n);
-#pragma unroll
-                        for (int k16 = 0; k16 < BK / 16; ++k16)
+                        for (int c = 0; c < ncols; c += 256)
                         {
-                            const uint64_t ad = smem_desc(a_base + k16 * 256, 128, 1024);
-                            const uint64_t bd = smem_desc(b_base + c * 128 + k16 * 256, 128, 1024);
-                            if constexpr (MODE == kSearch)
-                                mma_u8(d + uint32_t(c), ad, bd, idesc, (kb > 0 || k16 > 0) ? 1u : 0u);
-                            else
-                                mma_bf16(d + uint32_t(c), ad, bd, idesc, (kb > 0 || k16 > 0) ? 1u : 0u);
+                            const uint32_t idesc = ncols - c > 256 ? ifull : ilast;
+                            // the same 32-byte steps of each 128-byte row: 16 BF16
+                            // or 32 U8 elements per instruction
+#pragma unroll
+                            for (int k16 = 0; k16 < BK / 16; ++k16)
+                            {
+                                if (MODE == kSearch && (k16 & 1) && kb == half) continue;
+                                const uint32_t add = k16 > 0 ? 1u : (kb > 0 ? 1u : 0u);
+                                if constexpr (MODE == kSearch)
+                                    mma_u8(d + uint32_t(c), ad + k16 * 16, bd + c * 8 + k16 * 16, idesc, add);
+                                else
+                                    mma_bf16(d + uint32_t(c), ad + k16 * 16, bd + c * 8 + k16 * 16, idesc, add);
+                            }
                         }
+                        mma_commit(&empty_bar[s]);
                     }
-                    mma_commit(&empty_bar[s]);
+                    __syncwarp();
+                    if (++s == S) s = 0, ++u;
                 }
-                if (!failed) mma_commit(&accf_bar[a]);
+                if (!failed && leader) mma_commit(&accf_bar[a]);
+                __syncwarp();
+                if (++a == nacc) a = 0, ++ua;
             }
         }
         __syncwarp();
@@ -1938,16 +1994,16 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
         // warp w reads tensor-memory lanes 32 w .. 32 w + 31 (rows of the tile)
         const int row = (warp & 3) * 32 + lane;
         // the largest channel bound (search)
-        // and the grid of its keys: R < inputs 2^32, so `drop` bits fewer
+        // and the grid of its keys: R < inputs 2^31, so `drop` bits fewer
         // leave 31
         float emax = 0.f;
         double unit = 0.0;
-        int drop = 1;
+        int drop = 0;
         if constexpr (MODE == kSearch)
         {
             emax = __uint_as_float(P.sinfo[0]);
-            while ((1 << (drop - 1)) < P.cin * taps) ++drop;
-            unit = ldexp(1.0, drop + int(P.sinfo[1]) - 128 - 8 * kSearchTerms);
+            while ((1 << drop) < P.cin * taps) ++drop;
+            unit = ldexp(1.0, drop + int(P.sinfo[1]) - 128 - kSearchBits);
         }
         uint32_t j = 0, k = 0;
         const int parts = MODE == kSearch ? P.nparts : 1;
@@ -2027,9 +2083,15 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
             else if constexpr (MODE == kSearch)
             {
                 if (part == 0) scan = SearchScan{};
-                search_epilogue<kSearchTerms>(P, acc, s_ok, s_e.x, s_e.y, P.round == 2 ? s_aux : 0, s_st,
-                                              &acce_bar[a], emax, unit, drop, s_scale, s_bound, s_shift, int(tile * BM + row),
-                                              part, scan);
+                auto epilogue = [&](auto multi) {
+                    search_epilogue<kSearchTerms, multi.value>(
+                        P, acc, s_ok, s_e.x, s_e.y, P.round == 2 ? s_aux : 0, s_st, &acce_bar[a], emax, unit, drop,
+                        s_scale, s_bound, s_cent, s_shift, int(tile * BM + row), part, scan);
+                };
+                if (parts == 1)
+                    epilogue(std::false_type());
+                else
+                    epilogue(std::true_type());
             }
             else if constexpr (MODE == kFused)
             {
@@ -2218,32 +2280,37 @@ __global__ void __launch_bounds__(128) wta_records_warp_kernel(const int4 *__res
 }
 
 // ---- search path: weight split, exact recompute, outputs ---------------------
-// Split of output channel n's weights into NS base-256 digits (one CTA per
-// channel of the padded tile).  With 2^e the smallest power of two above the
-// channel's largest weight (e clamped to [-94, 100]), w = 2^e sum_j d_j
-// 256^-(j+1) + rem, digits d_j in [0, 255] (floor), 0 <= rem < 2^(e - 8 NS).
-// A 0/1 spike times a digit is an exact 8-bit product and the tensor core's
-// 32-bit integer sums are exact, so the row's term total R (an integer) times
-// cscale[n] = 2^(e - 8 NS) is the potential of the digit weights exactly.
-// echan[n] bounds |oracle - R cscale| for any 0/1 input: the sum of the
-// remainders (zero when every weight lies on the 2^(e - 8 NS) grid) plus,
+// Split of output channel n's weights into 31-bit integers (one CTA per channel
+// of the padded tile).  With 2^e a power of two above the channel's largest
+// weight (the smallest whose upper field fits; e clamped to [-94, 101]), w =
+// 2^e (hi 2^-16 + lo 2^-31) + rem, hi <= 65280 = 255 255 + 255, lo < 2^15, 0 <=
+// rem < 2^(e - 31).  Each field is 255 a + b with 8-bit a, b: the operand's two
+// halves, which meet 255 and 1 where an input has fired (search_producer), so
+// one 32-bit accumulator sums a whole field and a channel takes two columns of
+// tensor memory instead of four base-256 digits' (a second accumulator then
+// fits for up to 128 channels, and the scan of a tile runs beside the next
+// tile's multiplications).  All sums are exact integers, and the row's term
+// total R times cscale[n] = 2^(e - 31) is the potential of the split weights
+// exactly.  The remainders of a row sum to [0, err], err the sum of all of the
+// channel's (zero when every weight lies on the 2^(e - 31) grid), so the
+// oracle is within echan[n] of R cscale[n] + ccent[n]: about half of err plus,
 // unless the oracle's ordered FP64 sum is exact for these weights, K^2
-// 2^(e-52).  Negative weights only raise *negw (the search then stands down).
-// The operand layout is split_weights_kernel's, with 16 U8 elements per
-// 16-byte chunk (128 per K block), K in channels-last order.
-template <int NS>
+// 2^(e-52).  sinfo[0]: the largest bound on oracle - R cscale.  Negative
+// weights and those of 1e30 or more (NaN too) only raise *negw (the search then
+// stands down).  K in channels-last order, 64 inputs per block.
 __global__ void __launch_bounds__(256) fixed_split_kernel(const float *__restrict__ kernel, uint4 *__restrict__ wimg,
                                                           int cout, int cin, int taps, int cpad, int kblocks,
                                                           int n_tile, float *__restrict__ echan,
-                                                          float *__restrict__ cscale, unsigned *__restrict__ sinfo,
-                                                          int *__restrict__ negw, unsigned *__restrict__ wmax)
+                                                          float *__restrict__ cscale, float *__restrict__ ccent,
+                                                          unsigned *__restrict__ sinfo, int *__restrict__ negw,
+                                                          unsigned *__restrict__ wmax)
 {
     __shared__ float s_mx[8];
     __shared__ double s_err[8];
     __shared__ int s_lsb[8];
     const int n = blockIdx.x, tid = threadIdx.x;
     const int kreal = taps * cpad;
-    const int K = kblocks * 2 * BK;
+    const int K = kblocks * BK;
     auto weight = [&](int k) -> float {
         if (n >= cout || k >= kreal) return 0.f;
         const int tap = k / cpad, c = k % cpad;
@@ -2256,7 +2323,7 @@ __global__ void __launch_bounds__(256) fixed_split_kernel(const float *__restric
     {
         const float w = weight(k);
         mx = fmaxf(mx, fabsf(w));
-        neg |= !(w >= 0.f);
+        neg |= !(w >= 0.f && w < 1e30f);
         if (wmax && n < cout && k < kreal && w > 0.f)
         {
             // largest weight of each input over the channels (oracle layout)
@@ -2284,41 +2351,42 @@ __global__ void __launch_bounds__(256) fixed_split_kernel(const float *__restric
     if (mx > 0.f)
     {
         int ex;
-        frexpf(mx, &ex);  // mx = fr 2^ex, fr in [0.5, 1): mx < 2^ex
-        e = ex;
+        const float fr = frexpf(mx, &ex);  // mx = fr 2^ex, fr in [0.5, 1): mx < 2^ex
+        e = fr * 65536.f > 65280.f ? ex + 1 : ex;
     }
-    e = max(-94, min(100, e));
+    e = max(-94, min(101, e));
     double err = 0.0;
-    for (int i = tid; i < kblocks * 8; i += blockDim.x)
+    for (int i = tid; i < kblocks * 4; i += blockDim.x)
     {
-        const int kb = i / 8, kc = i % 8;
-        uint32_t parts[NS][4];
+        const int kb = i / 4, kc = i % 4;
+        uint32_t parts[2][2][4];  // [field][a, b][16 inputs]
 #pragma unroll
-        for (int j = 0; j < NS; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) parts[j][q] = 0u;
+        for (int j = 0; j < 16; ++j) parts[j >> 3][(j >> 2) & 1][j & 3] = 0u;
 #pragma unroll
         for (int e16 = 0; e16 < 16; ++e16)
         {
-            const double w = fmax(double(weight(kb * 2 * BK + kc * 16 + e16)), 0.0);
-            double r = ldexp(w, -e);  // in [0, 1)
+            const double r = ldexp(fmax(double(weight(kb * BK + kc * 16 + e16)), 0.0), 16 - e);
+            const double hi = floor(r), low = (r - hi) * double(1 << kLowBits), lo = floor(low);
+            err += ldexp(low - lo, e - kSearchBits);
+            const uint32_t field[2] = {uint32_t(fmin(hi, 65280.0)), uint32_t(lo)};
 #pragma unroll
-            for (int j = 0; j < NS; ++j)
+            for (int j = 0; j < 2; ++j)
             {
-                const double d = floor(r * 256.0);
-                r = r * 256.0 - d;
-                parts[j][e16 >> 2] |= uint32_t(d) << (8 * (e16 & 3));
+                const uint32_t a = min(field[j] / 255u, 255u);
+                parts[j][0][e16 >> 2] |= a << (8 * (e16 & 3));
+                parts[j][1][e16 >> 2] |= (field[j] - 255u * a) << (8 * (e16 & 3));
             }
-            err += ldexp(r, e - 8 * NS);
         }
 #pragma unroll
-        for (int j = 0; j < NS; ++j)
+        for (int j = 0; j < 2; ++j)
         {
             // part n / n_tile of the channels, row n % n_tile within it
             const int part = n / n_tile, nl = n % n_tile;
-            const int64_t idx = ((int64_t(part) * kblocks + kb) * NS + j) * (int64_t(n_tile) * 8) + (nl / 8) * 64 +
-                                kc * 8 + (nl % 8);
-            wimg[idx] = make_uint4(parts[j][0], parts[j][1], parts[j][2], parts[j][3]);
+            const int64_t idx =
+                ((int64_t(part) * kblocks + kb) * 2 + j) * (int64_t(n_tile) * 8) + (nl / 8) * 64 + kc * 8 + (nl % 8);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                wimg[idx + q * 32] = make_uint4(parts[j][q][0], parts[j][q][1], parts[j][q][2], parts[j][q][3]);
         }
     }
     for (int o = 16; o > 0; o >>= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
@@ -2334,13 +2402,16 @@ __global__ void __launch_bounds__(256) fixed_split_kernel(const float *__restric
         int lk = 0;
         while ((1 << lk) < kreal) ++lk;
         const bool exact64 = lsb == INT_MAX || e + lk - lsb <= 53;
-        const double bound = err + (exact64 ? 0.0 : double(kreal) * double(kreal) * ldexp(1.0, e - 52));
-        const float eb = __double2float_ru(bound);
-        echan[n] = eb;
-        cscale[n] = ldexpf(1.f, e - 8 * NS);
+        const double fp = exact64 ? 0.0 : double(kreal) * double(kreal) * ldexp(1.0, e - 52);
+        const float cent = float(0.5 * err);
+        // (and the rounding of the middle's FP64 sum)
+        const double half = err > 0.0 ? fmax(double(cent), err - double(cent)) + double(kreal) * ldexp(1.0, e - 52) : 0.0;
+        echan[n] = __double2float_ru(half + fp);
+        ccent[n] = cent;
+        cscale[n] = ldexpf(1.f, e - kSearchBits);
         if (n < cout)
         {
-            atomicMax(sinfo + 0, __float_as_uint(eb));
+            atomicMax(sinfo + 0, __float_as_uint(__double2float_ru(err + fp)));
             atomicMax(sinfo + 1, unsigned(e + 128));
         }
     }
@@ -2816,8 +2887,9 @@ Plan make_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64
     pl.n_tile = int(ceil_div(ceil_div(npad, pl.n_tiles), 16) * 16);
     if (nsplit > 0)
     {
-        // search: the channels in parts whose accumulators fit the tensor memory
-        while (int64_t(pl.nsplit) * ceil_div(ceil_div(npad, pl.parts), 16) * 16 > 512) ++pl.parts;
+        // search: the channels in parts of which two accumulators fit the
+        // tensor memory
+        while (int64_t(pl.nsplit) * ceil_div(ceil_div(npad, pl.parts), 16) * 16 > 256) ++pl.parts;
         pl.n_tile = int(ceil_div(ceil_div(npad, pl.parts), 16) * 16);
     }
     // channels-last from 8 input channels, and always where the fused layer
@@ -2825,9 +2897,8 @@ Plan make_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64
     pl.nhwc = cin >= 8 || cl || nsplit > 0;
     pl.cpad = int(ceil_div(cin, 8) * 8);
     const int64_t kreal = pl.nhwc ? kh * kw * pl.cpad : kh * kw * cin;
-    // search plans (nsplit given): 8-bit operands, 128 elements per K block
-    // in the same 128-byte rows
-    pl.kblocks = int(ceil_div(kreal, nsplit > 0 ? 2 * BK : BK));
+    // (search plans: 8-bit operands, each input twice in the 128-byte rows)
+    pl.kblocks = int(ceil_div(kreal, BK));
     // two accumulators (the epilogue of one tile overlaps the MMAs of the
     // next) when they fit in the 512 tensor-memory columns
     const uint32_t acc_cols = uint32_t(pl.nsplit * pl.n_tile);
@@ -2845,9 +2916,9 @@ Plan make_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64
         pl.xt_bytes = pl.nhwc ? size_t(n) * h * w * pl.cpad : 0;
     // (kTimes: the table is followed by the per-warp first-step candidates,
     // two buffers of 4 warps x n_tile ints)
-    // (search: 16 group entries per K block, the channels' scales, bounds and
-    // shifts and two buffers of tile rows)
-    const size_t tab = nsplit > 0   ? size_t(pl.kblocks) * 256 + size_t(pl.parts) * pl.n_tile * 12 + 2 * BM * 9
+    // (search: 8 group entries per K block, the channels' scales, bounds,
+    // middles and shifts and two buffers of tile rows)
+    const size_t tab = nsplit > 0   ? size_t(pl.kblocks) * 128 + size_t(pl.parts) * pl.n_tile * 16 + 2 * BM * 9
                        : t_fused > 0 ? (size_t(pl.kblocks) * BK + 8) * 16 + (times ? size_t(pl.n_tile) * 32 : 0)
                        : !pl.nhwc   ? size_t(pl.kblocks) * BK * 16
                                     : size_t(pl.kblocks) * 8 * 16;
@@ -2855,7 +2926,7 @@ Plan make_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64
     // the search kernel aims at two CTAs per SM where its tensor memory allows
     const bool two = nsplit > 0 && cols <= 256;
     const size_t budget = (two ? 110 * 1024 : 225 * 1024) - tab;
-    pl.stages = int(std::min<size_t>(g_schedule.stages > 0 ? size_t(g_schedule.stages) : 4, budget / stage));
+    pl.stages = int(std::min<size_t>(g_schedule.stages > 0 ? size_t(g_schedule.stages) : (nsplit > 0 ? 5 : 4), budget / stage));
     size_t smem = size_t(pl.stages) * stage + tab;
     // At most 512 / tmem_cols CTAs may share an SM's tensor memory: size the
     // shared memory so that no more fit.
@@ -3219,13 +3290,13 @@ FusedLayout fused_layout(int64_t b, int64_t t, int64_t cin, int64_t h, int64_t w
     L.pl4 = make_plan(b * t, cin, h, w, cout, kh, kw, precision, true, t, false, kSearchTerms);
     L.search_ok = nnets == 1 && t <= 127 && L.pl4.n_tiles == 1 && L.pl4.parts <= 8 &&
                   L.pl4.nsplit * L.pl4.n_tile <= 512 &&
-                  L.pl4.stages >= 2 && L.pl4.smem <= 227 * 1024 && L.pl4.kblocks <= kMaxKBlocks &&
+                  L.pl4.stages >= 2 && L.pl4.smem <= 227 * 1024 && L.pl4.kblocks <= 2 * kMaxKBlocks &&
                   L.pl.xt_bytes < (size_t(1) << 31) && h < 30000 && w < 30000;
     if (L.search_ok)
     {
         const size_t np = size_t(L.npix);
         L.w4_off = off, off += align256(L.pl4.wimg_bytes);
-        L.echan_off = off, off += align256(size_t(L.pl4.parts) * L.pl4.n_tile * 8 + 8);
+        L.echan_off = off, off += align256(size_t(L.pl4.parts) * L.pl4.n_tile * 12 + 8);
         L.wm_off = off, off += align256(size_t(cin * kh * kw) * 4);
         // 64 counters, then two buffers of per-block entry counts of the list
         // compaction (zeroed together)
@@ -3396,11 +3467,12 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
     const int nch = pl.parts * pl.n_tile;
     float *echan = reinterpret_cast<float *>(base + L.echan_off);
     float *cscale = echan + nch;
-    unsigned *sinfo = reinterpret_cast<unsigned *>(cscale + nch);
+    float *ccent = cscale + nch;
+    unsigned *sinfo = reinterpret_cast<unsigned *>(ccent + nch);
     P.nparts = pl.parts;
     P.cscale = cscale;
     int *cnt = reinterpret_cast<int *>(base + L.cnt_off);
-    P.echan = echan, P.sinfo = sinfo;
+    P.echan = echan, P.ccent = ccent, P.sinfo = sinfo;
     P.state = reinterpret_cast<int4 *>(base + L.state_off);
     int2 *la = reinterpret_cast<int2 *>(base + L.la_off), *lb = reinterpret_cast<int2 *>(base + L.lb_off);
     int4 *fa = reinterpret_cast<int4 *>(base + L.fa_off), *fb = reinterpret_cast<int4 *>(base + L.fb_off);
@@ -3458,9 +3530,9 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
     SPK_CUDA(cudaMemsetAsync(cnt, 0, 256 + 2 * bcn * 4, s));
     SPK_CUDA(cudaMemsetAsync(sinfo, 0, 8, s));
     if (prefilter) SPK_CUDA(cudaMemsetAsync(wmax, 0, size_t(kr) * 4, s));
-    fixed_split_kernel<kSearchTerms><<<unsigned(nch), 256, 0, s>>>(
+    fixed_split_kernel<<<unsigned(nch), 256, 0, s>>>(
         kernel, reinterpret_cast<uint4 *>(base + L.w4_off), P.cout, P.cin, taps, P.cpad, pl.kblocks, pl.n_tile, echan,
-        cscale, sinfo, P.negw, prefilter ? wmax : nullptr);
+        cscale, ccent, sinfo, P.negw, prefilter ? wmax : nullptr);
     SPK_LAUNCHED();
     if (count > 0)
     {

@@ -30,6 +30,13 @@
 // the walk the kernel kept a stack and spilled: 60 us instead of 46, and a
 // graph of the launches took 95 to 1300 ms to instantiate instead of 26.
 
+// Bytes 1 where the first-spike byte f <= t, else 0; tt = (t + 1) * 0x01010101
+// ((f | 0x80) - (t + 1) keeps bit 7 iff f > t, no borrow between bytes).
+__device__ __forceinline__ uint32_t spike_bytes(uint32_t f, uint32_t tt)
+{
+    return (~((f | 0x80808080u) - tt) >> 7) & 0x01010101u;
+}
+
 // wd[k][cz]: the integers of input k (channels-last order, `kreal` of them)
 // and channel n, echan / cscale as fixed_split_kernel's, the layer's largest
 // weight to *wmax.  A CTA per channel.

@@ -11,6 +11,14 @@ namespace spk
 {
 namespace tc
 {
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
