@@ -807,7 +807,8 @@ __device__ __forceinline__ RowInfo row_info(const TcParams &P, int64_t mt, int r
     return r;
 }
 
-// Raw bytes of four 8-wide K chunks of one A row (loads in flight until used).
+// Raw bytes of four 8-wide K chunks of one A row (loads in flight until used),
+// of channel-major spikes (one input channel).
 struct Gathered
 {
     uint2 v[4];
@@ -817,36 +818,21 @@ template <typename RI>
 __device__ __forceinline__ void gather_load(const TcParams &P, const int4 *tab, const RI &r, const uint8_t *ib, int kb,
                                             int c_lo, Gathered &g)
 {
-    if (P.nhwc)
+    const int64_t rowoff = int64_t(r.iy0) * P.rs + int64_t(r.ix0) * P.ps;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
     {
+        uint32_t w[2] = {0, 0};
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int e = 0; e < 8; ++e)
         {
-            const int4 t = tab[kb * 8 + c_lo + j];
-            const int iy = r.iy0 + t.x, ix = r.ix0 + t.y;
-            g.v[j] = make_uint2(0, 0);
-            if (r.ok && t.w && iy >= 0 && iy < P.h && ix >= 0 && ix < P.w)
-                g.v[j] = *reinterpret_cast<const uint2 *>(ib + int64_t(iy) * P.rs + int64_t(ix) * P.ps + t.z);
+            const int4 t = tab[kb * BK + (c_lo + j) * 8 + e];
+            const int iy = r.iy0 + t.y, ix = r.ix0 + t.z;
+            uint32_t b8 = 0;
+            if (r.ok && t.w && iy >= 0 && iy < P.h && ix >= 0 && ix < P.w) b8 = ib[rowoff + t.x];
+            w[e >> 2] |= b8 << (8 * (e & 3));
         }
-    }
-    else
-    {
-        const int64_t rowoff = int64_t(r.iy0) * P.rs + int64_t(r.ix0) * P.ps;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-        {
-            uint32_t w[2] = {0, 0};
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-            {
-                const int4 t = tab[kb * BK + (c_lo + j) * 8 + e];
-                const int iy = r.iy0 + t.y, ix = r.ix0 + t.z;
-                uint32_t b8 = 0;
-                if (r.ok && t.w && iy >= 0 && iy < P.h && ix >= 0 && ix < P.w) b8 = ib[rowoff + t.x];
-                w[e >> 2] |= b8 << (8 * (e & 3));
-            }
-            g.v[j] = make_uint2(w[0], w[1]);
-        }
+        g.v[j] = make_uint2(w[0], w[1]);
     }
 }
 
@@ -854,6 +840,151 @@ __device__ __forceinline__ void gather_store(const TcParams &, const Gathered &g
 {
 #pragma unroll
     for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4 *>(a + (c_lo + j) * 128) = bf16x8_of_bytes(g.v[j]);
+}
+
+// 16-byte chunk kc of row r of an operand tile.
+__device__ __forceinline__ unsigned char *a_row_chunk(unsigned char *sA, int r, int kc)
+{
+    return sA + (r >> 3) * 1024 + (r & 7) * 16 + kc * 128;
+}
+
+// 8 or 16 bytes, every word FILL where !ok (a predicated load: no branch, so
+// the loads of all units of a step are in flight together).
+template <int FILL>
+__device__ __forceinline__ uint2 ldg8_if(const uint8_t *p, bool ok)
+{
+    uint2 r;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.b32 %0, %4;\n\tmov.b32 %1, %4;\n\t"
+        "@p ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t}"
+        : "=&r"(r.x), "=&r"(r.y)
+        : "l"(p), "r"(uint32_t(ok)), "n"(FILL));
+    return r;
+}
+template <int FILL>
+__device__ __forceinline__ uint4 ldg16_if(const uint8_t *p, bool ok)
+{
+    uint4 r;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.b32 %0, %6;\n\tmov.b32 %1, %6;\n\tmov.b32 %2, %6;\n\t"
+        "mov.b32 %3, %6;\n\t@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w)
+        : "l"(p), "r"(uint32_t(ok)), "n"(FILL));
+    return r;
+}
+
+constexpr int kNoRow = 1 << 28;  // a row coordinate outside every input
+
+// Producers of the potentials from channels-last spikes.  The warps form groups
+// of four that take the 64-input K blocks in turn; a thread builds four (row,
+// 16-input chunk) units of its group's block: rows (p & 7) + 8 (p >> 5) + 32 i
+// of chunk (p >> 3) & 3, so the 8 lanes of a quarter warp store 8 consecutive
+// rows of one chunk (distinct 16-byte bank groups).  A unit's bytes are loaded
+// one block of the group ahead, right after the unit's block before it is
+// stored.  The rows' places (byte offset and coordinates of the receptive
+// field's origin) are worked out once per row by the first 128 threads and
+// handed over in shared memory (two buffers by tile parity).  WIDE: 16 channels
+// in one load (cpad a multiple of 16).
+//
+// The producers bound these convolutions: all eight warps on each K block, with
+// 64-bit addresses and branches around the loads, took 1400 .. 1500 cycles a
+// block against 700 for its multiplications (250 -> 200 maps 5 x 5).
+template <int NPW, bool WIDE>
+__device__ __forceinline__ void potentials_producer(const TcParams &P, const int4 *tab, unsigned char *smem,
+                                                    uint64_t *full_bar, uint64_t *empty_bar, int S, int stage_bytes,
+                                                    int a_bytes, int b_bytes, int tid, int4 *s_row, uint64_t *ent_bar)
+{
+    constexpr int G = NPW / 4, NU = 4;
+    static_assert(NPW % 4 == 0 && BM == 128, "a thread per row");
+    const int p = tid & 127, grp = tid >> 7;
+    const int row0 = (p & 7) + 8 * (p >> 5), kc = (p >> 3) & 3;
+    int64_t tile = blockIdx.x;
+    if (tile >= P.tiles) return;
+    auto setup = [&](uint32_t k) -> bool {
+        const int cb = int(k & 1);
+        if (grp == 0)
+        {
+            const RowInfo r = row_info<kPotentials>(P, tile / P.n_tiles, p);
+            const int64_t off = r.ok ? r.img * P.img_stride + (int64_t(r.iy0) * P.w + r.ix0) * P.cpad : 0;
+            s_row[cb * BM + p] = make_int4(int(uint32_t(off)), int(off >> 32), r.ok ? r.iy0 : kNoRow, r.ix0);
+        }
+        mbar_arrive(&ent_bar[cb]);
+        return wait_bounded(&ent_bar[cb], (k >> 1) & 1);
+    };
+    const uint8_t *ubase[NU];
+    int uy[NU], ux[NU];
+    uint4 f[NU];
+    auto place = [&](uint32_t k, int i) {
+        const int4 e = s_row[int(k & 1) * BM + row0 + 32 * i];
+        ubase[i] = P.in + ((int64_t(e.y) << 32) | uint32_t(e.x)), uy[i] = e.z, ux[i] = e.w;
+    };
+    // the chunk's bytes of unit i; ea, eb: its two groups' table entries
+    // (byte offset from the origin, ky, kx)
+    auto load = [&](int i, const int4 &ea, const int4 &eb) {
+        const bool oka = uint32_t(uy[i] + ea.y) < uint32_t(P.h) && uint32_t(ux[i] + ea.z) < uint32_t(P.w);
+        if constexpr (WIDE)
+            f[i] = ldg16_if<0>(ubase[i] + ea.x, oka);
+        else
+        {
+            const bool okb = uint32_t(uy[i] + eb.y) < uint32_t(P.h) && uint32_t(ux[i] + eb.z) < uint32_t(P.w);
+            const uint2 a = ldg8_if<0>(ubase[i] + ea.x, oka), b = ldg8_if<0>(ubase[i] + eb.x, okb);
+            f[i] = make_uint4(a.x, a.y, b.x, b.y);
+        }
+    };
+    uint32_t k = 0;
+    int step = grp;
+    if (!setup(0)) return;
+    // to the group's next block: 1 same tile, 2 a later one, 0 none left, -1 gave up
+    auto settle = [&]() -> int {
+        int moved = 1;
+        while (step >= P.kblocks)
+        {
+            if (tile + gridDim.x >= P.tiles) return 0;
+            tile += gridDim.x, step -= P.kblocks, moved = 2;
+            if (!setup(++k)) return -1;
+        }
+        return moved;
+    };
+    if (settle() <= 0) return;
+    {
+        const int4 ea = tab[step * 8 + 2 * kc], eb = tab[step * 8 + 2 * kc + 1];
+#pragma unroll
+        for (int i = 0; i < NU; ++i) place(k, i), load(i, ea, eb);
+    }
+    int ss = grp;  // the stage ring: slot and pass of the group's block
+    uint32_t su = 0;
+    while (ss >= S) ss -= S, ++su;
+    for (;;)
+    {
+        const int64_t now = (P.n_tiles > 1 ? tile % P.n_tiles : 0) * P.kblocks + step;  // the weights' block
+        step += G;
+        const int moved = settle();
+        if (moved < 0) return;
+        if (su > 0 && !wait_bounded(&empty_bar[ss], (su - 1) & 1)) return;
+        unsigned char *sA = smem + ss * stage_bytes;
+        if (p == 0)
+        {
+            arrive_expect_tx(&full_bar[ss], uint32_t(b_bytes));
+            bulk_g2s(sA + a_bytes, P.wimg + now * b_bytes, uint32_t(b_bytes), &full_bar[ss]);
+        }
+        auto store = [&](int i) {
+            unsigned char *c = a_row_chunk(sA, row0 + 32 * i, 2 * kc);
+            *reinterpret_cast<uint4 *>(c) = bf16x8_of_bytes(make_uint2(f[i].x, f[i].y));
+            *reinterpret_cast<uint4 *>(c + 128) = bf16x8_of_bytes(make_uint2(f[i].z, f[i].w));
+        };
+        int4 ea = make_int4(0, 0, 0, 0), eb = ea;
+        if (moved) ea = tab[step * 8 + 2 * kc], eb = tab[step * 8 + 2 * kc + 1];
+#pragma unroll
+        for (int i = 0; i < NU; ++i)
+        {
+            store(i);
+            if (moved == 2) place(k, i);
+            if (moved) load(i, ea, eb);
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(&full_bar[ss]);
+        if (!moved) break;
+        ss += G;
+        while (ss >= S) ss -= S, ++su;
+    }
 }
 
 // ---- fused producers ---------------------------------------------------------
@@ -919,11 +1050,6 @@ __device__ __forceinline__ uint2 fst_chunk(const TcParams &P, const int4 *tab, c
         w[i >> 2] |= b << (8 * (i & 3));
     }
     return make_uint2(w[0], w[1]);
-}
-
-__device__ __forceinline__ unsigned char *a_row_chunk(unsigned char *sA, int r, int kc)
-{
-    return sA + (r >> 3) * 1024 + (r & 7) * 16 + kc * 128;
 }
 
 // Rows t0 .. t0+R-1: byte b of the chunk is 1 where first-spike[b] <= t.
@@ -1485,27 +1611,6 @@ __device__ __forceinline__ uint32_t spike_mask(uint32_t f, uint32_t tt)
     return r;
 }
 
-// 8 or 16 bytes of a first-spike map, 0xFF where !ok (a predicated load: no
-// branch, so the loads of all units of a step are in flight together).
-__device__ __forceinline__ uint2 fst_ldg8(const uint8_t *p, bool ok)
-{
-    uint2 r;
-    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.b32 %0, -1;\n\tmov.b32 %1, -1;\n\t"
-        "@p ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t}"
-        : "=&r"(r.x), "=&r"(r.y)
-        : "l"(p), "r"(uint32_t(ok)));
-    return r;
-}
-__device__ __forceinline__ uint4 fst_ldg16(const uint8_t *p, bool ok)
-{
-    uint4 r;
-    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.b32 %0, -1;\n\tmov.b32 %1, -1;\n\tmov.b32 %2, -1;\n\t"
-        "mov.b32 %3, -1;\n\t@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
-        : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w)
-        : "l"(p), "r"(uint32_t(ok)));
-    return r;
-}
-
 // Search producers.  A K block is 64 inputs, each twice in a row's 128 bytes:
 // chunks 0 .. 3 hold 255 where the input has fired by the row's step (they
 // meet the multiples of 255 of the weights' fields, fixed_split_kernel),
@@ -1523,7 +1628,6 @@ __device__ __forceinline__ uint4 fst_ldg16(const uint8_t *p, bool ok)
 // WIDE: 16 channels of a chunk in one load (cpad a multiple of 16).  With
 // branches around each load, which kept two of them in flight, the producers
 // of a tile of 100 channels and 800 inputs took 18,000 cycles.
-constexpr int kNoRow = 1 << 28;  // a row coordinate outside every input
 template <int NPW, bool WIDE>
 __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *tab, unsigned char *smem,
                                                 uint64_t *full_bar, uint64_t *empty_bar, int S, int stage_bytes,
@@ -1602,12 +1706,12 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
     auto load = [&](int i, const int4 &ea, const int4 &eb) {
         const bool oka = uint32_t(uy[i] + ea.y) < uint32_t(P.h) && uint32_t(ux[i] + ea.z) < uint32_t(P.w);
         if constexpr (WIDE)
-            f[i] = fst_ldg16(P.in + int64_t(ubase[i] + ea.x), oka);
+            f[i] = ldg16_if<-1>(P.in + int64_t(ubase[i] + ea.x), oka);
         else
         {
             const bool okb = uint32_t(uy[i] + eb.y) < uint32_t(P.h) && uint32_t(ux[i] + eb.z) < uint32_t(P.w);
-            const uint2 a = fst_ldg8(P.in + int64_t(ubase[i] + ea.x), oka);
-            const uint2 b = fst_ldg8(P.in + int64_t(ubase[i] + eb.x), okb);
+            const uint2 a = ldg8_if<-1>(P.in + int64_t(ubase[i] + ea.x), oka);
+            const uint2 b = ldg8_if<-1>(P.in + int64_t(ubase[i] + eb.x), okb);
             f[i] = make_uint4(a.x, a.y, b.x, b.y);
         }
     };
@@ -1782,11 +1886,13 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     }
     else if (P.nhwc)
     {
+        // per 8-input group (channels-last): (byte offset from the receptive
+        // field's origin, ky, kx)
         const int groups = P.cpad / 8;
         for (int q = tid; q < P.kblocks * 8; q += blockDim.x)
         {
-            const int tap = q / groups, g = q % groups;
-            tab[q] = make_int4(tap / P.kw, tap % P.kw, g * 8, tap < taps ? 1 : 0);
+            const int tap = q / groups, g = q % groups, ky = tap / P.kw, kx = tap % P.kw;
+            tab[q] = tap < taps ? make_int4((ky * P.w + kx) * P.cpad + g * 8, ky, kx, 0) : make_int4(0, kNoRow, 0, 0);
         }
     }
     else
@@ -1800,7 +1906,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     if (tid == 0)
     {
         for (int s = 0; s < S; ++s)
-            mbar_init(&full_bar[s], 1 + (MODE == kSearch ? 128 : 32 * NPW)), mbar_init(&empty_bar[s], 1);
+            mbar_init(&full_bar[s], 1 + (MODE == kSearch || (MODE == kPotentials && P.nhwc) ? 128 : 32 * NPW)), mbar_init(&empty_bar[s], 1);
         for (int a = 0; a < 2; ++a) mbar_init(&accf_bar[a], 1), mbar_init(&acce_bar[a], 128);
         mbar_init(&tim_bar, 128);
         for (int b = 0; b < 2; ++b) mbar_init(&ent_bar[b], 32 * NPW);
@@ -1835,6 +1941,16 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
             fused_producer<1>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128);
         else
             fused_producer<4>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes, tid - 128);
+    }
+    else if (MODE == kPotentials && P.nhwc && warp >= 4 && warp < kMmaWarp)
+    {
+        int4 *s_place = tab + P.kblocks * 8;  // two buffers of the tile's rows
+        if (P.cpad % 16 == 0 && (reinterpret_cast<uintptr_t>(P.in) & 15) == 0)
+            potentials_producer<NPW, true>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes,
+                                           tid - 128, s_place, ent_bar);
+        else
+            potentials_producer<NPW, false>(P, tab, smem, full_bar, empty_bar, S, stage_bytes, a_bytes, b_bytes,
+                                            tid - 128, s_place, ent_bar);
     }
     else if (MODE == kPotentials && warp >= 4 && warp < kMmaWarp)
     {
@@ -2921,7 +3037,7 @@ Plan make_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64
     const size_t tab = nsplit > 0   ? size_t(pl.kblocks) * 128 + size_t(pl.parts) * pl.n_tile * 16 + 2 * BM * 9
                        : t_fused > 0 ? (size_t(pl.kblocks) * BK + 8) * 16 + (times ? size_t(pl.n_tile) * 32 : 0)
                        : !pl.nhwc   ? size_t(pl.kblocks) * BK * 16
-                                    : size_t(pl.kblocks) * 8 * 16;
+                                    : size_t(pl.kblocks) * 8 * 16 + 2 * BM * 16;
     const size_t stage = size_t(BM * BK * 2) + size_t(pl.nsplit) * pl.n_tile * BK * 2;
     // the search kernel aims at two CTAs per SM where its tensor memory allows
     const bool two = nsplit > 0 && cols <= 256;
