@@ -407,11 +407,14 @@ __device__ __forceinline__ float sum_terms(float h, float m, float l)
     return r;
 }
 
-// Potentials of one row and N tile: the accumulators in chunks of 8 columns,
-// the next chunk on its way while one is summed and stored.
+// Potentials of one row and channels [first, end) of an N tile (multiples of
+// 16): the accumulators in chunks of 8 columns, the next chunk on its way while
+// one is summed and stored.
 template <int NS>
-__device__ __forceinline__ void potentials_epilogue(const TcParams &P, uint32_t lane_base, bool ok, float *out, int n)
+__device__ __forceinline__ void potentials_epilogue(const TcParams &P, uint32_t lane_base, bool ok, float *out, int n,
+                                                    int first, int end)
 {
+    if (first >= end) return;
     uint32_t qa[3][kEpiChunk], qb[3][kEpiChunk];
     auto put = [&](const uint32_t(&q)[3][kEpiChunk], int c0) {
         float *o = out + int64_t(c0) * P.ohw;
@@ -423,14 +426,14 @@ __device__ __forceinline__ void potentials_epilogue(const TcParams &P, uint32_t 
             if (ok && c0 + j < n) *o = v;
         }
     };
-    tmem_chunk<NS>(lane_base, 0, P.n_tile, qa);
-    for (int c0 = 0; c0 < P.n_tile; c0 += 2 * kEpiChunk)  // n_tile is a multiple of 16
+    tmem_chunk<NS>(lane_base, first, P.n_tile, qa);
+    for (int c0 = first; c0 < end; c0 += 2 * kEpiChunk)
     {
         tmem_chunk_wait<NS>(qa);
         tmem_chunk<NS>(lane_base, c0 + kEpiChunk, P.n_tile, qb);
         put(qa, c0);
         tmem_chunk_wait<NS>(qb);
-        if (c0 + 2 * kEpiChunk < P.n_tile) tmem_chunk<NS>(lane_base, c0 + 2 * kEpiChunk, P.n_tile, qa);
+        if (c0 + 2 * kEpiChunk < end) tmem_chunk<NS>(lane_base, c0 + 2 * kEpiChunk, P.n_tile, qa);
         put(qb, c0 + kEpiChunk);
     }
 }
@@ -1792,13 +1795,14 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
     }
 }
 
-// Warp-specialised persistent kernel (416 threads):
+// Warp-specialised persistent kernel (544 threads; 416 without warps 13-16):
 //   warps 4-11 producers: per K block, wait for a free stage, bulk-copy the
 //              weight block (thread 128) and gather half an A row each;
 //   warp 12    one thread issues the tcgen05.mma of every stage into one of
 //              (up to) two tensor-memory accumulators and commits;
 //   warps 0-3  epilogue: read the accumulator of a finished tile (one row per
-//              thread) while the next tile is being multiplied.
+//              thread) while the next tile is being multiplied; warps 13-16
+//              share it for the potentials and the search.
 // Stage ring: full[s] (256 producer arrivals + the weight bytes), empty[s]
 // (MMA commit); accumulators: acc_full[a] (MMA commit), acc_empty[a] (128
 // epilogue arrivals).  Every wait is bounded; a timeout raises the device
@@ -1807,7 +1811,9 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
 // The search kernel (kSearch) runs with 4 producer warps (288 threads) so
 // that two CTAs fit on an SM where their tensor memory allows: its
 // per-tile work is latency-bound, and a second CTA hides those latencies.
-constexpr int kWsThreads = 416, kSearchThreads = 288, kMaxStages = 6;
+constexpr int kSearchThreads = 288, kMaxStages = 6;
+template <int MODE>
+constexpr int kWsThreads = MODE == kPotentials || MODE == kSearch ? 544 : 416;
 
 template <int MODE, int NPW>
 __device__ __forceinline__ void conv_ws_body(const TcParams &P)
@@ -1907,7 +1913,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     {
         for (int s = 0; s < S; ++s)
             mbar_init(&full_bar[s], 1 + (MODE == kSearch || (MODE == kPotentials && P.nhwc) ? 128 : 32 * NPW)), mbar_init(&empty_bar[s], 1);
-        for (int a = 0; a < 2; ++a) mbar_init(&accf_bar[a], 1), mbar_init(&acce_bar[a], 128);
+        for (int a = 0; a < 2; ++a) mbar_init(&accf_bar[a], 1), mbar_init(&acce_bar[a], MODE == kPotentials ? 256 : 128);
         mbar_init(&tim_bar, 128);
         for (int b = 0; b < 2; ++b) mbar_init(&ent_bar[b], 32 * NPW);
         for (int q = 0; q < 16; ++q) mbar_init(&tq_bar[q], 1);
@@ -2106,7 +2112,12 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     }
     else
     {
-        // ---------------- epilogue (warps 0-3) ----------------
+        // ---------------- epilogue (warps 0-3 and 13-16) ----------------
+        // The second four warps take the upper half of a tile's channels
+        // (potentials) or every other tile (search with one part and two
+        // accumulators, so that each group sees every phase of its own).
+        const bool second = warp > kMmaWarp;
+        const bool turns = MODE == kSearch && NPW == 8 && P.nparts == 1 && nacc == 2;
         // warp w reads tensor-memory lanes 32 w .. 32 w + 31 (rows of the tile)
         const int row = (warp & 3) * 32 + lane;
         // the largest channel bound (search)
@@ -2124,7 +2135,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
         uint32_t j = 0, k = 0;
         const int parts = MODE == kSearch ? P.nparts : 1;
         SearchScan scan;
-        int64_t tile = blockIdx.x;
+        int64_t tile = MODE == kSearch && second && !turns ? -1 : int64_t(blockIdx.x);
         // the MMA issuer's order of units (tile, part)
         for (int part = 0, nextp = 0; tile >= 0 && tile < ntiles; ++j, part = nextp)
         {
@@ -2144,6 +2155,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
             }
             nextp = part + 1;
             if (nextp == parts) nextp = 0, ++k;
+            if (turns && ((j & 1) != 0) != second) continue;
             const int a = int(j % uint32_t(nacc));
             const uint32_t ua = j / uint32_t(nacc);
             // search rows: the row's list entry and pixel state are loaded
@@ -2183,10 +2195,11 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
                 const uint32_t lane_base = acc + (uint32_t((warp & 3) * 32) << 16);
                 float *out = P.out + (r.img * P.cout + nt * P.n_tile) * P.ohw + r.pix;
                 const int n = P.cout - nt * P.n_tile;
+                const int mid = (P.n_tile / 16 + 1) / 2 * 16;
                 if (P.nsplit == 3)
-                    potentials_epilogue<3>(P, lane_base, r.ok, out, n);
+                    potentials_epilogue<3>(P, lane_base, r.ok, out, n, second ? mid : 0, second ? P.n_tile : mid);
                 else
-                    potentials_epilogue<2>(P, lane_base, r.ok, out, n);
+                    potentials_epilogue<2>(P, lane_base, r.ok, out, n, second ? mid : 0, second ? P.n_tile : mid);
             }
             if constexpr (MODE == kTimes)
             {
@@ -2235,7 +2248,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kWsThreads, 1) conv_ws_kernel(TcParams P)
+__global__ void __launch_bounds__(kWsThreads<MODE>, 1) conv_ws_kernel(TcParams P)
 {
     conv_ws_body<MODE, 8>(P);
 }
@@ -3347,7 +3360,7 @@ void launch(const TcParams &P, const Plan &pl, cudaStream_t s)
 {
     const bool two = MODE == kSearch && pl.tmem_cols <= 256;
     auto kern = two ? search_ws_kernel : conv_ws_kernel<MODE>;
-    const int threads = two ? kSearchThreads : kWsThreads;
+    const int threads = two ? kSearchThreads : kWsThreads<MODE>;
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.smem)));
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     int per_sm = 1;
