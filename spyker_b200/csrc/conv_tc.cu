@@ -222,8 +222,9 @@ __global__ void to_channels_last_kernel(const uint8_t *__restrict__ in, uint2 *_
 // row), K ordered as the A operand.  One thread per (tile, block, row, chunk).
 __global__ void split_weights_kernel(const float *__restrict__ kernel, uint4 *__restrict__ wimg, int cout, int cin,
                                      int taps, int nhwc, int cpad, int kblocks, int n_tile, int n_tiles, int nsplit,
-                                     int64_t wimg_stride16, int *negw)
+                                     int64_t wimg_stride16, int *negw, const int *lean_flag)
 {
+    if (lean_flag && !*negw && !*lean_flag) return;  // the search path has done the layer
     // blockIdx.y: network (kernels [N, Cout, Cin, KH, KW], images wimg_stride16 uint4 apart)
     kernel += int64_t(blockIdx.y) * cout * cin * taps;
     wimg += int64_t(blockIdx.y) * wimg_stride16;
@@ -2259,66 +2260,72 @@ __global__ void __launch_bounds__(kSearchThreads, 2) search_ws_kernel(TcParams P
 
 // WTA over the per-pixel records of one sample (one CTA per sample).  Keys
 // follow cpu/wta.cpp:53-62 with the sample's min / max; ties resolve to the
-// lowest flat index channel * H*W + pixel, as std::max_element does.
-__global__ void wta_records_kernel(const int4 *__restrict__ records, const unsigned *__restrict__ mins,
-                                   const unsigned *__restrict__ maxs, int hw, int w, int T, int ry, int rx, int count,
-                                   int32_t *__restrict__ winners, int32_t *__restrict__ counts)
+// lowest flat index channel * H*W + pixel, as std::max_element does.  A pixel's
+// key (order-encoded) and flat index stay in shared memory; a round is one pass
+// that also drops the pixels of the previous winner's channel, two integer
+// warp reductions and one over the warps' bests, and the winner's box is
+// cleared by its own few threads.  Latency bound (five rounds of some 1500
+// cycles): 300 maps of 33 x 33, 5 rounds, 13 us.
+__global__ void __launch_bounds__(1024) wta_records_kernel(const int4 *__restrict__ records,
+                                                           const unsigned *__restrict__ mins,
+                                                           const unsigned *__restrict__ maxs, int hw, int w, int T,
+                                                           int ry, int rx, int count, int32_t *__restrict__ winners,
+                                                           int32_t *__restrict__ counts)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
-    float *key = reinterpret_cast<float *>(wsm);
+    unsigned *key = reinterpret_cast<unsigned *>(wsm);
     int *flat = reinterpret_cast<int *>(key + hw);
-    __shared__ float s_v[32];
-    __shared__ int s_i[32];
+    __shared__ unsigned s_hi[32], s_lo[32];
     const int64_t b = blockIdx.x;
+    const int lane = threadIdx.x & 31, nw = int(blockDim.x >> 5), h = hw / w;
     const float mn = order_dec(mins[b]), mx = order_dec(maxs[b]);
     const float diff = __fmul_rn(__fsub_rn(mx, mn), 2.0f);
+#pragma unroll 4
     for (int p = threadIdx.x; p < hw; p += blockDim.x)
     {
         const int4 r = records[b * hw + p];
-        if (r.y < T)
-        {
-            key[p] = __fadd_rn(float(T - r.y - 1), __fdiv_rn(__fsub_rn(__int_as_float(r.z), mn), diff));
-            flat[p] = r.x * hw + p;
-        }
-        else
-        {
-            key[p] = -INFINITY;
-            flat[p] = INT_MAX;
-        }
+        const float k = __fadd_rn(float(T - r.y - 1), __fdiv_rn(__fsub_rn(__int_as_float(r.z), mn), diff));
+        const bool in = r.y < T && k == k;  // (a NaN key never wins)
+        key[p] = in ? order_enc(k) : 0u;
+        flat[p] = in ? r.x * hw + p : INT_MAX;
     }
     __syncthreads();
-    int found = 0;
+    int found = 0, zlo = 0, zhi = 0;
     for (int round = 0; round < count; ++round)
     {
-        float bv = -INFINITY;
-        int bi = INT_MAX;
+        // the largest key, then the lowest flat index (~flat largest)
+        unsigned hi = 0u, lo = 0u;
         for (int p = threadIdx.x; p < hw; p += blockDim.x)
-            if (key[p] > bv || (key[p] == bv && flat[p] < bi)) bv = key[p], bi = flat[p];
-        for (int o = 16; o > 0; o >>= 1)
         {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) bv = ov, bi = oi;
+            const int f = flat[p];
+            const unsigned k = key[p];
+            if (f >= zlo && f < zhi)
+                flat[p] = INT_MAX;
+            else if (f != INT_MAX && (k > hi || (k == hi && ~unsigned(f) > lo)))
+                hi = k, lo = ~unsigned(f);
         }
-        if ((threadIdx.x & 31) == 0) s_v[threadIdx.x >> 5] = bv, s_i[threadIdx.x >> 5] = bi;
+        auto reduce = [&] {
+            const unsigned top = __reduce_max_sync(0xffffffffu, lo ? hi : 0u);
+            lo = __reduce_max_sync(0xffffffffu, hi == top ? lo : 0u);
+            hi = top;
+        };
+        reduce();
+        if (lane == 0) s_hi[threadIdx.x >> 5] = hi, s_lo[threadIdx.x >> 5] = lo;
         __syncthreads();
-        bv = s_v[0], bi = s_i[0];
-        for (int q = 1; q < int(blockDim.x >> 5); ++q)
-            if (s_v[q] > bv || (s_v[q] == bv && s_i[q] < bi)) bv = s_v[q], bi = s_i[q];
-        __syncthreads();
-        if (bi == INT_MAX) break;  // only sentinels left
-        const int z = bi / hw, p0 = bi % hw, y = p0 / w, x = p0 % w;
+        hi = lane < nw ? s_hi[lane] : 0u, lo = lane < nw ? s_lo[lane] : 0u;
+        reduce();
+        if (lo == 0u) break;  // none left (the same in every thread)
+        const int bi = int(~lo), z = bi / hw, p0 = bi - z * hw, y = p0 / w, x = p0 - y * w;
         if (threadIdx.x == 0)
         {
             int32_t *e = winners + (b * count + round) * 5;
             e[0] = 0, e[1] = 0, e[2] = z, e[3] = y, e[4] = x;
         }
-        for (int p = threadIdx.x; p < hw; p += blockDim.x)
-        {
-            const int py = p / w, px = p % w;
-            const bool box = py >= y - ry && py <= y + ry && px >= x - rx && px <= x + rx;
-            if (box || (flat[p] != INT_MAX && flat[p] / hw == z)) key[p] = -INFINITY, flat[p] = INT_MAX;
-        }
+        // the winner's box (every channel) leaves now, its channel in the next pass
+        zlo = z * hw, zhi = zlo + hw;
+        const int y0 = max(y - ry, 0), x0 = max(x - rx, 0), bw = min(x + rx, w - 1) - x0 + 1;
+        const int area = bw * (min(y + ry, h - 1) - y0 + 1);
+        for (int q = threadIdx.x; q < area; q += blockDim.x) flat[(y0 + q / bw) * w + x0 + q % bw] = INT_MAX;
         __syncthreads();
         ++found;
     }
@@ -3255,16 +3262,30 @@ __global__ void times_fst_kernel(const float *__restrict__ tin, uint8_t *__restr
     }
 }
 
+// The weights' split into the workspace.  lean_flag: the map's flag of a layer
+// whose search path has run; the dense kernel, and so the split, is then only
+// needed off that path.
+void launch_split(const Plan &pl, const float *kernel, int64_t cin, int64_t cout, int64_t kh, int64_t kw, uint8_t *wimg,
+                  int64_t nnets, int *negw, const int *lean_flag, cudaStream_t s)
+{
+    const int64_t threads = int64_t(pl.n_tiles) * pl.kblocks * pl.n_tile * 8;
+    split_weights_kernel<<<dim3(grid_for(threads, 256), unsigned(nnets)), 256, 0, s>>>(
+        kernel, reinterpret_cast<uint4 *>(wimg), int(cout), int(cin), int(kh * kw), pl.nhwc ? 1 : 0, pl.cpad, pl.kblocks,
+        pl.n_tile, pl.n_tiles, pl.nsplit, int64_t(align256(pl.wimg_bytes) / 16), negw, lean_flag);
+    SPK_LAUNCHED();
+}
+
+
 // t_fused > 0: stage for the fused (pixel, time) rows of t_fused steps.
 TcParams prepare(const Plan &pl, const void *in, const float *kernel, int64_t n, int64_t cin, int64_t h, int64_t w,
                  int64_t cout, int64_t kh, int64_t kw, int64_t sy, int64_t sx, Pad4 p, int64_t oh, int64_t ow,
-                 uint8_t *ws, cudaStream_t s, int64_t t_fused = 0, int64_t nnets = 1, const float *times = nullptr)
+                 uint8_t *ws, cudaStream_t s, int64_t t_fused = 0, int64_t nnets = 1, const float *times = nullptr,
+                 bool split = true)
 {
     SPK_REQUIRE(pl.kblocks <= kMaxKBlocks, "Cin*KH*KW is too large for the tensor-core path");
     SPK_REQUIRE(pl.stages >= 2 && pl.smem <= 227 * 1024, "tile does not fit in shared memory");
     SPK_REQUIRE((reinterpret_cast<uintptr_t>(ws) & 255) == 0, "workspace must be 256-byte aligned");
     uint8_t *wimg = ws;
-    const int64_t wthreads = int64_t(pl.n_tiles) * pl.kblocks * pl.n_tile * 8;
     SPK_REQUIRE(nnets >= 1 && nnets <= 65535, "invalid number of networks");
     int *negw = nullptr;
     if (t_fused > 0)
@@ -3275,11 +3296,7 @@ TcParams prepare(const Plan &pl, const void *in, const float *kernel, int64_t n,
                                        align256(size_t(n / t_fused) * h * w * cp) + 128);
         SPK_CUDA(cudaMemsetAsync(negw - 32, 0, 256, s));  // the flag, this word and the walk's two
     }
-    const dim3 sgrid(grid_for(wthreads, 256), unsigned(nnets));
-    split_weights_kernel<<<sgrid, 256, 0, s>>>(kernel, reinterpret_cast<uint4 *>(wimg), int(cout), int(cin),
-                                               int(kh * kw), pl.nhwc ? 1 : 0, pl.cpad, pl.kblocks, pl.n_tile,
-                                               pl.n_tiles, pl.nsplit, int64_t(align256(pl.wimg_bytes) / 16), negw);
-    SPK_LAUNCHED();
+    if (split) launch_split(pl, kernel, cin, cout, kh, kw, ws, nnets, negw, nullptr, s);
     const uint8_t *a_src = static_cast<const uint8_t *>(in);
     TcParams P{};
     P.negw = negw;
@@ -3302,8 +3319,13 @@ TcParams prepare(const Plan &pl, const void *in, const float *kernel, int64_t n,
         else
         {
             // whole images when their tile fits in 48 KB, else the longest runs
-            // of whole words that do
-            const int64_t ppc = std::min<int64_t>(h * w, (48 * 1024 / (cp + 1)) & ~int64_t(3));
+            // of whole words that do; with fewer images than SMs, shorter runs
+            // (128 pixels or more) so that two CTAs a SM share them (24 images
+            // of 20 x 20 .. 64 x 64: 16 -> 7 us on average; 8 of 256 x 256: 183 -> 95)
+            int64_t ppc = std::min<int64_t>(h * w, (48 * 1024 / (cp + 1)) & ~int64_t(3));
+            if (b < sm_count() && (h * w) % 4 == 0 && reinterpret_cast<uintptr_t>(a_src) % 4 == 0)
+                ppc = std::min<int64_t>(
+                    ppc, std::max<int64_t>(128, ceil_div(ceil_div(b * h * w, 2 * int64_t(sm_count())), 32) * 32));
             const size_t tile = size_t(ppc) * (cp + 1);
             if (ppc == h * w && (cin * h * w) % 8 == 0 && reinterpret_cast<uintptr_t>(a_src) % 8 == 0 &&
                 b <= 65535)
@@ -3768,7 +3790,16 @@ void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b
     if (b == 0) return;
     cudaStream_t s = stream_of(stream);
     uint8_t *base = static_cast<uint8_t *>(ws);
-    TcParams P = prepare(L.pl, in, kernel, b * t, cin, h, w, cout, kh, kw, sy, sx, p, L.oh, L.ow, base, s, t, nets.n);
+    // The search path (lean layers, kSearch): chosen here by the thresholds
+    // and by the fit of the layer; the kernels themselves check the weights'
+    // signs and the input's form and leave the work to the dense kernel
+    // otherwise.
+    const float fthr = float(threshold), fthv = float(value), finh = float(inhibit_threshold);
+    const float ffire = float(fire_threshold), fwta = float(wta_threshold);
+    const bool search = L.search_ok && !nets.offsets && fthv <= finh && fthv <= ffire && fthv <= fwta &&
+                        finh <= fthr && ffire <= fthr && fwta <= fthr;
+    TcParams P = prepare(L.pl, in, kernel, b * t, cin, h, w, cout, kh, kw, sy, sx, p, L.oh, L.ow, base, s, t, nets.n,
+                         nullptr, !search);
     if (nets.offsets) P.snet = nets.sample_net, P.net_thr = nets.threshold;
     P.T = int(t), P.tp_log2 = L.tp_log2, P.pp = L.pp, P.npix = L.npix;
     int lp = 0;
@@ -3785,14 +3816,6 @@ void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b
         SPK_REQUIRE(L.oh >= pool_ky && L.ow >= pool_kx, "the pooling window is larger than the output");
         P.pooled = pooled, P.pky = int(pool_ky), P.pkx = int(pool_kx), P.poh = int(poh), P.pow_ = int(pow_);
     }
-    // The search path (lean layers, kSearch): chosen here by the thresholds
-    // and by the fit of the layer; the kernels themselves check the weights'
-    // signs and the input's form and leave the work to the dense kernel
-    // otherwise.
-    const float fthr = float(threshold), fthv = float(value), finh = float(inhibit_threshold);
-    const float ffire = float(fire_threshold), fwta = float(wta_threshold);
-    const bool search = L.search_ok && !nets.offsets && fthv <= finh && fthv <= ffire && fthv <= fwta &&
-                        finh <= fthr && ffire <= fthr && fwta <= fthr;
     if (count > 0 || search)
     {
         P.records = reinterpret_cast<int4 *>(base + L.rec_off);
@@ -3804,6 +3827,7 @@ void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b
     if (search)
     {
         search_layer(P, L, kernel, count, pool_ky, pool_kx, poh, pow_, spikes, pooled, base, s);
+        launch_split(L.pl, kernel, cin, cout, kh, kw, base, nets.n, P.negw, P.flag, s);
         P.skip_when_lean = 1;
         if (count == 0) P.records = nullptr;
     }
@@ -3821,18 +3845,23 @@ void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b
     if (count == 0) return;
     const int hw = int(L.oh * L.ow);
     const unsigned wgrid = unsigned(ceil_div(b, 4));
-    if (hw <= 256)
+    // a CTA per sample while all of them are resident (333 of 256 pixels: 9 us
+    // against 12 with a warp each, 64 of 784: 8 against 17) and for maps too
+    // large for a warp's registers; then a warp per sample (4096 of 784 and of
+    // 196: 73 us against 82)
+    if (hw > 1024 || b <= 8 * sm_count())
+        wta_records_kernel<<<unsigned(b), hw <= 256 ? 128 : hw <= 1024 ? 256 : hw <= 4096 ? 512 : 1024, size_t(hw) * 8,
+                             s>>>(P.records, P.mins, P.maxs, hw, int(L.ow), int(t), int(ry), int(rx), int(count), winners,
+                                  counts);
+    else if (hw <= 256)
         wta_records_warp_kernel<8><<<wgrid, 128, 0, s>>>(P.records, P.mins, P.maxs, b, hw, int(L.ow), int(t), int(ry),
                                                           int(rx), int(count), winners, counts);
     else if (hw <= 800)
         wta_records_warp_kernel<25><<<wgrid, 128, 0, s>>>(P.records, P.mins, P.maxs, b, hw, int(L.ow), int(t),
                                                            int(ry), int(rx), int(count), winners, counts);
-    else if (hw <= 1024)
+    else
         wta_records_warp_kernel<32><<<wgrid, 128, 0, s>>>(P.records, P.mins, P.maxs, b, hw, int(L.ow), int(t),
                                                            int(ry), int(rx), int(count), winners, counts);
-    else
-        wta_records_kernel<<<unsigned(b), 256, size_t(hw) * 8, s>>>(P.records, P.mins, P.maxs, hw, int(L.ow), int(t),
-                                                                    int(ry), int(rx), int(count), winners, counts);
     SPK_LAUNCHED();
 }
 }  // namespace
