@@ -647,26 +647,38 @@ __global__ void __launch_bounds__(128) sparse_conv_maps_kernel(MapsArgs A)
                 const int xlo = max(0, xx - KW + 1), xhi = min(ow - 1, xx);
                 const uint64_t m = ((xhi == 63 ? 0ull : (1ull << (xhi + 1))) - 1ull) & ~((1ull << xlo) - 1ull);
                 if (lane <= yb && lane > yb - KH) mask |= m;
-                float *p = pot + (yb * ow + xx) * 32;
-                const bool inside = xx >= KW - 1 && xx < ow;
-#pragma unroll
-                for (int ky = 0; ky < KH; ++ky, p -= ow * 32)
+                float *const p = pot + (yb * ow + xx) * 32;
+                if (xx >= KW - 1 && xx < ow)
                 {
-                    if (yb - ky < 0 || yb - ky >= ny) continue;
-                    if (inside)
-                    {
-                        float v[KW];
+                    // every row's values are read before the first is written:
+                    // their latencies overlap
+                    float v[KH * KW];
 #pragma unroll
-                        for (int kx = 0; kx < KW; ++kx) v[kx] = p[-kx * 32];
+                    for (int ky = 0; ky < KH; ++ky)
+                        if (yb - ky >= 0 && yb - ky < ny)
+                        {
 #pragma unroll
-                        for (int kx = 0; kx < KW; ++kx) p[-kx * 32] = v[kx] + w[ky * KW + kx];
-                    }
-                    else
-                    {
+                            for (int kx = 0; kx < KW; ++kx) v[ky * KW + kx] = p[-(ky * ow + kx) * 32];
+                        }
 #pragma unroll
-                        for (int kx = 0; kx < KW; ++kx)
-                            if (xx - kx >= 0 && xx - kx < ow) p[-kx * 32] += w[ky * KW + kx];
-                    }
+                    for (int ky = 0; ky < KH; ++ky)
+                        if (yb - ky >= 0 && yb - ky < ny)
+                        {
+#pragma unroll
+                            for (int kx = 0; kx < KW; ++kx)
+                                p[-(ky * ow + kx) * 32] = v[ky * KW + kx] + w[ky * KW + kx];
+                        }
+                }
+                else
+                {
+#pragma unroll
+                    for (int ky = 0; ky < KH; ++ky)
+                        if (yb - ky >= 0 && yb - ky < ny)
+                        {
+#pragma unroll
+                            for (int kx = 0; kx < KW; ++kx)
+                                if (xx - kx >= 0 && xx - kx < ow) p[-(ky * ow + kx) * 32] += w[ky * KW + kx];
+                        }
                 }
             }
             k = stop;
