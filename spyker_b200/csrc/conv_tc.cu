@@ -2917,16 +2917,60 @@ __device__ __forceinline__ double oracle_sum(const TcParams &P, const uint8_t *f
     return acc;
 }
 
+// A warp's form of the same sums: 32 inputs at a time, in the oracle's order,
+// a lane per input for the test of its step, then the fired ones one after
+// another.  One: all lanes sum channel o0.  Otherwise lane l sums channels o0 +
+// l + 32 g, g < ng, whose loads and additions are independent.  (A lane going
+// through a channel's inputs by itself waits for every kernel row's loads: one
+// open row of 256 channels and 1600 inputs took the launch 1400 us.)
+constexpr int kFixGroups = 8;
+template <bool ONE>
+__device__ __forceinline__ void oracle_sum_warp(const TcParams &P, const uint8_t *fm, const float *kernel, int o0, int ng,
+                                                int iy0, int ix0, int cp, int t, double (&acc)[kFixGroups])
+{
+    const int lane = threadIdx.x & 31, taps = P.kh * P.kw, K = P.cin * taps;
+#pragma unroll
+    for (int g = 0; g < kFixGroups; ++g) acc[g] = 0.0;
+    const float *wl = kernel + int64_t(o0) * K;
+    for (int k0 = 0; k0 < K; k0 += 32)
+    {
+        const int k = k0 + lane, c = k / taps, tap = k - c * taps, ky = tap / P.kw;
+        const int iy = iy0 + ky, ix = ix0 + tap - ky * P.kw;
+        const bool in = k < K && iy >= 0 && iy < P.h && ix >= 0 && ix < P.w;
+        const bool fired = in && int(__ldg(fm + (int64_t(iy) * P.w + ix) * cp + c)) <= t;
+        const float mine = ONE && fired ? __ldg(wl + k) : 0.f;
+        unsigned m = __ballot_sync(0xffffffffu, fired);
+        if constexpr (ONE)
+            while (m)
+            {
+                acc[0] += double(__shfl_sync(0xffffffffu, mine, __ffs(int(m)) - 1));
+                m &= m - 1u;
+            }
+        else
+            while (m)
+            {
+                const float *w = wl + k0 + (__ffs(int(m)) - 1);
+                m &= m - 1u;
+#pragma unroll
+                for (int g = 0; g < kFixGroups; ++g)
+                    if (g < ng && o0 + g * 32 + lane < P.cout) acc[g] += double(__ldg(w + int64_t(g * 32 + lane) * K));
+            }
+    }
+}
+
 __global__ void __launch_bounds__(128) search_fix_kernel(TcParams P, const float *__restrict__ kernel, int cp)
 {
     if (*P.negw || *P.flag) return;
     const int lane = threadIdx.x & 31;
     const int64_t nw = int64_t(gridDim.x) * (blockDim.x >> 5);
     const int taps = P.kh * P.kw;
-    // rows whose winner is decided: one lane per row sums the winner's
-    // products in the oracle's order
+    // rows whose winner is decided: the winner's products in the oracle's
+    // order, summed by a lane per row, or by a warp per row where that leaves
+    // none waiting
     const int nv = *P.val_count;
-    for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < nv; q += int64_t(gridDim.x) * blockDim.x)
+    const bool few = nv <= nw;
+    const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (int64_t q = few ? first >> 5 : first; q < nv; q += few ? nw : nw * 32)
     {
         const int4 e = P.val_list[q];
         const int pix = e.x, t = e.y, idx = e.z, o = e.w, round = P.round;
@@ -2934,8 +2978,16 @@ __global__ void __launch_bounds__(128) search_fix_kernel(TcParams P, const float
         const int oy = pp / P.ow, ox = pp - oy * P.ow;
         const int iy0 = oy * P.sy - P.top, ix0 = ox * P.sx - P.left;
         const uint8_t *fm = P.in + int64_t(smp) * P.img_stride;
-        const float *wk = kernel + int64_t(o) * P.cin * taps;
-        const double acc = oracle_sum(P, fm, wk, iy0, ix0, cp, t);
+        double acc;
+        if (few)
+        {
+            double sums[kFixGroups];
+            oracle_sum_warp<true>(P, fm, kernel, o, 1, iy0, ix0, cp, t, sums);
+            acc = sums[0];
+            if (lane != 0) continue;
+        }
+        else
+            acc = oracle_sum(P, fm, kernel + int64_t(o) * P.cin * taps, iy0, ix0, cp, t);
         atomicAdd(&g_recomputes, 1ull);
         const SearchAct r = search_act(P, round, pix, t, 2, o, float(acc), round == 1 ? P.state[pix] : int4{});
         if (round != 2) P.list_out[idx] = r.next ? r.next_e : make_int2(pix, -1);
@@ -2944,7 +2996,16 @@ __global__ void __launch_bounds__(128) search_fix_kernel(TcParams P, const float
         if (P.wta) s_extremes(P, pix, r);
     }
     const int n = *P.fix_count;
-    for (int64_t q = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); q < n; q += nw)
+    // the other open rows: every channel, a warp per row; a CTA per row, its
+    // warps on pairs of channel groups, where the rows are few (256 channels:
+    // 46 us a launch against 92)
+    __shared__ float s_best[4], s_mine[4];
+    __shared__ int s_besti[4];
+    const int warp = threadIdx.x >> 5;
+    const bool shared = P.cout > 64 && n <= int(gridDim.x);
+    const int gw = shared ? 2 : kFixGroups;  // channel groups of a warp at a time
+    for (int64_t q = shared ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * (blockDim.x >> 5) + warp; q < n;
+         q += shared ? int64_t(gridDim.x) : nw)
     {
         const int4 e = P.fix_list[q];
         const int pix = e.x, t = e.y, idx = e.z, aux = e.w, round = P.round;
@@ -2954,12 +3015,19 @@ __global__ void __launch_bounds__(128) search_fix_kernel(TcParams P, const float
         const uint8_t *fm = P.in + int64_t(smp) * P.img_stride;
         float best = -INFINITY, mine = 0.f;
         int besti = INT_MAX;
-        for (int o = lane; o < P.cout; o += 32)
+        for (int o0 = shared ? warp * 64 : 0; o0 < P.cout; o0 += 32 * kFixGroups)
         {
-            if (round == 2 && o != aux) continue;
-            const float pv = float(oracle_sum(P, fm, kernel + int64_t(o) * P.cin * taps, iy0, ix0, cp, t));
-            if (pv > best) best = pv, besti = o;
-            if (o == aux) mine = pv;
+            const int ng = min(gw, (P.cout - o0 + 31) / 32);
+            double sums[kFixGroups];
+            oracle_sum_warp<false>(P, fm, kernel, o0, ng, iy0, ix0, cp, t, sums);
+#pragma unroll
+            for (int g = 0; g < kFixGroups; ++g)
+            {
+                const int o = o0 + g * 32 + lane;
+                const float pv = float(sums[g]);
+                if (g < ng && o < P.cout && pv > best) best = pv, besti = o;
+                if (o == aux) mine = pv;
+            }
         }
         // first channel of the largest potential across the lanes
         for (int off = 16; off > 0; off >>= 1)
@@ -2969,7 +3037,15 @@ __global__ void __launch_bounds__(128) search_fix_kernel(TcParams P, const float
             if (ob > best || (ob == best && oi < besti)) best = ob, besti = oi;
         }
         mine = __shfl_sync(0xffffffffu, mine, aux & 31);
-        if (lane == 0)
+        if (shared)  // (one row per CTA, so the whole CTA is here)
+        {
+            if (lane == 0) s_best[warp] = best, s_besti[warp] = besti, s_mine[warp] = mine;
+            __syncthreads();
+            for (int i = 0; i < 4; ++i)
+                if (s_best[i] > best || (s_best[i] == best && s_besti[i] < besti)) best = s_best[i], besti = s_besti[i];
+            mine = s_mine[(aux >> 6) & 3];
+        }
+        if (lane == 0 && (!shared || warp == 0))
         {
             atomicAdd(&g_recomputes, 1ull);
             int dec, a;
