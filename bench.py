@@ -55,12 +55,12 @@ def bf16_peak():
 def path_dtype(precision: str):
     """(dtype, arithmetic) of the fused layers.  With non-negative weights
     (STDP keeps them in [0, 1]) a fused layer takes the first-crossing search:
-    u8 spikes x u8 base-256 weight digits on the tensor cores with exact S32
+    u8 spikes x 31-bit weights in u8 fields on the tensor cores with exact S32
     sums, each potential rounded once from the exact sum; other weights take
     the dense split kernel of ``precision``."""
     if precision == "fp32":
         return "f32", "FP32 SIMT convolution, op by op"
-    return "u8", (f"u8 spikes x 4 u8 weight digits (tcgen05 kind::i8, exact S32 sums, potentials rounded once "
+    return "u8", (f"u8 spikes x 31-bit weights in u8 fields (tcgen05 kind::i8, exact S32 sums, potentials rounded once "
                   f"from the exact sum); {precision}-split/f32-acc dense kernel when a weight is negative")
 
 

@@ -19,7 +19,8 @@
  *  - Work is enqueued on `stream` (a cudaStream_t; NULL = legacy default).
  *    Calls never synchronise the stream unless documented.
  *  - Winners travel as int32 records [B, count, 5] = (c, t, z, y, x)
- *    (src/spyker/utils.h:483-502) plus int32 per-sample counts [B].
+ *    (src/spyker/utils.h:483-502) plus int32 per-sample counts [B]; the
+ *    selections write zeros past a sample's count.
  *  - Entry points that need scratch memory take a caller-provided workspace
  *    (`ws`, `ws_bytes`); the matching `_workspace` query returns the bytes
  *    needed.  The library never allocates device memory on these paths.
@@ -260,9 +261,9 @@ spk_status spk_conv(const void *in, spk_dtype itype, const float *kernel, float 
  * with two terms (a three-term request above 170 channels keeps two: every
  * near-threshold decision is re-made exactly at either split).  With no
  * negative weight, cumulative 0/1 input and value <= the inhibit / fire / WTA
- * thresholds <= threshold, the layer runs as a first-crossing search on u8
- * weight digits (exact integer sums) instead of the dense kernel; results
- * are the same.  spk_recheck_count / spk_recompute_count count its rows
+ * thresholds <= threshold, the layer runs as a first-crossing search on
+ * exact integer sums (u8 tensor cores, or, for few output pixels, each pixel's
+ * inputs in spike order) instead of the dense kernel; results are the same.  spk_recheck_count / spk_recompute_count count its rows
  * re-decided from exact sums and recomputed from the F32 weights. */
 size_t spk_conv_fire_wta_workspace(int64_t b, int64_t t, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh,
                                    int64_t kw, int64_t sy, int64_t sx, const int64_t *pad4_host, int precision);
@@ -348,12 +349,14 @@ spk_status spk_fst_conv_backward(const float *t_in, int64_t b, int64_t cin, int6
                                  const float *grad_out, int64_t oh, int64_t ow, const int64_t *stride2_host,
                                  const int64_t *pad4_host, float *grad_in, float *grad_kernel, void *ws,
                                  size_t ws_bytes, spk_stream stream);
-/* Forward of a first-spike conv layer on the tensor cores in one fused
- * kernel: t_out[b,z,oy,ox] = first t in 0..T-1 with potential(t) > threshold,
+/* Forward of a first-spike conv layer in one call: t_out[b,z,oy,ox] = first t in 0..T-1 with potential(t) > threshold,
  * T when none, where potential(t) = conv of the cumulative spikes [t_in <= t]
  * (BF16x2/x3 split weights, the FP64 sum of the split terms rounded once to
  * F32, exactly as spk_conv's potentials followed by spk_rank_gather); the
- * potentials are never written.  t_in [B, Cin, H, W] F32 (values >= T =
+ * potentials are never written.  With the queried workspace and weights that
+ * fit it walks each pixel's inputs in time order, with a smaller one it
+ * evaluates every step on the tensor cores; the results are the same up to
+ * the FP64 sums' order.  t_in [B, Cin, H, W] F32 (values >= T =
  * never); T <= 126; all output channels in one CTA (workspace query 0
  * otherwise). */
 size_t spk_fst_conv_times_workspace(int64_t b, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh,

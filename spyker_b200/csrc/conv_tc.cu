@@ -3461,12 +3461,10 @@ void launch(const TcParams &P, const Plan &pl, cudaStream_t s)
     const int threads = two ? kSearchThreads : kWsThreads<MODE>;
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.smem)));
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    int per_sm = 1;
-    SPK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, pl.smem));
-    // the two-CTA search kernel is sized for two per SM (its registers, shared
-    // memory and tensor memory were chosen for it); the runtime's estimate
-    // can fall short of what the hardware places
-    if (two) per_sm = std::max(per_sm, 2);
+    // resident CTAs per SM: two of the search kernel sized for it (registers,
+    // shared and tensor memory), one of the others (416 threads or more of 80
+    // registers or more)
+    int per_sm = two ? 2 : 1;
     per_sm = std::max(1, std::min<int>(per_sm, int(512 / pl.tmem_cols)));
     if (g_schedule.ctas > 0) per_sm = std::min(per_sm, g_schedule.ctas);
     const int64_t grid = std::min<int64_t>(P.tiles, int64_t(sm_count()) * per_sm);
