@@ -920,16 +920,16 @@ __device__ __forceinline__ void potentials_producer(const TcParams &P, const int
         const int4 e = s_row[int(k & 1) * BM + row0 + 32 * i];
         ubase[i] = P.in + ((int64_t(e.y) << 32) | uint32_t(e.x)), uy[i] = e.z, ux[i] = e.w;
     };
+    auto offset = [](const int4 &e) { return uint64_t(uint32_t(e.x)) * 8u; };
     // the chunk's bytes of unit i; ea, eb: its two groups' table entries
-    // (byte offset from the origin, ky, kx)
     auto load = [&](int i, const int4 &ea, const int4 &eb) {
         const bool oka = uint32_t(uy[i] + ea.y) < uint32_t(P.h) && uint32_t(ux[i] + ea.z) < uint32_t(P.w);
         if constexpr (WIDE)
-            f[i] = ldg16_if<0>(ubase[i] + ea.x, oka);
+            f[i] = ldg16_if<0>(ubase[i] + offset(ea), oka);
         else
         {
             const bool okb = uint32_t(uy[i] + eb.y) < uint32_t(P.h) && uint32_t(ux[i] + eb.z) < uint32_t(P.w);
-            const uint2 a = ldg8_if<0>(ubase[i] + ea.x, oka), b = ldg8_if<0>(ubase[i] + eb.x, okb);
+            const uint2 a = ldg8_if<0>(ubase[i] + offset(ea), oka), b = ldg8_if<0>(ubase[i] + offset(eb), okb);
             f[i] = make_uint4(a.x, a.y, b.x, b.y);
         }
     };
@@ -1893,13 +1893,14 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     }
     else if (P.nhwc)
     {
-        // per 8-input group (channels-last): (byte offset from the receptive
+        // per 8-input group (channels-last): (groups from the receptive
         // field's origin, ky, kx)
         const int groups = P.cpad / 8;
         for (int q = tid; q < P.kblocks * 8; q += blockDim.x)
         {
             const int tap = q / groups, g = q % groups, ky = tap / P.kw, kx = tap % P.kw;
-            tab[q] = tap < taps ? make_int4((ky * P.w + kx) * P.cpad + g * 8, ky, kx, 0) : make_int4(0, kNoRow, 0, 0);
+            const int64_t off8 = (int64_t(ky) * P.w + kx) * groups + g;
+            tab[q] = tap < taps ? make_int4(int(uint32_t(off8)), ky, kx, 0) : make_int4(0, kNoRow, 0, 0);
         }
     }
     else
