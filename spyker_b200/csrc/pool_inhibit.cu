@@ -198,6 +198,46 @@ __global__ void __launch_bounds__(256) pool_plane_kernel(const T *__restrict__ i
     }
 }
 
+// 3x3 windows, stride 3, no padding, of U8 planes with at most 32 outputs (14 x
+// 14 -> 4 x 4 and smaller).  A lane keeps its output's place in a plane, a warp
+// takes 32 / outputs planes at a time, four such groups in flight, so there is
+// no index arithmetic in the loop; a window's bytes come from L1 after the
+// first.  Bound by the loads (nine of a byte per output): 750,000 planes of 14 x
+// 14 55 us; staging whole planes in shared memory and dividing per output took
+// 130 us.
+__global__ void __launch_bounds__(256) pool3x3_u8_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out,
+                                                         int64_t n, int hw, int w, int ow, int outputs)
+{
+    const int lane = threadIdx.x & 31, planes = 32 / outputs;
+    const int sub = lane / outputs, o = lane - sub * outputs, oy = o / ow, ox = o - oy * ow;
+    const bool mine = sub < planes;
+    const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+    const uint8_t *src = in + int64_t(sub) * hw + oy * 3 * w + ox * 3;
+    for (int64_t g = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); g * planes < n; g += 4 * warps)
+    {
+        uint8_t v[4][9];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const int64_t p0 = (g + u * warps) * planes;
+            const bool in_range = mine && p0 + sub < n;
+            const uint8_t *s = src + p0 * hw;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) v[u][k] = in_range ? __ldg(s + (k / 3) * w + k % 3) : uint8_t(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            const int64_t p0 = (g + u * warps) * planes;
+            if (!mine || p0 + sub >= n) continue;
+            uint32_t m = v[u][0];
+#pragma unroll
+            for (int k = 1; k < 9; ++k) m = max(m, uint32_t(v[u][k]));
+            out[(p0 + sub) * outputs + o] = uint8_t(m);
+        }
+    }
+}
+
 // src/spyker/cpu/inhibit.cpp:41-121 over [B, T, C, X], one thread per (b, x):
 // per step the first channel with the largest value (strict >), the number
 // of steps whose maximum exceeds the threshold, the winning channel taken at
@@ -462,6 +502,15 @@ spk_status spk_rank_pool(const void *in, void *out, spk_dtype type, int64_t n, i
             {
                 pool2x2_u8_kernel<<<grid_for(n * ceil_div(oh, 7) * (ow / 2), 256), 256, 0, stream_of(stream)>>>(
                     (const uint8_t *)in, (uint8_t *)out, n, int(h), int(w), int(oh), int(ow));
+                SPK_LAUNCHED();
+                return;
+            }
+            if (sizeof(T) == 1 && ky == 3 && kx == 3 && sy == 3 && sx == 3 && oh * ow <= 32 && p.top == 0 && p.left == 0 &&
+                oh * 3 <= h && ow * 3 <= w && h * w < (int64_t(1) << 30))
+            {
+                pool3x3_u8_kernel<<<unsigned(std::min<int64_t>(ceil_div(n, 8), int64_t(sm_count()) * 8)), 256, 0,
+                                    stream_of(stream)>>>((const uint8_t *)in, (uint8_t *)out, n, int(h * w), int(w), int(ow),
+                                                         int(oh * ow));
                 SPK_LAUNCHED();
                 return;
             }
