@@ -7,24 +7,23 @@
 // Each F32 weight is split into BF16 terms w = h + m (+ l) (h = bf16(w),
 // m = bf16(w - h), l = bf16(w - h - m)); every term gets its own FP32
 // accumulator in tensor memory, so each partial sum stays exact for weights
-// in [2^-6, 1]; the terms are added once in FP64 and rounded once to F32.
+// in [2^-6, 1]; the terms' total is rounded once to F32 (sum_terms).
 // BF16X3 therefore reproduces the exactly rounded potential; BF16X2 (hi+lo)
 // is within 2^-18 relative.
 //
 // Two A layouts:
-//  * channels-last (Cin >= 8): the spikes are first transposed to
-//    [N, H, W, Cpad] u8 (Cpad = Cin rounded up to 8) and k = tap * Cpad + c,
-//    so every 8-wide K chunk of a row is one 8-byte load;
-//  * channel-major (Cin < 8): k = c * KH*KW + tap (the reference's order),
-//    gathered element by element (keeps K small for 1-2 input channels).
+//  * channels-last (Cin >= 2, where the workspace holds it): the spikes are
+//    first transposed to [N, H, W, Cpad] u8 (Cpad = Cin rounded up to 8) and
+//    k = tap * Cpad + c, so every 8-wide K chunk of a row is one 8-byte load
+//    (16 bytes where Cpad is a multiple of 16);
+//  * channel-major: k = c * KH*KW + tap (the reference's order), gathered
+//    element by element.
 //
-// CTA (persistent, 256 threads) per 128-row M tile and N tile walks K in
-// 64-wide blocks through a two-stage shared-memory ring: thread 0 starts a
-// bulk copy (TMA engine, no multicast) of the pre-split weight block, stored
-// in global memory in the K-major no-swizzle canonical layout, while all
-// threads gather the A block; thread 0 then issues the tcgen05.mma
-// instructions (M=128, N=n_tile, K=16) and commits them to the stage's
-// mbarrier.  The epilogue reads the accumulators with tcgen05.ld.  Every
+// The kernels are persistent and warp-specialised (conv_ws_body): producer
+// warps gather the A blocks, bulk copies (TMA engine, no multicast) bring the
+// pre-split weight blocks, stored in global memory in the K-major no-swizzle
+// canonical layout, one elected lane issues the tcgen05.mma instructions (M =
+// 128) and the epilogue warps read the accumulators with tcgen05.ld.  Every
 // mbarrier wait is bounded: on timeout the kernel records an error in the
 // device status word (spk_device_status) and leaves.
 #include <algorithm>
@@ -136,10 +135,10 @@ struct TcParams
     int4 *val_list;  // rows whose winner is decided but not its value: (pixel, step, row index, winner)
     int *val_count;
     int4 *state;     // per pixel: (lo | hi << 8 | winner << 16, value, winner at T-1, value at T-1)
-    const float *echan;     // per channel bound of |oracle potential - exact term sum|
+    const float *echan;     // per channel bound of |oracle potential - (exact term sum + ccent)| (walk: ccent = 0)
     const float *cscale;    // per channel, the value of one unit of the term total (2^(e - 31); the walk 2^(e - 32))
     const float *ccent;     // per channel, the middle of what the split left out
-    const unsigned *sinfo;  // [0] largest echan (bits), [1] largest channel exponent + 128
+    const unsigned *sinfo;  // [0] largest bound on oracle potential - exact term sum (bits), [1] largest channel exponent + 128
     int kreal;              // real K (taps x input channels)
     int r0_list;            // round 0 takes the (pixel, T - 1) entries of list_in (bound pre-filter ran)
     int nparts;             // channel parts of n_tile per tile (search)
@@ -1189,15 +1188,14 @@ __device__ __forceinline__ void fused_producer(const TcParams &P, const int4 *ta
 // Every decision is the oracle's: the potential of a row is the F32 rounding
 // of the FP64 sum of its products in (channel, ky, kx) order.  The weights
 // are split on fixed per-channel grids (fixed_split_kernel), so each
-// tensor-memory sum is exact and their total r_q is within echan[c] of the
-// oracle's FP64 sum.  Tier 1 adds the terms in FP32 and decides when the
-// rigorous bound 3.125 * 2^-24 |f| + c0 separates the largest potential from
-// the threshold and from the runner-up by more than an ulp; the winner's
-// value is then r_q rounded once, kept when r_q +- echan stays inside that
-// float's rounding interval.  Tier 2 (rows tier 1 leaves open) does the same
-// for every channel of the row and decides on the exact values, with the
-// possible neighbours of each uncertified one.  Rows still open go to
-// search_fix_kernel, which recomputes them as the oracle does.
+// tensor-memory sum is exact and the total's value plus ccent[c] is within
+// echan[c] of the oracle's FP64 sum.  Tier 1 (search_epilogue) compares
+// integer keys of the totals and decides when the bounds separate the largest
+// potential from the threshold and from the runner-up; the winner's value is
+// kept when every sum within its bound rounds to one float.  Tier 2 (rows tier
+// 1 leaves open) does the same for every channel of the row and decides on the
+// exact values, with the possible neighbours of each uncertified one.  Rows
+// still open go to search_fix_kernel, which recomputes them as the oracle does.
 template <int NS>
 __device__ __forceinline__ void s_chunk(uint32_t lane_base, int c0, int n_tile, uint32_t (&q)[NS][kEpiChunk])
 {
@@ -3475,7 +3473,7 @@ void launch(const TcParams &P, const Plan &pl, cudaStream_t s)
 
 struct FusedLayout
 {
-    Plan pl, pl4;  // dense fused kernel; search kernels (3 or 4 split terms)
+    Plan pl, pl4;  // dense fused kernel; search kernels
     int tp_log2, pp;
     int64_t npix, oh, ow;
     size_t rec_off, min_off, max_off;
@@ -3721,8 +3719,8 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
     const int groups = taps * (P.cpad / 8);
     if (P.nhwc && P.T <= 32 && groups <= 256 && P.cout <= 256 && walk_pays(L.npix, groups, P.cout))
     {
-        // (the integers take the digit image's bytes: 128 rows per K block,
-        // four bytes per channel and row)
+        // (the integers take the weight image's bytes: four per input and
+        // channel in both)
         uint32_t *wd = reinterpret_cast<uint32_t *>(base + L.w4_off);
         unsigned *wtop = reinterpret_cast<unsigned *>(P.negw - 16);
         walk_split_kernel<<<unsigned(nch), 256, 0, s>>>(kernel, wd, P.cout, P.cin, taps, P.cpad, nch, echan, cscale,

@@ -20,15 +20,15 @@
 // one image of 14 x 14 13.5 us.  The rounds took about 115 us for each of them
 // (64 images: 140 us) and win above some 100,000 pixels (walk_pays).
 //
-// Arithmetic: a channel's weights are the 32-bit integers floor(w 2^(32-e)) of
-// the digit split (the same 2^e, remainder bound and certification as the
-// tensor-core rounds), so a running sum is the exact term total R, in 64-bit
-// integers and in any order.  A winner's value that the remainders leave open
-// comes from an FP64 sum whose error bound rounds to one float; pixels with a
-// decision (or such a sum) left open go to a list, and walk_exact_kernel
-// bisects them with the oracle's ordered FP64 sums.  With that bisection inside
-// the walk the kernel kept a stack and spilled: 60 us instead of 46, and a
-// graph of the launches took 95 to 1300 ms to instantiate instead of 26.
+// Arithmetic: a channel's weights are the 32-bit integers floor(w 2^(32-e)),
+// 2^e the smallest power of two above the largest (remainder bound and
+// certification as for the tensor-core rounds' 31-bit ones), so a running sum
+// is the exact term total R, in 64-bit integers and in any order.  A winner's
+// value that the remainders leave open comes from an FP64 sum whose error bound
+// rounds to one float; pixels with a decision (or such a sum) left open go to a
+// list, and walk_exact_kernel bisects them with the oracle's ordered FP64 sums
+// (with that bisection inside the walk the kernel kept a stack and spilled: 60
+// us instead of 46).
 
 // Bytes 1 where the first-spike byte f <= t, else 0; tt = (t + 1) * 0x01010101
 // ((f | 0x80) - (t + 1) keeps bit 7 iff f > t, no borrow between bytes).
