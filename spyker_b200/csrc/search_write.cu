@@ -143,6 +143,8 @@ struct TableSource
 };
 
 // Positions [lo, hi) of every step's slab (C x hw bytes from dst + step * slab).
+// Off the search path (!lean) they are zero and the source is not read: its
+// arrays are then unwritten, and the table of a large pooled map has no bytes.
 template <typename Source>
 __device__ __forceinline__ void write_range(uint8_t *dst, int T, int slab, int lo, int hi, bool lean, bool wide,
                                             const Source &src)
@@ -151,9 +153,8 @@ __device__ __forceinline__ void write_range(uint8_t *dst, int T, int slab, int l
     {
         for (int f = lo + 16 * threadIdx.x; f < hi; f += 16 * kThreads)
         {
-            uint32_t eq[4], tw[4];
-            src.get(f, eq, tw);
-            if (!lean) eq[0] = eq[1] = eq[2] = eq[3] = 0u;
+            uint32_t eq[4] = {}, tw[4] = {};
+            if (lean) src.get(f, eq, tw);
             for (int t = 0; t < T; ++t)
             {
                 const uint32_t t4 = uint32_t(t) * 0x01010101u;
@@ -188,9 +189,8 @@ __device__ __forceinline__ void write_range(uint8_t *dst, int T, int slab, int l
                 for (int g = max(f, lo); g < min(f + 16, hi); ++g) run[g] = lean ? src.one(g, t) : uint8_t(0);
                 continue;
             }
-            uint32_t eq[4], tw[4];
-            src.get(f, eq, tw);
-            if (!lean) eq[0] = eq[1] = eq[2] = eq[3] = 0u;
+            uint32_t eq[4] = {}, tw[4] = {};
+            if (lean) src.get(f, eq, tw);
             const uint32_t t4 = uint32_t(t) * 0x01010101u;
             *reinterpret_cast<uint4 *>(run + f) =
                 make_uint4((eq[0] & bytes_le(tw[0], t4)) >> 7, (eq[1] & bytes_le(tw[1], t4)) >> 7,
