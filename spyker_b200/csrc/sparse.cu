@@ -556,16 +556,27 @@ __global__ void sparse_conv_kernel(const int64_t *__restrict__ offsets, const ui
 //
 // Needs thr >= 0 (an untouched neuron stays below it) and rows of at most 64
 // neurons.
+//
+// A parked neuron cannot fire again unless some weight reaches kLifts: below it
+// an addition is less than half the spacing of floats at FLT_MAX and leaves
+// -FLT_MAX as it is.  With such weights a map may list more events than it has
+// neurons, and the surplus of the whole map is dropped, which bands cannot
+// count for one another: the warps of a group then take its maps one by one, as
+// the kernel above does, each with the map's plane in its band's memory.
 constexpr int kBandBytes = 14 * 1024;
+constexpr float kLifts = 0x1p103f;
 
-// [group of 32 maps][input map and tap][32]
+// [group of 32 maps][input map and tap][32]; *lifts where a weight is kLifts or
+// more
 __global__ void sparse_weights_kernel(const float *__restrict__ kernel, float *__restrict__ wt, int cout, int groups,
-                                      int k)
+                                      int k, int32_t *__restrict__ lifts)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < groups * k * 32; i += gridDim.x * blockDim.x)
     {
         const int l = i & 31, r = (i >> 5) % k, q = (i >> 5) / k * 32 + l;
-        wt[i] = q < cout ? kernel[int64_t(q) * k + r] : 0.f;
+        const float w = q < cout ? kernel[int64_t(q) * k + r] : 0.f;
+        wt[i] = w;
+        if (!(fabsf(w) < kLifts)) atomicOr(lifts, 1);
     }
 }
 
@@ -577,10 +588,60 @@ struct MapsArgs
     uint16_t *fired;   // [u][cout][oh * ow]: band b's from its first neuron's slot on
     uint16_t *ends;    // [u * t][bands][cout]: fired neurons of the band up to the step
     int32_t *counts;   // [u * t]
+    const int32_t *lifts;
     int64_t tasks;
+    int region;        // floats of shared memory of a warp
     int t, c, cout, groups, bands, rows, top, left, oh, ow;
     float thr;
 };
+
+// Maps q0, q0 + qstep, .. of a group (weights that lift parked neurons): a map's
+// whole plane at a time, lanes over the taps of an event.  Band 0 counts all of a
+// map's events (they are listed from the map's first slot on), the others none.
+template <int KH, int KW>
+__device__ __noinline__ void sparse_whole_maps(const MapsArgs &A, int64_t s, int g, int q0, int qstep, float *pot)
+{
+    const int lane = threadIdx.x & 31, ohw = A.oh * A.ow;
+    for (int l = q0; l < 32 && g * 32 + l < A.cout; l += qstep)
+    {
+        const int q = g * 32 + l;
+        for (int i = lane; i < ohw; i += 32) pot[i] = 0.f;
+        __syncwarp();
+        const float *wq = A.wt + int64_t(g) * A.c * KH * KW * 32 + l;
+        uint16_t *slot = A.fired + (s * A.cout + q) * int64_t(ohw);
+        int done = 0;
+        for (int step = 0; step < A.t; ++step)
+        {
+            const int64_t b = A.offsets[s * A.t + step], e = A.offsets[s * A.t + step + 1];
+            for (int64_t k = b; k < e; ++k)
+            {
+                const uint32_t ev = A.events[k];
+                const int ky = lane / KW, y = ev_y(ev) + A.top - ky, x = ev_x(ev) + A.left - (lane - ky * KW);
+                if (ev_z(ev) < A.c && lane < KH * KW && y >= 0 && y < A.oh && x >= 0 && x < A.ow)
+                    pot[y * A.ow + x] += wq[(ev_z(ev) * (KH * KW) + lane) * 32];
+                __syncwarp();
+            }
+            const int before = done;
+            for (int i0 = 0; e > b && i0 < ohw; i0 += 32)
+            {
+                const int i = i0 + lane;
+                const bool f = i < ohw && pot[i] > A.thr;
+                const unsigned m = __ballot_sync(0xffffffffu, f);
+                const int at = done + __popc(m & ((1u << lane) - 1u));
+                if (f)
+                {
+                    if (at < ohw) slot[at] = uint16_t(i);
+                    pot[i] = -FLT_MAX;
+                }
+                done = min(done + __popc(m), ohw);
+            }
+            __syncwarp();
+            if (lane == 0 && done > before) atomicAdd(&A.counts[s * A.t + step], done - before);
+            for (int band = lane; band < A.bands; band += 32)
+                A.ends[((s * A.t + step) * A.bands + band) * A.cout + q] = uint16_t(band == 0 ? done : 0);
+        }
+    }
+}
 
 template <int KH, int KW>
 __global__ void __launch_bounds__(128) sparse_conv_maps_kernel(MapsArgs A)
@@ -591,9 +652,15 @@ __global__ void __launch_bounds__(128) sparse_conv_maps_kernel(MapsArgs A)
     if (task >= A.tasks) return;
     const int64_t s = task / (A.groups * A.bands);
     const int gb = int(task - s * (A.groups * A.bands)), g = gb / A.bands, band = gb - g * A.bands;
+    const int32_t lifts = *A.lifts;
     const int q = g * 32 + lane, y0 = band * A.rows, ny = min(A.rows, A.oh - y0), most = ny * ow;
-    float *pot = splanes + int64_t(warp) * A.rows * ow * 32 + lane;
+    float *pot = splanes + int64_t(warp) * A.region + lane;
     for (int i = 0; i < most; ++i) pot[i * 32] = 0.f;
+    if (lifts)
+    {
+        sparse_whole_maps<KH, KW>(A, s, g, band, A.bands, splanes + int64_t(warp) * A.region);
+        return;
+    }
     uint64_t mask = 0;  // lane r: the touched neurons of the band's row r
     uint16_t *slot = A.fired + (s * A.cout + q) * (int64_t(A.oh) * ow) + y0 * ow;
     const float *wg = A.wt + int64_t(g) * A.c * KH * KW * 32 + lane;
@@ -705,10 +772,8 @@ __global__ void __launch_bounds__(128) sparse_conv_maps_kernel(MapsArgs A)
                         {
                             const int j = __ffs(hit) - 1;
                             hit &= hit - 1;
-                            p[j * 32] = -FLT_MAX;
-                            // (a parked neuron fires again only if additions of
-                            // about FLT_MAX lift it back; extra events are dropped)
-                            if (done < most) slot[done++] = uint16_t((y0 + r) * ow + x0 + j);
+                            p[j * 32] = -FLT_MAX;  // for good: each neuron fires once
+                            slot[done++] = uint16_t((y0 + r) * ow + x0 + j);
                         }
                 }
             }
@@ -782,15 +847,18 @@ bool conv_maps(const int64_t *offsets, const uint32_t *events, int64_t u, int t,
     Carve cv{rest};
     float *wt = cv.take<float>(size_t(k) * groups * 32);
     uint16_t *ends = cv.take<uint16_t>(size_t(lists) * bands * cout);
-    int32_t *counts = cv.take<int32_t>(size_t(lists));
+    int32_t *counts = cv.take<int32_t>(size_t(lists) + 1);  // and the weights' flag
     void *scan_ws = cv.take<char>(scan_workspace(lists));
     if (cv.used > rest_bytes || ceil_div(tasks, 4) > 0x7FFFFFFF) return false;
-    sparse_weights_kernel<<<grid_for(int64_t(k) * groups * 32, 256), 256, 0, s>>>(kernel, wt, cout, groups, k);
+    SPK_CUDA(cudaMemsetAsync(counts, 0, size_t(lists + 1) * 4, s));
+    sparse_weights_kernel<<<grid_for(int64_t(k) * groups * 32, 256), 256, 0, s>>>(kernel, wt, cout, groups, k,
+                                                                                 counts + lists);
     SPK_LAUNCHED();
-    SPK_CUDA(cudaMemsetAsync(counts, 0, size_t(lists) * 4, s));
-    const int64_t plane = int64_t(rows) * ow * 128;
+    // a warp's memory: a band of 32 maps, or one map's plane (the smaller up to
+    // 32 bands)
+    const int64_t plane = std::max<int64_t>(int64_t(rows) * ow * 128, int64_t(oh) * ow * 4);
     const int wpc = plane * 4 <= 100 * 1024 ? 4 : 1;
-    const MapsArgs A{offsets, events, wt,     fired, ends,       counts,      tasks, t, c, cout,
+    const MapsArgs A{offsets, events, wt,     fired, ends,       counts,      counts + lists, tasks, int(plane / 4), t, c, cout,
                      groups,  bands,  rows,   int(p.top), int(p.left), oh,    ow,    thr};
     const auto kern = k5 ? sparse_conv_maps_kernel<5, 5> : sparse_conv_maps_kernel<3, 3>;
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wpc * plane)));
