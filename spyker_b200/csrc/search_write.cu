@@ -34,6 +34,7 @@ namespace
 constexpr int kThreads = 256;
 constexpr int kSmemPixels = 16384;    // larger maps keep their bytes in global memory
 constexpr int kTableBytes = 48 * 1024;  // pooled table of a CTA's channel range
+constexpr int64_t kRangeBytes = int64_t(1) << 30;  // a range's bytes of a step
 constexpr int kTableMax = 160 * 1024;   // of one channel; above it cells are read from their windows
 
 // bytes of one sample's extended array: the map, 16 bytes more, and what
@@ -102,15 +103,16 @@ struct WriteArgs
     int ptab;  // pooled cells from a table in shared memory
 };
 
-// The chunk of 16 bytes of (channel, pixel) positions f .. f + 15 of a step:
-// as 0x80 flags of the pixels won by their channel, and first steps.
+// The chunk of 16 bytes of (channel, pixel) positions f .. f + 15 of a step's run
+// (from the range's first channel on): as 0x80 flags of the pixels won by their
+// channel, and first steps.
 struct SpikeSource
 {
     const uint8_t *w, *t;
-    int hw;
+    int hw, c0;
     __device__ __forceinline__ void get(int f, uint32_t (&eq)[4], uint32_t (&tw)[4]) const
     {
-        const int c = f / hw, px = f - c * hw;
+        const int k = f / hw, px = f - k * hw, c = c0 + k;
         load16u(w + px, eq);
         load16u(t + px, tw);
         const uint32_t c4 = uint32_t(c) * 0x01010101u, d4 = uint32_t(c + 1) * 0x01010101u;
@@ -124,54 +126,53 @@ struct SpikeSource
     }
     __device__ __forceinline__ uint8_t one(int f, int step) const
     {
-        const int c = f / hw, px = f - c * hw;
-        return int(w[px]) == c && int(t[px]) <= step;
+        const int k = f / hw, px = f - k * hw;
+        return int(w[px]) == c0 + k && int(t[px]) <= step;
     }
 };
 
 struct TableSource
 {
     const uint8_t *first;  // [channel][cell] from the range's first channel
-    int f0;                // position of first[0]
     __device__ __forceinline__ void get(int f, uint32_t (&eq)[4], uint32_t (&tw)[4]) const
     {
-        load16u(first + (f - f0), tw);
+        load16u(first + f, tw);
 #pragma unroll
         for (int j = 0; j < 4; ++j) eq[j] = 0x80808080u;
     }
-    __device__ __forceinline__ uint8_t one(int f, int step) const { return int(first[f - f0]) <= step; }
+    __device__ __forceinline__ uint8_t one(int f, int step) const { return int(first[f]) <= step; }
 };
 
-// Positions [lo, hi) of every step's slab (C x hw bytes from dst + step * slab).
-// Off the search path (!lean) they are zero and the source is not read: its
-// arrays are then unwritten, and the table of a large pooled map has no bytes.
+// The n bytes from dst on of every step's slab (slab bytes apart).  Off the
+// search path (!lean) they are zero and the source is not read: its arrays are
+// then unwritten, and the table of a large pooled map has no bytes.
 template <typename Source>
-__device__ __forceinline__ void write_range(uint8_t *dst, int T, int slab, int lo, int hi, bool lean, bool wide,
+__device__ __forceinline__ void write_range(uint8_t *dst, int T, int64_t slab, int n, bool lean, bool wide,
                                             const Source &src)
 {
-    if (wide && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && slab % 16 == 0 && lo % 16 == 0 && hi % 16 == 0)
+    if (wide && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && slab % 16 == 0 && n % 16 == 0)
     {
-        for (int f = lo + 16 * threadIdx.x; f < hi; f += 16 * kThreads)
+        for (int f = 16 * threadIdx.x; f < n; f += 16 * kThreads)
         {
             uint32_t eq[4] = {}, tw[4] = {};
             if (lean) src.get(f, eq, tw);
             for (int t = 0; t < T; ++t)
             {
                 const uint32_t t4 = uint32_t(t) * 0x01010101u;
-                *reinterpret_cast<uint4 *>(dst + int64_t(t) * slab + f) =
+                *reinterpret_cast<uint4 *>(dst + t * slab + f) =
                     make_uint4((eq[0] & bytes_le(tw[0], t4)) >> 7, (eq[1] & bytes_le(tw[1], t4)) >> 7,
                                (eq[2] & bytes_le(tw[2], t4)) >> 7, (eq[3] & bytes_le(tw[3], t4)) >> 7);
             }
         }
         return;
     }
-    const int n = hi - lo;
     if (!wide || n < 64)
     {
+        // (planes of fewer than 16 pixels, or few bytes)
         for (int i = threadIdx.x; i < T * n; i += kThreads)
         {
-            const int t = i / n, f = lo + i - t * n;
-            dst[int64_t(t) * slab + f] = lean ? src.one(f, t) : uint8_t(0);
+            const int t = i / n, f = i - t * n;
+            dst[t * slab + f] = lean ? src.one(f, t) : uint8_t(0);
         }
         return;
     }
@@ -181,12 +182,12 @@ __device__ __forceinline__ void write_range(uint8_t *dst, int T, int slab, int l
         for (int i = threadIdx.x; i < min(tn, T - tb) * per; i += kThreads)
         {
             const int dt = i / per, k = i - dt * per, t = tb + dt;
-            uint8_t *run = dst + int64_t(t) * slab;
-            const int f = lo - int(reinterpret_cast<uintptr_t>(run + lo) & 15) + 16 * k;
-            if (f >= hi) continue;
-            if (f < lo || f + 16 > hi)
+            uint8_t *run = dst + t * slab;
+            const int f = 16 * k - int(reinterpret_cast<uintptr_t>(run) & 15);
+            if (f >= n) continue;
+            if (f < 0 || f + 16 > n)
             {
-                for (int g = max(f, lo); g < min(f + 16, hi); ++g) run[g] = lean ? src.one(g, t) : uint8_t(0);
+                for (int g = max(f, 0); g < min(f + 16, n); ++g) run[g] = lean ? src.one(g, t) : uint8_t(0);
                 continue;
             }
             uint32_t eq[4] = {}, tw[4] = {};
@@ -250,14 +251,14 @@ __global__ void __launch_bounds__(kThreads) search_write_kernel(WriteArgs A)
                 __syncthreads();
             }
         }
-        write_range(A.spikes + smp * A.T * int64_t(A.C) * ohw, A.T, A.C * ohw, c0 * ohw, c1 * ohw, lean, ohw >= 16,
-                    SpikeSource{wsrc, tsrc, ohw});
+        const int64_t slab = int64_t(A.C) * ohw, pslab = int64_t(A.C) * phw;
+        write_range(A.spikes + smp * A.T * slab + int64_t(c0) * ohw, A.T, slab, (c1 - c0) * ohw, lean, ohw >= 16,
+                    SpikeSource{wsrc, tsrc, ohw, c0});
         if (A.pooled)
         {
-            uint8_t *dst = A.pooled + smp * A.T * int64_t(A.C) * phw;
+            uint8_t *dst = A.pooled + smp * A.T * pslab + int64_t(c0) * phw;
             if (A.ptab || !lean)
-                write_range(dst, A.T, A.C * phw, c0 * phw, c1 * phw, lean, true,
-                            TableSource{first, c0 * phw});
+                write_range(dst, A.T, pslab, (c1 - c0) * phw, lean, true, TableSource{first});
             else
                 for (int64_t i = threadIdx.x; i < int64_t(c1 - c0) * phw; i += kThreads)
                 {
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(kThreads) search_write_kernel(WriteArgs A)
                             const int q = (py * A.pky + dy) * A.ow + px * A.pkx + dx;
                             if (int(wsrc[q]) == c) m = min(m, int(tsrc[q]));
                         }
-                    for (int t = 0; t < A.T; ++t) dst[int64_t(t) * A.C * phw + int64_t(c) * phw + cell] = m <= t;
+                    for (int t = 0; t < A.T; ++t) dst[t * pslab + i] = m <= t;
                 }
         }
         __syncthreads();
@@ -282,7 +283,6 @@ void search_write(const SearchWrite &W, cudaStream_t s)
     const int64_t ohw = int64_t(W.oh) * W.ow, phw = W.pooled ? int64_t(W.poh) * W.pow_ : 0;
     WriteArgs A{W.records, nullptr, W.negw, W.flag, W.spikes, W.pooled, W.b, W.T, W.C, int(ohw), W.ow, W.pky, W.pkx,
                 W.poh, W.pow_, W.C, 0};
-    SPK_REQUIRE(int64_t(W.C) * ohw < (int64_t(1) << 31) - 65536, "a step's spikes of one sample exceed 2^31 bytes");
     if (ohw > kSmemPixels)
     {
         A.codes = W.codes;
@@ -293,15 +293,17 @@ void search_write(const SearchWrite &W, cudaStream_t s)
     A.ptab = W.pooled && phw <= kTableMax ? 1 : 0;
     // Channel ranges: enough CTAs for a few per SM when there are few samples
     // (each CTA reads the whole map's records once more), as many as keep
-    // the pooled table small, in steps that keep the runs 16-byte aligned.
+    // the pooled table small and a range's bytes of a step below 2^31 (its
+    // positions are 32-bit), in steps that keep the runs 16-byte aligned.
     int64_t g = 16, r = ohw;
     while (r) { const int64_t q = g % r; g = r, r = q; }  // gcd(16, ohw)
     const int64_t unit = 16 / g;
     const int64_t want = ceil_div(int64_t(sm_count()) * 6, W.b);
     int64_t nc = ceil_div(W.C, std::min<int64_t>(want, W.C));
     if (A.ptab && phw > 0) nc = std::min<int64_t>(nc, std::max<int64_t>(1, kTableBytes / phw));
+    nc = std::min(nc, std::max<int64_t>(1, kRangeBytes / ohw));
     if (nc >= unit) nc = nc / unit * unit;
-    else if (phw * unit <= kTableBytes) nc = std::min<int64_t>(unit, W.C);
+    else if (phw * unit <= kTableBytes && ohw * unit <= kRangeBytes) nc = std::min<int64_t>(unit, W.C);
     A.nc = int(nc);
     const size_t smem = (A.codes ? 0 : size_t(2 * ext_bytes(ohw))) + (A.ptab ? size_t(nc * phw + 32) & ~size_t(15) : 0);
     SPK_CUDA(cudaFuncSetAttribute(search_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
