@@ -3923,9 +3923,14 @@ void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b
     // large for a warp's registers; then a warp per sample (4096 of 784 and of
     // 196: 73 us against 82)
     if (hw > 1024 || b <= 8 * sm_count())
+    {
+        // (keys and positions of up to 16384 pixels: 128 KB)
+        if (hw > 4096)
+            SPK_CUDA(cudaFuncSetAttribute(wta_records_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hw * 8));
         wta_records_kernel<<<unsigned(b), hw <= 256 ? 128 : hw <= 1024 ? 256 : hw <= 4096 ? 512 : 1024, size_t(hw) * 8,
                              s>>>(P.records, P.mins, P.maxs, hw, int(L.ow), int(t), int(ry), int(rx), int(count), winners,
                                   counts);
+    }
     else if (hw <= 256)
         wta_records_warp_kernel<8><<<wgrid, 128, 0, s>>>(P.records, P.mins, P.maxs, b, hw, int(L.ow), int(t), int(ry),
                                                           int(rx), int(count), winners, counts);
