@@ -24,6 +24,7 @@
 //    step its lanes update different pixels and the order of the sums (map,
 //    then position) is fixed.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 
 #include "fst_grad.cuh"
@@ -193,6 +194,26 @@ __global__ void __launch_bounds__(kMaxTapGroups * 32)
         if (zw * ZP + u < nz) part[(blockIdx.z * int64_t(F.cout) + z0 + zw * ZP + u) * K + k] = acc[u];
 }
 
+// The terms of a block's zero gradients (output row `row`, positions p0 .. p0 +
+// np - 1), for weights that are not finite: the others add nothing there.
+template <int TP>
+__device__ __noinline__ void zero_terms(const FstGrad &F, const Stage &S, const float *s_in, float *mine,
+                                        const int (&off)[TP], const bool (&on)[TP], const float (&wv)[TP], int64_t row,
+                                        int p0, int np)
+{
+    for (int p = p0; p < p0 + np; ++p)
+    {
+        const float go = F.grad_out[row + p], to = F.t_out[row + p];
+        if (go != 0.f) continue;  // (in the list)
+        const int oy = p / F.ow, base = oy * F.sy * S.wp + (p - oy * F.ow) * F.sx;
+#pragma unroll
+        for (int u = 0; u < TP; ++u)
+            if (on[u] && !(fabsf(wv[u]) <= FLT_MAX) && s_in[base + off[u]] < to)
+                mine[base + off[u]] = __fmaf_rn(wv[u], go, mine[base + off[u]]);
+        __syncwarp();
+    }
+}
+
 // grid (channel blocks, samples); TP taps per lane (KK <= 32 * TP)
 template <int TP>
 __global__ void __launch_bounds__(512) fst_grad_in_kernel(FstGrad F, Stage S, float *__restrict__ gi, int cb,
@@ -250,6 +271,13 @@ __global__ void __launch_bounds__(512) fst_grad_in_kernel(FstGrad F, Stage S, fl
                                 mine[v.base + off[u]] = __fmaf_rn(wv[u], v.go, mine[v.base + off[u]]);
                         __syncwarp();  // the next entry's pixels overlap this one's
                     }
+                    // infinite and NaN weights meet the zero gradients too (NaN)
+                    bool odd = false;
+#pragma unroll
+                    for (int u = 0; u < TP; ++u) odd |= !(fabsf(wv[u]) <= FLT_MAX);
+                    if (__any_sync(0xffffffffu, odd))
+                        zero_terms<TP>(F, S, s_in, mine, off, on, wv, (s * F.cout + z0 + z) * int64_t(P), p0,
+                                       min(kPositions, P - p0));
                 }
             }
         }
