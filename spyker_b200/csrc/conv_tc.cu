@@ -3667,15 +3667,28 @@ struct Nets
 // device (each launch reads them).  Off the search path (device flags) every
 // one of these kernels leaves at once, except the writer, which zero-fills
 // the spikes for the dense kernel.
-// Up to how many output pixels the walk (search_walk.cuh) is the faster
-// search: its time grows with the pixels from a few microseconds, the rounds
-// start near 100 us (some 20 dependent launches) and then spend less per
-// pixel.  2 -> 30 channels 5 x 5: 50k pixels 46 against 140 us, 363k 340
-// against 230; 30 -> 100 channels: 0.2k 14 against 120, 85k 515 against 233.
-bool walk_pays(int64_t npix, int groups, int cout)
+// Whether the walk (search_walk.cuh) is the faster search.  Its time grows with
+// the pixels and, per pixel, with the inputs of a receptive field and the
+// channels a lane holds (at most some 0.02 ns a pixel and input for one channel a
+// lane, less the earlier the pixels cross); with fewer pixels than the chip has
+// warps it is the latency of one.  The rounds take some 35 us each (25 without
+// the pre-filter, whose launches join the first) before the pixels count.  The
+// line is where both take the same for a threshold of some 15 % of the summed
+// weights: an early crossing would put it at twice the pixels, one at 30 % at
+// half.  us, walk at 5 / 10 / 30 %, rounds, T = 15: 2 -> 30 channels 5 x 5, 131k
+// pixels 180 / 183 / 214, 271 (128 Ki at most); 8 -> 32, 44k 117 / 128 / 176, 260,
+// 87k 177 / 199 / 291, 290; 30 -> 100, 4.5k 107 / 123 / 192, 275, 9k 176 / 214 /
+// 360, 270, 14k 251 / 318 / 507, 270; 64 -> 64 3 x 3, 8.6k 110 / 121 / 166, 205,
+// 16k 153 / 171 / 253, 205, 34k 254 / 288 / 463, 228; 64 -> 32 5 x 5, 7.4k 151 /
+// 180 / 298, 240; 64 -> 100, 2.7k 140 / 176 / 303, 237; 8 -> 256, 12k 172 / 216 /
+// 356, 280; 64 -> 256, 2.3k 215 / 270 / 500, 300, 16k 2260 at 15 %, 650.
+bool walk_pays(int64_t npix, int inputs, int cout, int T, bool prefilter, bool wta)
 {
-    const bool small = groups <= 32 && cout <= 32;  // one load and one channel per lane
-    return npix <= (small ? 128 * 1024 : 20 * 1024);
+    int rounds = wta ? 2 : 1;
+    for (int steps = 1; steps < T; steps *= 2) ++rounds;
+    const double lane = cout <= 32 ? 1.0 : cout <= 64 ? 1.2 : cout <= 128 ? 2.75 : 7.5;  // 1, 2, 4, 8 channels
+    const double pixels = double(std::max<int64_t>(npix, 8 * sm_count()));
+    return npix <= 128 * 1024 && pixels * (inputs + 20) * lane <= rounds * (prefilter ? 3.6e6 : 2.4e6);
 }
 
 void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel, int64_t count, int64_t pool_ky,
@@ -3714,10 +3727,21 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
                                  int(pool_kx), int(poh), int(pow_)},
                      s);
     };
+    // the bound pre-filter of round 0, for layers with few inputs per output
+    const int cp = P.nhwc ? P.cpad : P.cin;
+    const int kr = P.cin * taps;
+    // with T <= 32 the pre-filter also bounds each pixel's first step (a bin
+    // per step and thread, and the map's bytes, in shared memory)
+    const bool want_tlo = P.T <= 32;
+    const int64_t bound_base = ((int64_t(P.h) * P.w * 4 + 15) & ~int64_t(15)) + ((int64_t(taps) * P.cpad * 4 + 15) & ~int64_t(15));
+    const int64_t bound_tlo = bound_base + ((int64_t(P.T) * 256 * 4 + 15) & ~int64_t(15)) + int64_t(P.h) * P.w * P.cpad;
+    const bool use_tlo = want_tlo && bound_tlo <= 48 * 1024;
+    const int64_t bound_smem = use_tlo ? bound_tlo : bound_base;
+    const bool prefilter = P.nhwc && P.cpad <= 32 && bound_smem <= 48 * 1024;
     // Walking each pixel's inputs in spike order (search_walk.cuh) instead of
     // the rounds below.
     const int groups = taps * (P.cpad / 8);
-    if (P.nhwc && P.T <= 32 && groups <= 256 && P.cout <= 256 && walk_pays(L.npix, groups, P.cout))
+    if (P.nhwc && P.T <= 32 && groups <= 256 && P.cout <= 256 && walk_pays(L.npix, kr, P.cout, P.T, prefilter, count > 0))
     {
         // (the integers take the weight image's bytes: four per input and
         // channel in both)
@@ -3737,17 +3761,6 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
         write();
         return;
     }
-    // the bound pre-filter of round 0, for layers with few inputs per output
-    const int cp = P.nhwc ? P.cpad : P.cin;
-    const int kr = P.cin * taps;
-    // with T <= 32 the pre-filter also bounds each pixel's first step (a bin
-    // per step and thread, and the map's bytes, in shared memory)
-    const bool want_tlo = P.T <= 32;
-    const int64_t bound_base = ((int64_t(P.h) * P.w * 4 + 15) & ~int64_t(15)) + ((int64_t(taps) * P.cpad * 4 + 15) & ~int64_t(15));
-    const int64_t bound_tlo = bound_base + ((int64_t(P.T) * 256 * 4 + 15) & ~int64_t(15)) + int64_t(P.h) * P.w * P.cpad;
-    const bool use_tlo = want_tlo && bound_tlo <= 48 * 1024;
-    const int64_t bound_smem = use_tlo ? bound_tlo : bound_base;
-    const bool prefilter = P.nhwc && P.cpad <= 32 && bound_smem <= 48 * 1024;
     unsigned *wmax = reinterpret_cast<unsigned *>(base + L.wm_off);
     uint8_t *tlo = base + L.tlo_off;
     const size_t bcn = align256((size_t(L.npix) / kCompactItems + 2) * 4) / 4;  // ints per count buffer
