@@ -353,10 +353,10 @@ spk_status spk_fst_conv_backward(const float *t_in, int64_t b, int64_t cin, int6
  * T when none, where potential(t) = conv of the cumulative spikes [t_in <= t]
  * (BF16x2/x3 split weights, the FP64 sum of the split terms rounded once to
  * F32, exactly as spk_conv's potentials followed by spk_rank_gather); the
- * potentials are never written.  With the queried workspace and weights that
- * fit it walks each pixel's inputs in time order, with a smaller one it
- * evaluates every step on the tensor cores; the results are the same up to
- * the FP64 sums' order.  t_in [B, Cin, H, W] F32 (values >= T =
+ * potentials are never written.  Layers of many steps for their inputs walk
+ * each pixel's inputs in time order (with the queried workspace), the others
+ * evaluate every step on the tensor cores; the results are the same up to
+ * the sums' order.  t_in [B, Cin, H, W] F32 (values >= T =
  * never); T <= 126; all output channels in one CTA (workspace query 0
  * otherwise). */
 size_t spk_fst_conv_times_workspace(int64_t b, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh,

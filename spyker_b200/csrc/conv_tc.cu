@@ -4011,10 +4011,13 @@ spk_status spk_fst_conv_times(const float *t_in, int64_t b, int64_t cin, int64_t
         if (b == 0) return;
         cudaStream_t s = stream_of(stream);
         // Walking each pixel's inputs in time order costs K additions a
-        // channel against the dense kernel's T x K products; the dense kernel
-        // is left to layers whose weights fit neither shared memory nor L1.
+        // channel against the dense kernel's T x K products: whichever is the
+        // faster, the walk where the dense kernel does not take the layer.
         const size_t walk = fst_walk_workspace(b, cin, h, w, cout, kh, kw);
-        if (walk > 0 && ws_bytes >= walk && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && oh * ow < (1 << 30))
+        const bool dense = pl.kblocks <= kMaxKBlocks && pl.stages >= 2 && pl.smem <= 227 * 1024 &&
+                           reinterpret_cast<uintptr_t>(ws) % 256 == 0;
+        if (walk > 0 && ws_bytes >= walk && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && oh * ow < (1 << 30) &&
+            (!dense || fst_walk_pays(npix, cin, kh * kw, cout, time)))
         {
             fst_walk(FstWalk{t_in, kernel, t_out, b, int(cin), int(h), int(w), int(cout), int(kh), int(kw), int(sy),
                              int(sx), int(p.top), int(p.left), int(oh), int(ow), int(time), float(threshold),

@@ -15,8 +15,11 @@
 // order, so the sums do not depend on scheduling), then the lanes, one channel
 // each (NG groups of 32), walk the list and compare at the last input of each
 // step.  Bound by the weight reads (8 bytes per channel and input) and the
-// sort's issue slots; the weights sit in shared memory as FP64 [k][channel]
-// where they fit, else they are read through L1.
+// sort's issue slots.  The weights, FP64 [k][channel], are read through L1; small
+// ones are copied to shared memory where a CTA has many pixels.  (Up to 150 KB
+// of them there took as long for many pixels, 128 images of 14 x 14, 32 -> 64 3 x 3:
+// 120 us against 113, and for few the copy by a CTA's few warps bounded the call,
+// 6 images: 117 against 24.)
 //
 // Arithmetic: the BF16 split terms (h + m, or h + m + l = the F32 weight) of a
 // weight are one exact FP64 number and the sums are FP64, the values that the
@@ -34,8 +37,8 @@ namespace spk
 namespace
 {
 constexpr int kMaxInputs = 4096;           // K: the list of a warp in shared memory
-constexpr size_t kSmemWeights = 150 * 1024;
-constexpr int64_t kL1Weights = 64 * 1024;  // weights read through L1 up to this count
+constexpr size_t kSmemWeights = 16 * 1024;
+constexpr int64_t kMaxWeights = 64 * 1024;  // K x channels: read through L1
 constexpr int kTile = 128;
 constexpr int kBatch = 4;  // rounds of input times in flight
 // warps per CTA (registers: 64, 80 or 128 a thread)
@@ -106,6 +109,8 @@ __global__ void __launch_bounds__(max_warps(NG) * 32) fst_walk_kernel(WalkArgs A
             const int k = i / nz;
             s_w[i] = A.wt[int64_t(k) * A.cout + z0 + (i - k * nz)];
         }
+    // (loads through a pointer of either space: with global loads in their place
+    // the compiler's order of the walk is 3 to 15 % slower)
     const double *wbase = A.smem_weights ? s_w : A.wt + z0;
     const int wstride = A.smem_weights ? nz : A.cout;
     int zi[NG];
@@ -330,10 +335,10 @@ WalkPlan walk_plan(int64_t npix, int64_t K, int64_t cout)
     WalkPlan pl{};
     pl.ng = cout <= 32 ? 1 : cout <= 64 ? 2 : 4;
     const int64_t nz = std::min<int64_t>(cout, 32 * pl.ng);
-    pl.smem_weights = size_t(K) * nz * 8 <= kSmemWeights;
     // tiles of up to 128 pixels, smaller while they leave SMs without one
     pl.tile = kTile;
     while (pl.tile > 1 && ceil_div(npix, pl.tile) < 2 * sm_count()) pl.tile /= 2;
+    pl.smem_weights = pl.tile >= 32 && size_t(K) * nz * 8 <= kSmemWeights;
     const size_t word = size_t(K + 128 + (K + 3) / 4) * 4;
     const size_t fixed = (pl.smem_weights ? size_t(K) * nz * 8 : 0) + size_t(K) * 8 + size_t(nz) * pl.tile;
     pl.warps = std::min(max_warps(pl.ng), pl.tile);
@@ -342,14 +347,53 @@ WalkPlan walk_plan(int64_t npix, int64_t K, int64_t cout)
     pl.smem = fixed + pl.warps * word + 16;
     return pl;
 }
+// Warps per CTA of the per-step sums, 0 where a warp per pixel takes the layer:
+// few CTAs (three an SM, all resident), up to 64 steps to sum over, and no more
+// weight reads than the L2 brings in the time of one pixel's walk.  us, sums /
+// warp per pixel / dense kernel: fc 3136 -> 10, T = 64, 37 samples 43-53 / 86-211 /
+// 57, 256 54-63 / 86-216 / 61, 590 92-112 / 87-216 / 96; T = 126, 256 80-119 / 86-213 /
+// 92; 32 -> 64 3 x 3 on one 14 x 14, T = 16 21-23 / 27-45 / 33, T = 64 38-67 / 25-44 / 32.
+int step_warps(int64_t npix, int64_t K, int64_t cout, int64_t time)
+{
+    if (K < 256 || time > 64 || npix * K * cout > (int64_t(1) << 24)) return 0;
+    const int64_t nz = std::min<int64_t>(cout, kStepMaps);
+    const int64_t warps = std::min({int64_t(kStepWarps), ceil_div(K, 32), 160 * 1024 / (time * nz * 8)});
+    const int64_t resident = std::min<int64_t>(3, 225 * 1024 / (warps * time * nz * 8 + 1024)) * sm_count();
+    return npix * ceil_div(cout, kStepMaps) <= resident ? int(warps) : 0;
+}
 }  // namespace
+
+// The walk's time grows with the pixels, inputs and channels a lane, the dense
+// kernel's with the pixels and steps (rounded up to a power of two), its K
+// blocks or its columns; both start from the latency of one pixel, or of one
+// tile.  The line is where both take the same for a threshold that the pixels
+// reach after about a third of their inputs.  us, walk at 10 / 50 % of the summed
+// weights, dense, 256 images of 14 x 14: 32 -> 64 3 x 3, T = 8 217 / 446 / 212, 16
+// 212 / 441 / 384, 64 230 / 468 / 1440; 64 -> 64, T = 16 378 / 906 / 437, 64 407 /
+// 931 / 1615; 128 -> 32, T = 16 552 / 1300 / 577, 64 618 / 1373 / 2125; 8 -> 128 5 x 5,
+// T = 8 247 / 486 / 360; 28 x 28, 1 -> 32 5 x 5, T = 4 170 / 225 / 193, 8 161 / 233 / 360.
+// 12 images of 14 x 14, T = 16: 32 -> 64 26 / 40 / 39, 128 -> 16 47 / 89 / 48.
+bool fst_walk_pays(int64_t npix, int64_t cin, int64_t taps, int64_t cout, int64_t time)
+{
+    const int64_t K = cin * taps;
+    if (step_warps(npix, K, cout, time)) return true;
+    const int64_t kblocks = ceil_div(taps * ceil_div(cin, 8) * 8, 64), columns = ceil_div(cout, 16) * 16;
+    int64_t steps = 1;
+    while (steps < time) steps *= 2;
+    // ns
+    const double input = cout <= 32 ? 0.019 : cout <= 64 ? 0.023 : 0.034;
+    const double walk = 12e3 + double(std::max<int64_t>(npix * ceil_div(cout, 128), 16 * sm_count())) * (0.6 + input * K);
+    const double row = 0.04 + std::max(0.034 * kblocks, 0.0062 * columns);
+    const double dense = 22e3 + 650.0 * kblocks + 100.0 * columns +
+                         double(std::max<int64_t>(npix * steps - 128 * sm_count(), 0)) * row;
+    return walk <= dense;
+}
 
 size_t fst_walk_workspace(int64_t b, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh, int64_t kw)
 {
     const int64_t K = cin * kh * kw;
     if (K > kMaxInputs || kh > 255 || kw > 255 || cin * h * w >= (int64_t(1) << 30)) return 0;
-    const int64_t nz = std::min<int64_t>(cout, cout <= 32 ? 32 : cout <= 64 ? 64 : 128);
-    if (size_t(K) * nz * 8 > kSmemWeights && K * cout > kL1Weights) return 0;
+    if (K * cout > kMaxWeights) return 0;
     return align256(size_t(K) * cout * 8) + align256(size_t(b) * cin * h * w);
 }
 
@@ -368,12 +412,9 @@ void fst_walk(const FstWalk &F, void *ws, cudaStream_t s)
     WalkArgs A{map,  wt,     F.t_out, npix,   F.cin, F.h,           F.w,    F.cout, F.kh,    F.kw,
                F.sy, F.sx,   F.top,   F.left, F.ow,  F.oh * F.ow,   F.time, K,      pl.tile, pl.smem_weights,
                rounding_bound(F.threshold)};
-    // at most four pixels per SM: per-step sums by all warps of a CTA
-    if (npix <= 4 * sm_count() && K >= 256 && ceil_div(F.cout, kStepMaps) <= 65535)
+    if (const int warps = step_warps(npix, K, F.cout, F.time))
     {
-        const int nz = std::min(F.cout, kStepMaps);
-        const int warps = int(std::min<int64_t>(kStepWarps, std::min<int64_t>(ceil_div(K, 32), 160 * 1024 / (F.time * nz * 8))));
-        const size_t smem = size_t(warps) * F.time * nz * 8;
+        const size_t smem = size_t(warps) * F.time * std::min(F.cout, kStepMaps) * 8;
         SPK_CUDA(cudaFuncSetAttribute(fst_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         fst_steps_kernel<<<dim3(unsigned(npix), unsigned(ceil_div(F.cout, kStepMaps))), warps * 32, smem, s>>>(A);
         SPK_LAUNCHED();

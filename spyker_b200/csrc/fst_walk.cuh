@@ -19,5 +19,7 @@ struct FstWalk
 
 // Bytes of scratch, 0 where the walk does not apply.
 size_t fst_walk_workspace(int64_t b, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh, int64_t kw);
+// Whether it is the faster one of the two forms (the dense kernel's: conv_tc.cu).
+bool fst_walk_pays(int64_t npix, int64_t cin, int64_t taps, int64_t cout, int64_t time);
 void fst_walk(const FstWalk &F, void *ws, cudaStream_t s);
 }  // namespace spk
