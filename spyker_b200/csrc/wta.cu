@@ -289,11 +289,21 @@ size_t keys_bytes(int64_t b, int64_t x) { return x <= kWtaSmemKeys ? 0 : (size_t
 // the scan's candidates: block extremes, values, steps
 size_t candidate_bytes(int64_t b, int64_t x) { return size_t(b) * (size_t(ceil_div(x, kScanThreads)) * 8 + size_t(x) * 6); }
 
-bool scan_applies(int64_t t, int64_t x) { return t * x >= 16384 && t < kNever && x < (int64_t(1) << 31); }
+// The scan pays where one CTA's two readings of a sample (some 80 ps a value)
+// take longer than the second launch (some 8 us) and the scan's T steps (0.1 us
+// each); sooner where the samples are several waves of CTAs.  us, scan and rounds
+// / one CTA, 1 winner: 1 sample of 1000 steps x 100 positions 128 / 23, 100 x 800 33 /
+// 23, 100 x 2000 33 / 29, 15 x 1890 30 / 22, 15 x 7000 23 / 25, 15 x 10000 25 / 29; 64 of
+// 100 x 1400 43 / 26, 100 x 2200 49 / 31; 512 of 60 x 400 57 / 39, 15 x 1890 60 / 45, 15 x 4000 68 / 82, 15 x
+// 7000 86 / 114.
+bool scan_applies(int64_t b, int64_t t, int64_t x)
+{
+    return t * (x - 1250) > (b > sm_count() ? 25000 : 120000) && t < kNever && x < (int64_t(1) << 31);
+}
 
 size_t wta_workspace(int64_t b, int64_t t, int64_t x)
 {
-    return keys_bytes(b, x) + (scan_applies(t, x) ? candidate_bytes(b, x) : 0);
+    return keys_bytes(b, x) + (scan_applies(b, t, x) ? candidate_bytes(b, x) : 0);
 }
 
 template <typename T, bool kFloat>
@@ -319,7 +329,7 @@ void launch_wta(const void *in, int64_t b, int64_t t, int64_t c, int64_t h, int6
     if constexpr (std::is_same<T, float>::value)
     {
         const size_t all = used + candidate_bytes(b, x);
-        if (scan_applies(t, x) && b <= 65535 && ws != nullptr && ws_bytes >= all &&
+        if (scan_applies(b, t, x) && b <= 65535 && ws != nullptr && ws_bytes >= all &&
             reinterpret_cast<uintptr_t>(ws) % 8 == 0)
         {
             char *base = static_cast<char *>(ws) + used;
