@@ -830,13 +830,16 @@ __global__ void conv_runs_kernel(const uint16_t *__restrict__ fired, const uint1
     }
 }
 
-// The lane-per-map form of a whole call; false where it does not apply.
+// The lane-per-map form of a whole call; false where it does not apply, or for
+// fewer than 12 maps, which leave most lanes idle (us, lanes / a warp per map: 500
+// samples of 2 x 28 x 28 at 2 %, 1 map 132 / 84, 8 133 / 110, 12 137 / 143; 2000 at 10 %,
+// 1 map 673 / 137, 8 678 / 463, 12 692 / 654, 30 860 / 1520).
 bool conv_maps(const int64_t *offsets, const uint32_t *events, int64_t u, int t, int c, const float *kernel, int cout,
                int kh, int kw, Pad4 p, int oh, int ow, float thr, uint16_t *fired, char *rest, size_t rest_bytes,
                int64_t *out_offsets, uint32_t *out_events, cudaStream_t s)
 {
     const bool k5 = kh == 5 && kw == 5, k3 = kh == 3 && kw == 3;
-    if (!(thr >= 0.f) || ow > 64 || !(k5 || k3) || p.top > 65535 || p.left > 65535) return false;
+    if (!(thr >= 0.f) || cout < 12 || ow > 64 || !(k5 || k3) || p.top > 65535 || p.left > 65535) return false;
     // bands of equal height; at most 32 rows (a lane per row)
     int bands = (oh * ow * 128 + kBandBytes - 1) / kBandBytes;
     int rows = (oh + bands - 1) / bands;

@@ -18,6 +18,8 @@ SHAPES = [
     (1, 12, 2, 60, 60, 3, 5, 2, 10),
     (1, 9, 3, 100, 40, 5, 3, 1, 30),  # more than 32 bands
     (3, 6, 3, 10, 10, 64, 5, 2, 10),  # one band
+    (1, 12, 2, 60, 60, 13, 5, 2, 10),
+    (1, 9, 3, 100, 40, 12, 3, 1, 30),  # more than 32 bands, a lane per map
 ]
 
 
