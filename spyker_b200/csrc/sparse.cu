@@ -344,8 +344,11 @@ __global__ void remap_offsets_kernel(const int64_t *__restrict__ offsets, int64_
 // events, flags the events that stay (a byte each) and counts them per list;
 // after a scan of the lists' counts a warp per list moves its events.  Nothing
 // is sized by the lists' capacity: filling and scanning maps of all cells and
-// all possible events took 2.3 ms of the 4096-image event step (9.5 ms).
-constexpr int kFilterThreads = 256;
+// all possible events took 2.3 ms of the 4096-image event step (9.5 ms).  Long
+// lists of few samples wait for one event after another, so a lane has several
+// in flight: inhibition of 16 samples of 58,000 events 153 -> 98 us (110 with the
+// batch's maps), 4096 samples' step 3380 -> 3342.
+constexpr int kFilterThreads = 256, kFilterBatch = 4;  // events of a lane in flight
 
 template <bool POOL, typename Cell>
 __global__ void __launch_bounds__(kFilterThreads)
@@ -359,10 +362,21 @@ __global__ void __launch_bounds__(kFilterThreads)
     for (int i = threadIdx.x; i < cells; i += kFilterThreads) first[i] = kNone;
     __syncthreads();
     const int64_t begin = offsets[u * t], end = min(offsets[u * t + t], cap);
-    for (int64_t k = begin + threadIdx.x; k < end; k += kFilterThreads)
+    for (int64_t k0 = begin + threadIdx.x; k0 < end; k0 += kFilterBatch * kFilterThreads)
     {
-        const int64_t q = cell.cell(events[k]);
-        if (q >= 0) atomicMin(&first[q], int32_t(k - begin));
+        uint32_t ev[kFilterBatch];
+#pragma unroll
+        for (int j = 0; j < kFilterBatch; ++j)
+        {
+            const int64_t k = k0 + j * kFilterThreads;
+            ev[j] = k < end ? events[k] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < kFilterBatch; ++j)
+        {
+            const int64_t k = k0 + j * kFilterThreads, q = k < end ? cell.cell(ev[j]) : -1;
+            if (q >= 0) atomicMin(&first[q], int32_t(k - begin));
+        }
     }
     __syncthreads();
     if (!POOL)
@@ -375,20 +389,23 @@ __global__ void __launch_bounds__(kFilterThreads)
     for (int step = warp; step < t; step += kFilterThreads / 32)
     {
         const int64_t b = offsets[u * t + step], e = min(offsets[u * t + step + 1], cap);
-        int n = 0;
-        for (int64_t k0 = b; k0 < e; k0 += 32)
+        int n = 0;  // of this lane
+        for (int64_t k0 = b; k0 < e; k0 += 32 * kFilterBatch)
         {
-            const int64_t k = k0 + lane;
-            bool kept = false;
-            if (k < e)
+            uint32_t ev[kFilterBatch];
+#pragma unroll
+            for (int j = 0; j < kFilterBatch; ++j) ev[j] = k0 + 32 * j + lane < e ? events[k0 + 32 * j + lane] : 0u;
+#pragma unroll
+            for (int j = 0; j < kFilterBatch; ++j)
             {
-                const uint32_t ev = events[k];
-                const int64_t q = cell.cell(ev);
-                kept = q >= 0 && first[q] == (POOL ? int32_t(k - begin) : ev_z(ev));
-                keep[k] = kept;
+                if (k0 + 32 * j >= e) break;
+                const int64_t k = k0 + 32 * j + lane, q = k < e ? cell.cell(ev[j]) : -1;
+                const bool kept = q >= 0 && first[q] == (POOL ? int32_t(k - begin) : ev_z(ev[j]));
+                if (k < e) keep[k] = kept;
+                n += kept;
             }
-            n += __popc(__ballot_sync(0xffffffffu, kept));
         }
+        n = __reduce_add_sync(0xffffffffu, n);
         if (lane == 0) counts[u * t + step] = n;
     }
 }
@@ -403,19 +420,27 @@ __global__ void filter_move_kernel(const int64_t *__restrict__ offsets, const ui
     const int lane = threadIdx.x & 31;
     const int64_t b = offsets[list], e = min(offsets[list + 1], cap);
     int64_t dst = out_offsets[list];
-    for (int64_t k0 = b; k0 < e; k0 += 32)
+    for (int64_t k0 = b; k0 < e; k0 += 32 * kFilterBatch)
     {
-        const int64_t k = k0 + lane;
-        const bool kept = k < e && keep[k];
-        const unsigned m = __ballot_sync(0xffffffffu, kept);
-        if (kept)
+        uint32_t ev[kFilterBatch];
+        bool kept[kFilterBatch];
+#pragma unroll
+        for (int j = 0; j < kFilterBatch; ++j)
         {
-            const uint32_t ev = events[k];
-            uint32_t o = ev;
-            if constexpr (POOL) o = ev_pack(ev_z(ev), cell.oy(ev), cell.ox(ev));
-            out[dst + __popc(m & ((1u << lane) - 1u))] = o;
+            const int64_t k = k0 + 32 * j + lane;
+            kept[j] = k < e && keep[k];
+            ev[j] = k < e ? events[k] : 0u;
         }
-        dst += __popc(m);
+#pragma unroll
+        for (int j = 0; j < kFilterBatch; ++j)
+        {
+            if (k0 + 32 * j >= e) break;
+            const unsigned m = __ballot_sync(0xffffffffu, kept[j]);
+            uint32_t o = ev[j];
+            if constexpr (POOL) o = ev_pack(ev_z(ev[j]), cell.oy(ev[j]), cell.ox(ev[j]));
+            if (kept[j]) out[dst + __popc(m & ((1u << lane) - 1u))] = o;
+            dst += __popc(m);
+        }
     }
 }
 
