@@ -271,7 +271,10 @@ __global__ void __launch_bounds__(512) fst_grad_in_kernel(FstGrad F, Stage S, fl
                                 mine[v.base + off[u]] = __fmaf_rn(wv[u], v.go, mine[v.base + off[u]]);
                         __syncwarp();  // the next entry's pixels overlap this one's
                     }
-                    // infinite and NaN weights meet the zero gradients too (NaN)
+                    // Infinite and NaN weights meet the zero gradients too (NaN).  The
+                    // vote waits for a map's weights, 11 us of an fc layer's 44; one
+                    // vote a block behind its lists took 50, the block's weights in
+                    // registers twice the time of a whole call.
                     bool odd = false;
 #pragma unroll
                     for (int u = 0; u < TP; ++u) odd |= !(fabsf(wv[u]) <= FLT_MAX);
@@ -336,32 +339,48 @@ int64_t fst_grad_w(const FstGrad &F, double *part, int64_t groups, cudaStream_t 
     return used;
 }
 
-bool fst_grad_in(const FstGrad &F, float *grad_in, cudaStream_t s)
+bool fst_grad_in(const FstGrad &F, float *grad_in, double general_us, cudaStream_t s)
 {
     if (!fits(F) || F.b > 65535) return false;
     const Stage S = stage_of(F);
     const int KK = F.kh * F.kw;
     if (KK > 128) return false;
     const int cpw = std::max(1, 32 / KK);
-    // Channels per CTA: whole warps' worth, two CTAs per SM.  A step waits for
-    // the one before it in the same warp (about 60 cycles), so where the
-    // samples leave room, 2 or 4 sets of warps share the maps, each with sums
-    // of its own.
-    int copies = F.b <= sm_count() ? 4 : 1;
-    while (copies > 1 && F.cout < copies) copies /= 2;
-    int64_t cb, warps;
-    size_t smem;
-    for (;; copies /= 2)
+    // A warp waits for each step's sums before the next (0.1 us a step and group
+    // of channels), so the steps are shared: `copies` sets of warps take turns at
+    // the maps, each with sums of its own, and a CTA takes as few channels as
+    // leave no SM without one.  Every CTA compacts all of its sample's gradients.
+    // The costs are for a third of the gradients non-zero, the kernel of
+    // temporal.cu, which takes every position, the cheaper one for dense gradients
+    // of few maps.  us, a third of the gradients / all of them / that kernel: 1 -> 32
+    // 5 x 5 on 28 x 28, 256 images 167 / 361 / 375 (two CTAs an SM with one warp at
+    // work each: 855 / 2370); 32 -> 64 3 x 3 on 14 x 14, 16 images 92 / 188 / 278, 37
+    // 112 / 232 / 289, 256 485 / 1400 / 1045; 128 -> 128, 8 images 199 / 444 / 557; 16 ->
+    // 16 on 32 x 32, 4 images 150 / 410 / 79 (not taken).
+    const double step = KK <= 32 ? 0.1 : KK <= 64 ? 0.18 : 0.36, nz = double(F.cout) * F.oh * F.ow / 3;
+    const int64_t groups = ceil_div(F.cin, cpw), blocks = ceil_div(F.cout, kMaps) * ceil_div(F.oh * F.ow, kPositions);
+    int copies = 0;
+    int64_t cb = 0, warps = 0;
+    size_t smem = 0;
+    double best = general_us;
+    for (int n = 1; n <= std::min(F.cout, kMaps); n *= 2)
     {
-        const int64_t room = (copies > 1 ? 200 : 110) * 1024 - int64_t(kListBytes);
-        cb = room / (int64_t(S.plane) * 4 * (1 + copies));
-        cb = std::min<int64_t>(std::max<int64_t>(cpw, cb / cpw * cpw), F.cin);
-        const int64_t sets = std::min<int64_t>(16 / copies, std::max<int64_t>(1, ceil_div(cb, cpw)));
-        warps = copies * std::max<int64_t>(sets, ceil_div(4, copies));
-        smem = kListBytes + size_t(cb) * S.plane * 4 * (1 + copies);
-        if (copies == 1 || smem <= 220 * 1024) break;
+        const int64_t sets = std::min<int64_t>(16 / n, groups);
+        for (int64_t each = 1;; each *= 2)  // groups of channels of a warp
+        {
+            const int64_t c = std::min<int64_t>(cpw * sets * each, F.cin), w = std::max<int64_t>(n * sets, ceil_div(4, n) * n);
+            const size_t bytes = kListBytes + size_t(c) * S.plane * 4 * (1 + n);
+            if (bytes > 220 * 1024) break;
+            const int64_t resident = std::min<int64_t>(220 * 1024 / int64_t(bytes + 1024), 64 / w);
+            const int64_t ctas = F.b * ceil_div(F.cin, c);
+            const double us = double(ceil_div(ctas, std::max<int64_t>(resident, 1) * sm_count())) *
+                              (nz / n * double(ceil_div(ceil_div(c, cpw), sets)) * step + double(blocks) * (1.0 + 5.0 / w));
+            // (more sets of sums cost their clearing and adding: for a clear gain only)
+            if (us < (n > 1 && copies > 0 && copies < n ? 0.8 : 1.0) * best) best = us, copies = n, cb = c, warps = w, smem = bytes;
+            if (c == F.cin) break;
+        }
     }
-    if (smem > 220 * 1024) return false;
+    if (copies == 0) return false;
     const auto k = KK <= 32 ? fst_grad_in_kernel<1> : KK <= 64 ? fst_grad_in_kernel<2> : fst_grad_in_kernel<4>;
     SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     k<<<dim3(unsigned(ceil_div(F.cin, cb)), unsigned(F.b)), unsigned(warps * 32), smem, s>>>(F, S, grad_in, int(cb), copies);

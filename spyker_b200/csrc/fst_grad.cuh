@@ -16,8 +16,9 @@ struct FstGrad
 // Partial sums of the kernel gradient: at least `least` sample groups, more
 // (to fill the chip) within 64 MB.
 int64_t fst_grad_w_groups(int64_t b, int64_t weights, int64_t least);
-// Returns false, having done nothing, where the layer does not fit.
-bool fst_grad_in(const FstGrad &F, float *grad_in, cudaStream_t s);
+// Returns false, having done nothing, where the layer does not fit or the other
+// kernel, of about general_us, is the faster.
+bool fst_grad_in(const FstGrad &F, float *grad_in, double general_us, cudaStream_t s);
 // part: [groups][cout * cin * kh * kw] FP64 sums over consecutive samples;
 // returns the groups written, 0 (having done nothing) where the layer does
 // not fit.

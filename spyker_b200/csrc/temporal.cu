@@ -467,7 +467,10 @@ spk_status spk_fst_conv_backward(const float *t_in, int64_t b, int64_t cin, int6
             SPK_REQUIRE(b <= 65535, "batch too large for one call (split it)");
             const dim3 grid(unsigned(ceil_div(cin, cb)), unsigned(b));
             const size_t smem = size_t(zc) * per_z * 4;
-            if (!fst_grad_in(F, grad_in, s))
+            // (0.12 us a map, tap and item of a thread, four CTAs an SM)
+            const double us = 0.12 * double(cout) * KK * double(ceil_div(cb * HW, kGiThreads)) *
+                              std::max(1.0, double(grid.x) * double(grid.y) / (4.0 * sm_count()));
+            if (!fst_grad_in(F, grad_in, us, s))
             {
                 const auto k = g.sy == 1 && g.sx == 1 ? fst_conv_grad_in_kernel<true> : fst_conv_grad_in_kernel<false>;
                 k<<<grid, kGiThreads, smem, s>>>(t_in, kernel, t_out, grad_out, grad_in, int(cin), int(cout), g, cb, zc);
