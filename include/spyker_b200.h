@@ -152,6 +152,8 @@ spk_status spk_rank_inhibit(void *data, spk_dtype type, int64_t b, int64_t t, in
                             spk_stream stream);
 
 /* ---- winner-take-all (Core::rank_convwta/rank_fcwta, impl.h:276-282) ---- */
+/* Workspace of the selection; t = 0: for U8 and I32 input, whose selection has no
+ * use for the F32 scan's part (F32 input takes the smaller one too, more slowly). */
 size_t spk_rank_convwta_workspace(int64_t b, int64_t t, int64_t c, int64_t h, int64_t w);
 /* in [B, T, C, H, W] -> winners [B, count, 5], counts [B] (cpu/wta.cpp:123-152). */
 spk_status spk_rank_convwta(const void *in, spk_dtype type, int64_t b, int64_t t, int64_t c, int64_t h, int64_t w,

@@ -516,7 +516,7 @@ inline Winners convwta(Tensor input, Expand2 radius, Size count, F64 threshold =
     const Shape s = input.shape();
     if (count == 0) return Winners(size_t(s[0]));
     Tensor rec(Type::I32, {s[0], count, 5}), cnt(Type::I32, {s[0]});
-    detail::Scratch ws(spk_rank_convwta_workspace(s[0], s[1], s[2], s[3], s[4]));
+    detail::Scratch ws(spk_rank_convwta_workspace(s[0], input.type() == Type::F32 ? s[1] : 0, s[2], s[3], s[4]));
     detail::check(spk_rank_convwta(input.data(), detail::dt(input.type()), s[0], s[1], s[2], s[3], s[4], radius[0],
                                    radius[1], count, threshold, rec.data<int32_t>(), cnt.data<int32_t>(), ws.ptr,
                                    ws.bytes, stream()),
@@ -532,7 +532,7 @@ inline Winners fcwta(Tensor input, Size radius, Size count, F64 threshold = 0)
     const Shape s = input.shape();
     if (count == 0) return Winners(size_t(s[0]));
     Tensor rec(Type::I32, {s[0], count, 5}), cnt(Type::I32, {s[0]});
-    detail::Scratch ws(spk_rank_fcwta_workspace(s[0], s[1], s[2]));
+    detail::Scratch ws(spk_rank_fcwta_workspace(s[0], input.type() == Type::F32 ? s[1] : 0, s[2]));
     detail::check(spk_rank_fcwta(input.data(), detail::dt(input.type()), s[0], s[1], s[2], radius, count, threshold,
                                  rec.data<int32_t>(), cnt.data<int32_t>(), ws.ptr, ws.bytes, stream()),
                   "fcwta");

@@ -310,7 +310,7 @@ bool fits(const FstGrad &F)
 int64_t fst_grad_w_groups(int64_t b, int64_t weights, int64_t least)
 {
     const int64_t room = (int64_t(64) << 20) / (weights * 8);
-    return std::max(least, std::min({b, room, int64_t(3 * 148)}));  // 148 SMs
+    return std::max(least, std::min({b, room, int64_t(3) * sm_count()}));
 }
 
 int64_t fst_grad_w(const FstGrad &F, double *part, int64_t groups, cudaStream_t s)

@@ -573,7 +573,8 @@ def convwta(array, radius, count: int, threshold: float = 0.0) -> Winners:
     x = Bound(array).dev
     s = to5(list(x.shape))
     rec, cnt = _winner_buffers(s[0], count, x.device)
-    ws, wsb = _workspace(_lib.lib.spk_rank_convwta_workspace(*s), x.device)
+    steps = s[1] if x.dtype == torch.float32 else 0  # (the F32 scan's part)
+    ws, wsb = _workspace(_lib.lib.spk_rank_convwta_workspace(s[0], steps, *s[2:]), x.device)
     call("spk_rank_convwta", ptr(x), type_code(x.dtype), *s, r2[0], r2[1], count, float(threshold), ptr(rec), ptr(cnt),
          ptr(ws), wsb, stream())
     return Winners(rec, cnt)
@@ -587,7 +588,8 @@ def fcwta(array, radius: int, count: int, threshold: float = 0.0) -> Winners:
     x = Bound(array).dev
     s = to3(list(x.shape))
     rec, cnt = _winner_buffers(s[0], count, x.device)
-    ws, wsb = _workspace(_lib.lib.spk_rank_fcwta_workspace(*s), x.device)
+    steps = s[1] if x.dtype == torch.float32 else 0  # (the F32 scan's part)
+    ws, wsb = _workspace(_lib.lib.spk_rank_fcwta_workspace(s[0], steps, *s[2:]), x.device)
     call("spk_rank_fcwta", ptr(x), type_code(x.dtype), *s, radius, count, float(threshold), ptr(rec), ptr(cnt), ptr(ws),
          wsb, stream())
     return Winners(rec, cnt)

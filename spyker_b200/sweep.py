@@ -155,7 +155,7 @@ class Sweep:
             self.tune()
         self.graph = None
         # the search path's networks run side by side (see _layer_search)
-        self.lanes = [torch.cuda.Stream(dev) for _ in range(min(LANES, nets))]
+        self.lanes = [torch.cuda.Stream(dev) for _ in range(min(LANES, nets))] if path == "search" else []
 
     # -- one layer of one size group, all networks -----------------------
     def _layer(self, gi, layer, x, pool, sched=None):
