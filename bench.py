@@ -34,11 +34,11 @@ sys.path.insert(0, ROOT)
 
 BATCH, T, H = 4096, 15, 28
 IN_FLIGHT = 3  # steps the host may be ahead of the GPU
-# DRAM bytes (read + write) of one conv2 layer call (its 27 launches, the
-# 4096-image step): ncu's dram__bytes_read.sum + dram__bytes_write.sum summed
-# over the call's launches, 611.6 MB read + 1169.6 MB written (1.20 GB of it
-# the layer's [B, T, 100, 14, 14] spike output).
-CONV2_TRAFFIC_BYTES = int((611.6 + 1169.6) * 1e6)
+# DRAM bytes of one conv2 layer call (25 launches) of 4096 images: four times
+# the reads of a 1024-image call (ncu's dram__bytes_read.sum over its launches,
+# 154.2 MB) and the layer's [B, T, 100, 14, 14] spike output, 1204 MB (244 of that
+# call's 301 MB had left L2 when it ended).
+CONV2_TRAFFIC_BYTES = int((4 * 154.2 + 1204.2) * 1e6)
 METRIC = "images/s (STDP train + fwd), BF16-split vs FP32 on 1 B200; spike match %"
 WORKLOAD = "kheradpisheh-2layer-stdp: 4096 x 28x28 strokes, T=15, conv1 30x5x5 th15 r3k5, conv2 100x5x5 th10 r1k8"
 
@@ -430,8 +430,10 @@ def gpu_arm(args, rank, world):
         "roofline": {"bound": "tensor", "kernel": "conv2 (30->100, 5x5, M=12.0M, K=750)", "achieved": achieved,
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": CONV2_TRAFFIC_BYTES * BATCH // 4096 if args.precision != "fp32" else None,
-                     "traffic_source": "ncu dram__bytes_read+write summed over the conv2 layer call's launches "
-                                       "(4096 images; scaled by the batch)",
+                     "traffic_source": "ncu dram__bytes_read summed over the conv2 layer call's launches (1024 images) and "
+                                       "the spike output's bytes, scaled by the batch",
+                     "achieved_counts": "the dense layer's products at every step; the search makes those of about "
+                                        "log2 T + 2 of the T steps, so this is no share of the tensor pipe",
                      "peak_source": peak_source},
         "kernels_ms": {"conv1": c1_ms, "conv2": c2_ms, "rest": ms - c1_ms - c2_ms},
         "clocks": clk.summary(),

@@ -1794,22 +1794,31 @@ __device__ __forceinline__ void search_producer(const TcParams &P, const int4 *t
     }
 }
 
-// Warp-specialised persistent kernel (544 threads; 416 without warps 13-16):
+// Warp-specialised persistent kernel (544 threads for the potentials and the
+// search, 416, without warps 13-16, for the fused and first-step kernels):
 //   warps 4-11 producers: per K block, wait for a free stage, bulk-copy the
-//              weight block (thread 128) and gather half an A row each;
-//   warp 12    one thread issues the tcgen05.mma of every stage into one of
-//              (up to) two tensor-memory accumulators and commits;
+//              weight block and build the A tile.  Search and channels-last
+//              potentials: two groups of four warps on alternate K blocks, each
+//              group's first thread copies its block's weights; otherwise all
+//              eight warps on every block, thread 128 copies;
+//   warp 12    runs the loops converged; one elected lane issues the tcgen05.mma
+//              of every stage into one of (up to) two tensor-memory accumulators
+//              and commits;
 //   warps 0-3  epilogue: read the accumulator of a finished tile (one row per
-//              thread) while the next tile is being multiplied; warps 13-16
-//              share it for the potentials and the search.
-// Stage ring: full[s] (256 producer arrivals + the weight bytes), empty[s]
-// (MMA commit); accumulators: acc_full[a] (MMA commit), acc_empty[a] (128
-// epilogue arrivals).  Every wait is bounded; a timeout raises the device
-// status word and makes every role leave.
+//              thread) while the next tile is being multiplied; warps 13-16 take
+//              the upper half of the potentials' channels, or every other tile of
+//              a search with one channel part and two accumulators (they leave at
+//              once in other searches).
+// Arrivals: full[s] one expect_tx with the weight bytes and one of each producer
+// thread of the block (128 of a group, else 256), empty[s] an MMA commit;
+// acc_full[a] an MMA commit, acc_empty[a] 256 epilogue threads for the potentials,
+// else 128.  Every wait is bounded; a timeout raises the device status word and
+// makes every role leave.
 //
-// The search kernel (kSearch) runs with 4 producer warps (288 threads) so
-// that two CTAs fit on an SM where their tensor memory allows: its
-// per-tile work is latency-bound, and a second CTA hides those latencies.
+// A search whose accumulators take at most 256 tensor-memory columns (up to 64
+// channels) runs as search_ws_kernel instead, 288 threads with 4 producer warps
+// (one group) and no second epilogue group, two CTAs an SM: its per-tile work is
+// latency-bound, and a second CTA hides those latencies.
 constexpr int kSearchThreads = 288, kMaxStages = 6;
 template <int MODE>
 constexpr int kWsThreads = MODE == kPotentials || MODE == kSearch ? 544 : 416;
@@ -1960,7 +1969,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
     }
     else if (MODE == kPotentials && warp >= 4 && warp < kMmaWarp)
     {
-        // ---------------- producers (8 warps) ----------------
+        // ---------------- producers of channel-major spikes (8 warps) ----------------
         // Thread p gathers K chunks c_lo..c_lo+3 of row prow.  The loads of the
         // next K block are issued before waiting for a free stage, so the
         // gather latency overlaps the wait and the previous block's stores.
@@ -1972,8 +1981,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
         if (tile < P.tiles)
         {
             RowInfo r = row_info<MODE>(P, tile / P.n_tiles, prow);
-            const uint8_t *ib = (MODE == kPotentials) ? P.in + r.img * P.img_stride
-                                                      : P.in + r.sample * P.img_stride + r.tstep * P.ts;
+            const uint8_t *ib = P.in + r.img * P.img_stride;
             Gathered cur;
             gather_load(P, tab, r, ib, kb, c_lo, cur);
             while (true)
@@ -1991,8 +1999,7 @@ __device__ __forceinline__ void conv_ws_body(const TcParams &P)
                     if (ntile != tile)
                     {
                         nr = row_info<MODE>(P, ntile / P.n_tiles, prow);
-                        nib = (MODE == kPotentials) ? P.in + nr.img * P.img_stride
-                                                    : P.in + nr.sample * P.img_stride + nr.tstep * P.ts;
+                        nib = P.in + nr.img * P.img_stride;
                     }
                     gather_load(P, tab, nr, nib, nkb, c_lo, nxt);
                 }

@@ -1,9 +1,10 @@
 """Temporal backprop through first-spike layers, on torch.autograd.
 
 A rank-coded layer maps input first-spike times to output first-spike times:
-the input times become cumulative spikes (``scatter``), the tensor-core conv
-gives the potentials at every step, and the output time of a neuron is the
-first step whose potential exceeds the threshold (``gather``; T = never).
+the output time of a neuron is the first step at which the sum of the weights
+of the inputs that have spiked exceeds the threshold (T = never), found by
+walking each neuron's inputs in time order or, for few steps, from the tensor
+cores' potentials of every step.
 The backward is the reference's temporal-backprop rule (the fc backward of
 src/spyker/cpu/backprop.cpp:105-160: ``select = (t_in < t_out) * grad``,
 ``next = sum kernel * select``) for conv and fc layers, run by the
@@ -44,7 +45,8 @@ def conv_forward(t_in: torch.Tensor, kernel: torch.Tensor, threshold: float, tim
                  precision: str = "bf16x3") -> torch.Tensor:
     """Output first-spike times of a conv layer (no gradient tracking).
 
-    On the tensor-core precisions one fused kernel (``spk_fst_conv_times``)
+    On the tensor-core precisions one call (``spk_fst_conv_times``: a walk of
+    each neuron's inputs or a fused tensor-core kernel, by the layer's sizes)
     writes the times without materialising the potentials; otherwise (FP32,
     or layers that do not fit one CTA) the potentials of every step are
     computed and gathered, in batch chunks."""
