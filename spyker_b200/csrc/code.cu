@@ -581,7 +581,7 @@ void large_sorted_times(const I *in, uint16_t *tm, int64_t b, int64_t t, int64_t
     uint64_t *k0 = static_cast<uint64_t *>(ws);
     uint64_t *k1 = reinterpret_cast<uint64_t *>(static_cast<char *>(ws) + ((size_t(b * xp) * 8 + 255) / 256) * 256);
     const size_t smem = size_t(kChunk) * 8;
-    SPK_CUDA(cudaFuncSetAttribute(chunk_sort_kernel<I>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(chunk_sort_kernel<I>, smem);
     chunk_sort_kernel<I><<<dim3(unsigned(xp / kChunk), unsigned(b)), kCodeThreads, smem, s>>>(in, k0, x, xp);
     SPK_LAUNCHED();
     for (int64_t L = kChunk; L < xp; L *= 2)
@@ -613,7 +613,7 @@ bool rank_reg(const I *in, O *out, int64_t b, int64_t t, int64_t x, cudaStream_t
     if (x <= 256 || x > kRegMax || b > 0x7FFFFFFF) return false;
     auto go = [&](auto k, int threads) {
         const int smem = threads * kRegItems * 10;
-        SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        allow_smem(k, smem);
         k<<<unsigned(b), threads, smem, s>>>(in, out, x, int(t));
         SPK_LAUNCHED();
         return true;
@@ -644,7 +644,7 @@ void rank_times(const void *in, spk_dtype itype, uint16_t *times, int64_t b, int
         while (npow2 < x) npow2 <<= 1;
         const size_t smem = size_t(npow2) * 8 + size_t(x) * 2 + 16;
         auto go = [&](auto k, const auto *p) {
-            SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+            allow_smem(k, smem);
             k<<<unsigned(b), kCodeThreads, smem, s>>>(p, times, x, int(t), npow2);
         };
         if (itype == SPK_F32)
@@ -714,21 +714,21 @@ spk_status spk_rank_code(const void *in, spk_dtype itype, void *out, spk_dtype o
             if (itype == SPK_F32 && otype == SPK_U8)
             {
                 auto k = rank_sorted_kernel<float, uint8_t>;
-                SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+                allow_smem(k, smem);
                 k<<<unsigned(b), kCodeThreads, smem, stream_of(stream)>>>((const float *)in, (uint8_t *)out, x, int(t),
                                                                           npow2);
             }
             else if (itype == SPK_F32 && otype == SPK_F32)
             {
                 auto k = rank_sorted_kernel<float, float>;
-                SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+                allow_smem(k, smem);
                 k<<<unsigned(b), kCodeThreads, smem, stream_of(stream)>>>((const float *)in, (float *)out, x, int(t),
                                                                           npow2);
             }
             else if (itype == SPK_U8 && otype == SPK_U8)
             {
                 auto k = rank_sorted_kernel<uint8_t, uint8_t>;
-                SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+                allow_smem(k, smem);
                 k<<<unsigned(b), kCodeThreads, smem, stream_of(stream)>>>((const uint8_t *)in, (uint8_t *)out, x,
                                                                           int(t), npow2);
             }

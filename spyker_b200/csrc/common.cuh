@@ -71,6 +71,16 @@ inline cudaStream_t stream_of(spk_stream s) { return reinterpret_cast<cudaStream
 
 int sm_count();
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory.  The limit is
+// the kernel's own, on all streams and threads, so it is never lowered: another
+// thread may be about to launch with the larger size.
+void allow_smem_of(const void *kernel, size_t bytes);
+template <typename K>
+void allow_smem(K *kernel, size_t bytes)
+{
+    allow_smem_of(reinterpret_cast<const void *>(kernel), bytes);
+}
+
 // Grid for a grid-stride loop over `work` items with `threads` per block.
 inline unsigned grid_for(int64_t work, int threads, int per_sm = 8)
 {

@@ -311,7 +311,7 @@ bool launch_tiled(const I *in, const float *kernel, float *out, int64_t n, Fp32T
     G.cb = int(std::min<int64_t>(std::min<int64_t>(G.cin, kCb), budget / (2 * per)));
     const size_t smem = size_t((G.cin > G.cb ? 2 : 1) * G.cb * per + rows) * 4;
     auto k = conv_fp32_tiled_kernel<I, KW, PX>;
-    SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(k, smem);
     const dim3 grid(unsigned(ceil_div(G.groups, int64_t(G.wp) * 32)), unsigned(ceil_div(octs, G.wc)));
     k<<<grid, kTiledWarps * 32, smem, s>>>(in, kernel, out, G);
     SPK_LAUNCHED();
@@ -362,7 +362,7 @@ void launch_fp32(const I *in, const float *kernel, float *out, int64_t n, int64_
     SPK_REQUIRE(smem <= 200 * 1024, "kernel or stride too large for the FP32 path");
     SPK_REQUIRE(n <= 65535, "N (batch x time) is limited to 65535 per call on the FP32 path");
     auto k = conv_fp32_kernel<I>;
-    SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(k, smem);
     dim3 grid(unsigned(tiles_x * tiles_y), unsigned(ceil_div(cout, kGroup)), unsigned(n));
     k<<<grid, kTileW * kTileH, smem, s>>>(in, kernel, out, int(cin), int(h), int(w), int(cout), int(kh), int(kw),
                                           int(oh), int(ow), int(sy), int(sx), int(p.top), int(p.left), tiles_x);

@@ -3465,7 +3465,7 @@ void launch(const TcParams &P, const Plan &pl, cudaStream_t s)
     const bool two = MODE == kSearch && pl.tmem_cols <= 256;
     auto kern = two ? search_ws_kernel : conv_ws_kernel<MODE>;
     const int threads = two ? kSearchThreads : kWsThreads<MODE>;
-    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.smem)));
+    allow_smem(kern, pl.smem);
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     // resident CTAs per SM: two of the search kernel sized for it (registers,
     // shared and tensor memory), one of the others (416 threads or more of 80
@@ -3946,7 +3946,7 @@ void fused_layer(const void *in, spk_dtype itype, const float *kernel, int64_t b
     {
         // (keys and positions of up to 16384 pixels: 128 KB)
         if (hw > 4096)
-            SPK_CUDA(cudaFuncSetAttribute(wta_records_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hw * 8));
+            allow_smem(wta_records_kernel, hw * 8);
         wta_records_kernel<<<unsigned(b), hw <= 256 ? 128 : hw <= 1024 ? 256 : hw <= 4096 ? 512 : 1024, size_t(hw) * 8,
                              s>>>(P.records, P.mins, P.maxs, hw, int(L.ow), int(t), int(ry), int(rx), int(count), winners,
                                   counts);

@@ -333,7 +333,7 @@ int64_t fst_grad_w(const FstGrad &F, double *part, int64_t groups, cudaStream_t 
     if (zb > 65535 || used > 65535) return 0;
     const size_t smem = kListBytes + size_t(nc) * S.plane * 4;
     const auto k = zp == 8 ? fst_grad_w_kernel<8> : zp == 4 ? fst_grad_w_kernel<4> : zp == 2 ? fst_grad_w_kernel<2> : fst_grad_w_kernel<1>;
-    SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(k, smem);
     k<<<dim3(unsigned(tb), unsigned(zb), unsigned(used)), tg * (kMaps / zp) * 32, smem, s>>>(F, S, part, tg, per, int(nc));
     SPK_LAUNCHED();
     return used;
@@ -382,7 +382,7 @@ bool fst_grad_in(const FstGrad &F, float *grad_in, double general_us, cudaStream
     }
     if (copies == 0) return false;
     const auto k = KK <= 32 ? fst_grad_in_kernel<1> : KK <= 64 ? fst_grad_in_kernel<2> : fst_grad_in_kernel<4>;
-    SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(k, smem);
     k<<<dim3(unsigned(ceil_div(F.cin, cb)), unsigned(F.b)), unsigned(warps * 32), smem, s>>>(F, S, grad_in, int(cb), copies);
     SPK_LAUNCHED();
     return true;

@@ -415,13 +415,13 @@ void fst_walk(const FstWalk &F, void *ws, cudaStream_t s)
     if (const int warps = step_warps(npix, K, F.cout, F.time))
     {
         const size_t smem = size_t(warps) * F.time * std::min(F.cout, kStepMaps) * 8;
-        SPK_CUDA(cudaFuncSetAttribute(fst_steps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        allow_smem(fst_steps_kernel, smem);
         fst_steps_kernel<<<dim3(unsigned(npix), unsigned(ceil_div(F.cout, kStepMaps))), warps * 32, smem, s>>>(A);
         SPK_LAUNCHED();
         return;
     }
     const auto k = pl.ng == 1 ? fst_walk_kernel<1> : pl.ng == 2 ? fst_walk_kernel<2> : fst_walk_kernel<4>;
-    SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.smem)));
+    allow_smem(k, pl.smem);
     int occ = 0;
     SPK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, pl.warps * 32, pl.smem));
     SPK_REQUIRE(occ > 0, "the layer does not fit one CTA");

@@ -588,7 +588,7 @@ bool inhibit_strips(float *data, int64_t b, int64_t t, int64_t c, int64_t x, flo
     const int64_t strip = 32 * t * c * 4;
     const int64_t res = std::max<int64_t>(1, std::min<int64_t>(kStripL2 / (strip * sm_count()), 64 / warps));
     const int64_t smem = std::max<int64_t>(table, 220 * 1024 / (res + 1) + 1024);
-    SPK_CUDA(cudaFuncSetAttribute(inhibit_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(inhibit_strip_kernel, smem);
     inhibit_strip_kernel<<<unsigned(strips), warps * 32, size_t(smem), s>>>(data, total, int(t), int(c), x, thr);
     SPK_LAUNCHED();
     return true;
@@ -651,7 +651,7 @@ spk_status spk_rank_pool(const void *in, void *out, spk_dtype type, int64_t n, i
                          : warp  ? pool_plane_kernel<T, 1>
                                  : pool_plane_kernel<T, 0>;
                 if (smem > 48 * 1024)
-                    SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+                    allow_smem(k, smem);
                 int occ = 0;
                 SPK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, smem));
                 const int64_t tiles = ceil_div(n, per_tile);

@@ -1,8 +1,10 @@
 // Library runtime: error reporting, device queries and the host-side kernel
 // generators of the reference's layer constructors (src/spyker/cpu/init.cpp).
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <ctime>
+#include <map>
 #include <mutex>
 #include <random>
 
@@ -28,6 +30,19 @@ int sm_count()
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+void allow_smem_of(const void *kernel, size_t bytes)
+{
+    static std::mutex lock;
+    static std::map<std::pair<int, const void *>, size_t> most;
+    int dev = 0;
+    SPK_CUDA(cudaGetDevice(&dev));
+    const std::lock_guard<std::mutex> guard(lock);
+    size_t &limit = most[{dev, kernel}];
+    const size_t want = std::max(limit, bytes);
+    SPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(want)));
+    limit = want;
 }
 
 size_t dtype_size(spk_dtype t)

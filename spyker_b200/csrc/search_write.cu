@@ -306,7 +306,7 @@ void search_write(const SearchWrite &W, cudaStream_t s)
     else if (phw * unit <= kTableBytes && ohw * unit <= kRangeBytes) nc = std::min<int64_t>(unit, W.C);
     A.nc = int(nc);
     const size_t smem = (A.codes ? 0 : size_t(2 * ext_bytes(ohw))) + (A.ptab ? size_t(nc * phw + 32) & ~size_t(15) : 0);
-    SPK_CUDA(cudaFuncSetAttribute(search_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(search_write_kernel, smem);
     const dim3 grid(unsigned(ceil_div(W.C, nc)), unsigned(std::min<int64_t>(W.b, 65535)));
     search_write_kernel<<<grid, kThreads, smem, s>>>(A);
     SPK_LAUNCHED();

@@ -140,14 +140,14 @@ void times_to_lists(const uint16_t *tm, int64_t u, int64_t t, int64_t c, int64_t
     void *scan_ws = ws.take<char>(scan_workspace(u * t));
     const size_t hist = size_t(t) * 4;
     if (hist > 48 * 1024)
-        SPK_CUDA(cudaFuncSetAttribute(times_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hist)));
+        allow_smem(times_count_kernel, hist);
     times_count_kernel<<<unsigned(u), 256, hist, s>>>(tm, x, int(t), counts);
     SPK_LAUNCHED();
     scan_exclusive<int32_t>(counts, offsets, u * t, scan_ws, s);
     const int warps = int(std::max<int64_t>(1, std::min<int64_t>(8, 8192 / t)));
     const size_t cur = size_t(warps) * t * 4;
     if (cur > 48 * 1024)
-        SPK_CUDA(cudaFuncSetAttribute(times_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cur)));
+        allow_smem(times_scatter_kernel, cur);
     times_scatter_kernel<<<unsigned(u), warps * 32, cur, s>>>(tm, x, int(t), int(h), int(w), offsets, events);
     SPK_LAUNCHED();
 }
@@ -464,7 +464,7 @@ void filter_lists(const int64_t *offsets, const uint32_t *events, int64_t in_cap
         void *scan_ws = ws.take<char>(scan_workspace(lists));
         const size_t smem = size_t(ncells) * 4;
         const auto k = filter_sample_kernel<POOL, Cell>;
-        SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        allow_smem(k, smem);
         k<<<unsigned(u), kFilterThreads, smem, s>>>(offsets, events, in_cap, int(t), cell, keep, counts);
         SPK_LAUNCHED();
         scan_exclusive<int32_t>(counts, out_offsets, lists, scan_ws, s);
@@ -889,7 +889,7 @@ bool conv_maps(const int64_t *offsets, const uint32_t *events, int64_t u, int t,
     const MapsArgs A{offsets, events, wt,     fired, ends,       counts,      counts + lists, tasks, int(plane / 4), t, c, cout,
                      groups,  bands,  rows,   int(p.top), int(p.left), oh,    ow,    thr};
     const auto kern = k5 ? sparse_conv_maps_kernel<5, 5> : sparse_conv_maps_kernel<3, 3>;
-    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(wpc * plane)));
+    allow_smem(kern, wpc * plane);
     kern<<<unsigned(ceil_div(tasks, wpc)), wpc * 32, size_t(wpc * plane), s>>>(A);
     SPK_LAUNCHED();
     scan_exclusive<int32_t>(counts, out_offsets, lists, scan_ws, s);
@@ -1196,7 +1196,7 @@ spk_status spk_sparse_gather(const int64_t *offsets, const uint32_t *events, int
             const size_t smem = size_t(c * h * w) * 4;
             dispatch(otype, [&](auto z) {
                 const auto k = gather_sample_kernel<decltype(z)>;
-                SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+                allow_smem(k, smem);
                 k<<<unsigned(u), 256, smem, s>>>(offsets, events, int(t), int(c), int(h), int(w), (decltype(z) *)out);
                 SPK_LAUNCHED();
             });
@@ -1420,8 +1420,7 @@ spk_status spk_sparse_stdp(const int64_t *offsets, const uint32_t *events, int64
         if (c * hp * wp <= kSmemCells)
         {
             const size_t smem = size_t(c * hp * wp) * 4;
-            SPK_CUDA(cudaFuncSetAttribute(sparse_prepost_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(smem)));
+            allow_smem(sparse_prepost_sample_kernel, smem);
             sparse_prepost_sample_kernel<<<unsigned(u), 256, smem, s>>>(offsets, events, int(t), int(c), int(hp),
                                                                         int(wp), int(p.top), int(p.left), int(kh),
                                                                         int(kw), winners, counts, int(count), pre, post);

@@ -345,7 +345,7 @@ void launch_wta(const void *in, int64_t b, int64_t t, int64_t c, int64_t h, int6
         }
     }
     auto k = wta_kernel<T, kFloat>;
-    SPK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    allow_smem(k, smem);
     k<<<unsigned(b), kWtaThreads, smem, s>>>((const T *)in, int(t), x, int(c), int(h), int(w), int(ry), int(rx),
                                              int(count), whole, scalar_to<T>(thr), winners, counts, gkeys, C);
     SPK_LAUNCHED();
