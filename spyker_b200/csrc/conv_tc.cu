@@ -3674,28 +3674,33 @@ struct Nets
 // device (each launch reads them).  Off the search path (device flags) every
 // one of these kernels leaves at once, except the writer, which zero-fills
 // the spikes for the dense kernel.
-// Whether the walk (search_walk.cuh) is the faster search.  Its time grows with
-// the pixels and, per pixel, with the inputs of a receptive field and the
-// channels a lane holds (at most some 0.02 ns a pixel and input for one channel a
-// lane, less the earlier the pixels cross); with fewer pixels than the chip has
-// warps it is the latency of one.  The rounds take some 35 us each (25 without
-// the pre-filter, whose launches join the first) before the pixels count.  The
-// line is where both take the same for a threshold of some 15 % of the summed
-// weights: an early crossing would put it at twice the pixels, one at 30 % at
-// half.  us, walk at 5 / 10 / 30 %, rounds, T = 15: 2 -> 30 channels 5 x 5, 131k
-// pixels 180 / 183 / 214, 271 (128 Ki at most); 8 -> 32, 44k 117 / 128 / 176, 260,
-// 87k 177 / 199 / 291, 290; 30 -> 100, 4.5k 107 / 123 / 192, 275, 9k 176 / 214 /
-// 360, 270, 14k 251 / 318 / 507, 270; 64 -> 64 3 x 3, 8.6k 110 / 121 / 166, 205,
-// 16k 153 / 171 / 253, 205, 34k 254 / 288 / 463, 228; 64 -> 32 5 x 5, 7.4k 151 /
-// 180 / 298, 240; 64 -> 100, 2.7k 140 / 176 / 303, 237; 8 -> 256, 12k 172 / 216 /
-// 356, 280; 64 -> 256, 2.3k 215 / 270 / 500, 300, 16k 2260 at 15 %, 650.
-bool walk_pays(int64_t npix, int inputs, int cout, int T, bool prefilter, bool wta)
+// Whether the walk (search_walk.cuh) is the faster search: an estimate of both in
+// us.  A pixel of the walk sorts its inputs and adds the weights of those that fire
+// up to its crossing; how many those are is not known here, so weights of some 0.8
+// are taken for it (a trained kernel's lie in [0, 1]), which for smaller ones
+// errs by a factor of two at the line and for larger ones towards the rounds.
+// With fewer pixels than the chip has warps the walk is the latency of one.  The
+// rounds are a fixed time each (some 20 launches, each tile's chain of K blocks and
+// channel parts) before the pixels count.  us, walk with the threshold at 5 / 10 /
+// 30 % of the summed weights, rounds, T = 15: 2 -> 30 channels 5 x 5, 131k pixels 180 /
+// 183 / 214, 271 (128 Ki at most); 8 -> 32, 87k 177 / 199 / 291, 290; 30 -> 100, 4.5k
+// 107 / 123 / 192, 275, 9k 176 / 214 / 360, 270, 18k 335 / 422 / 669, 270; 64 -> 64 3 x 3,
+// 16k 153 / 171 / 253, 205, 34k 254 / 288 / 463, 228; 64 -> 32 5 x 5, 15k 220 / 271 /
+// 475, 246; 64 -> 100, 2.7k 140 / 176 / 303, 237; 8 -> 256, 12k 172 / 216 / 356, 280;
+// 64 -> 256, 2.3k 211 / 270 / 497, 300, 16k 2260 at 15 %, 650.
+bool walk_pays(const TcParams &P, int inputs, int kblocks, int parts, bool prefilter, bool wta)
 {
+    if (P.npix > 128 * 1024) return false;
+    const int lanes = P.cout <= 32 ? 0 : P.cout <= 64 ? 1 : P.cout <= 128 ? 2 : 3;  // 1, 2, 4, 8 channels
+    const double sort = 1e-3 * (lanes == 0 ? 5 : lanes == 1 ? 9 : lanes == 2 ? 12.5 : 32);   // ns an input
+    const double adds = 1e-3 * (lanes == 0 ? 40 : lanes == 1 ? 45 : lanes == 2 ? 110 : 330);
+    const double share = std::min(std::max(double(P.thr) / (0.8 * inputs), 0.05), 0.4);
+    const double pixels = double(std::max<int64_t>(P.npix, 8 * sm_count()));
+    const double walk = 45.0 + 1e-3 * pixels * (0.6 + inputs * (sort + adds * share));
     int rounds = wta ? 2 : 1;
-    for (int steps = 1; steps < T; steps *= 2) ++rounds;
-    const double lane = cout <= 32 ? 1.0 : cout <= 64 ? 1.2 : cout <= 128 ? 2.75 : 7.5;  // 1, 2, 4, 8 channels
-    const double pixels = double(std::max<int64_t>(npix, 8 * sm_count()));
-    return npix <= 128 * 1024 && pixels * (inputs + 20) * lane <= rounds * (prefilter ? 3.6e6 : 2.4e6);
+    for (int steps = 1; steps < P.T; steps *= 2) ++rounds;
+    const double each = (prefilter ? 38.0 : 30.0) + 0.4 * kblocks * parts;
+    return walk <= rounds * each + 1e-3 * double(P.npix) * (0.5 + 8e-4 * inputs * (1 << lanes));
 }
 
 void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel, int64_t count, int64_t pool_ky,
@@ -3748,7 +3753,8 @@ void search_layer(const TcParams &P0, const FusedLayout &L, const float *kernel,
     // Walking each pixel's inputs in spike order (search_walk.cuh) instead of
     // the rounds below.
     const int groups = taps * (P.cpad / 8);
-    if (P.nhwc && P.T <= 32 && groups <= 256 && P.cout <= 256 && walk_pays(L.npix, kr, P.cout, P.T, prefilter, count > 0))
+    if (P.nhwc && P.T <= 32 && groups <= 256 && P.cout <= 256 &&
+        walk_pays(P, kr, pl.kblocks, pl.parts, prefilter, count > 0))
     {
         // (the integers take the weight image's bytes: four per input and
         // channel in both)

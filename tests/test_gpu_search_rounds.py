@@ -17,9 +17,9 @@ pytestmark = pytest.mark.gpu
 LAYERS = [
     # b, t, cin, h, w, cout, k, pad, theta, radius, count
     (172, 15, 2, 28, 28, 30, 5, 2, 15.0, 3, 5),
-    (58, 15, 30, 14, 14, 100, 5, 2, 10.0, 1, 8),
+    (125, 15, 30, 14, 14, 100, 5, 2, 10.0, 1, 8),
 ]
-PARTS = (110, 6, 16, 10, 10, 256, 5, 2, 10.0, 1, 4)  # two parts of 128 channels
+PARTS = (150, 6, 16, 10, 10, 256, 5, 2, 10.0, 1, 4)  # two parts of 128 channels
 
 
 def rounds(port, x, w, *args, **kwargs):
@@ -67,7 +67,8 @@ def test_trained_weights(port, trained):  # noqa: F811
     w1, w2, codes = trained
     spk1 = port.fire(port.inhibit(port.threshold(port.conv(codes, w1, (1, 1), (2,) * 4), 15.0)))
     assert rounds(port, np.concatenate([codes, codes[::-1]]), w1, 15.0, 3, 5, 2)[0] > 0
-    assert rounds(port, port.pool(spk1, (2, 2)), w2, 10.0, 1, 8, 2, pool=7)[0] > 0
+    maps = port.pool(spk1, (2, 2))
+    assert rounds(port, np.concatenate([maps, maps[::-1]]), w2, 10.0, 1, 8, 2, pool=7)[0] > 0
 
 
 @pytest.mark.parametrize("schedule", [(2, 1, 1), (3, 2, 1), (6, 1, 2)])
@@ -86,7 +87,7 @@ def test_schedules(port, schedule):
 def test_walk_and_rounds_agree():
     """A layer of 256 channels in one call (rounds) and image by image (walk)."""
     g = torch.Generator("cuda").manual_seed(4)
-    x = (torch.randint(0, 12, (60, 1, 12, 16, 16), generator=g, device="cuda")
+    x = (torch.randint(0, 12, (100, 1, 12, 16, 16), generator=g, device="cuda")
          <= torch.arange(9, device="cuda").view(1, 9, 1, 1, 1)).to(torch.uint8)
     conv = spyker.Conv(12, 200, 5, pad=2)
     conv.kernel.copy_(torch.exp2(-20 * torch.rand(conv.kernel.shape, generator=g, device="cuda")))
@@ -95,7 +96,7 @@ def test_walk_and_rounds_agree():
     n = count()
     spk, wins, pooled = spyker.conv_fire_wta(x, conv, 8.0, 1, 5, pool=2)
     assert count() - n > 12
-    for i in range(0, 60, 13):
+    for i in range(0, 100, 23):
         n = count()
         s, w, p = spyker.conv_fire_wta(x[i:i + 1], conv, 8.0, 1, 5, pool=2)
         assert count() - n < 12
