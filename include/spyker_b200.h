@@ -264,7 +264,7 @@ spk_status spk_conv(const void *in, spk_dtype itype, const float *kernel, float 
  * near-threshold decision is re-made exactly at either split).  With no
  * negative weight, cumulative 0/1 input and value <= the inhibit / fire / WTA
  * thresholds <= threshold, the layer runs as a first-crossing search on
- * exact integer sums (u8 tensor cores, or, for few output pixels, each pixel's
+ * exact integer sums (u8 tensor cores, or, for layers of less work, each pixel's
  * inputs in spike order) instead of the dense kernel; results are the same.  spk_recheck_count / spk_recompute_count count its rows
  * re-decided from exact sums and recomputed from the F32 weights. */
 size_t spk_conv_fire_wta_workspace(int64_t b, int64_t t, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh,
