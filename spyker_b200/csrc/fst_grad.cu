@@ -368,15 +368,18 @@ bool fst_grad_in(const FstGrad &F, float *grad_in, double general_us, cudaStream
         const int64_t sets = std::min<int64_t>(16 / n, groups);
         for (int64_t each = 1;; each *= 2)  // groups of channels of a warp
         {
-            const int64_t c = std::min<int64_t>(cpw * sets * each, F.cin), w = std::max<int64_t>(n * sets, ceil_div(4, n) * n);
+            const int64_t c = std::min<int64_t>(cpw * sets * each, F.cin);
+            const int64_t w = std::max<int64_t>(n * sets, ceil_div(4, n) * n);
             const size_t bytes = kListBytes + size_t(c) * S.plane * 4 * (1 + n);
             if (bytes > 220 * 1024) break;
             const int64_t resident = std::min<int64_t>(220 * 1024 / int64_t(bytes + 1024), 64 / w);
             const int64_t ctas = F.b * ceil_div(F.cin, c);
+            const double walk = nz / n * double(ceil_div(ceil_div(c, cpw), sets)) * step;
             const double us = double(ceil_div(ctas, std::max<int64_t>(resident, 1) * sm_count())) *
-                              (nz / n * double(ceil_div(ceil_div(c, cpw), sets)) * step + double(blocks) * (1.0 + 5.0 / w));
+                              (walk + double(blocks) * (1.0 + 5.0 / w));
             // (more sets of sums cost their clearing and adding: for a clear gain only)
-            if (us < (n > 1 && copies > 0 && copies < n ? 0.8 : 1.0) * best) best = us, copies = n, cb = c, warps = w, smem = bytes;
+            const double gain = copies > 0 && copies < n ? 0.8 : 1.0;
+            if (us < gain * best) best = us, copies = n, cb = c, warps = w, smem = bytes;
             if (c == F.cin) break;
         }
     }

@@ -382,7 +382,8 @@ bool fst_walk_pays(int64_t npix, int64_t cin, int64_t taps, int64_t cout, int64_
     while (steps < time) steps *= 2;
     // ns
     const double input = cout <= 32 ? 0.019 : cout <= 64 ? 0.023 : 0.034;
-    const double walk = 12e3 + double(std::max<int64_t>(npix * ceil_div(cout, 128), 16 * sm_count())) * (0.6 + input * K);
+    const int64_t pixels = std::max<int64_t>(npix * ceil_div(cout, 128), 16 * sm_count());
+    const double walk = 12e3 + double(pixels) * (0.6 + input * K);
     const double row = 0.04 + std::max(0.034 * kblocks, 0.0062 * columns);
     const double dense = 22e3 + 650.0 * kblocks + 100.0 * columns +
                          double(std::max<int64_t>(npix * steps - 128 * sm_count(), 0)) * row;

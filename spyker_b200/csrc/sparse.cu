@@ -886,8 +886,8 @@ bool conv_maps(const int64_t *offsets, const uint32_t *events, int64_t u, int t,
     // 32 bands)
     const int64_t plane = std::max<int64_t>(int64_t(rows) * ow * 128, int64_t(oh) * ow * 4);
     const int wpc = plane * 4 <= 100 * 1024 ? 4 : 1;
-    const MapsArgs A{offsets, events, wt,     fired, ends,       counts,      counts + lists, tasks, int(plane / 4), t, c, cout,
-                     groups,  bands,  rows,   int(p.top), int(p.left), oh,    ow,    thr};
+    const MapsArgs A{offsets, events, wt, fired, ends, counts, counts + lists, tasks, int(plane / 4), t, c, cout, groups,
+                     bands, rows, int(p.top), int(p.left), oh, ow, thr};
     const auto kern = k5 ? sparse_conv_maps_kernel<5, 5> : sparse_conv_maps_kernel<3, 3>;
     allow_smem(kern, wpc * plane);
     kern<<<unsigned(ceil_div(tasks, wpc)), wpc * 32, size_t(wpc * plane), s>>>(A);
