@@ -12,10 +12,11 @@
 // is within 2^-18 relative.
 //
 // Two A layouts:
-//  * channels-last (Cin >= 2, where the workspace holds it): the spikes are
-//    first transposed to [N, H, W, Cpad] u8 (Cpad = Cin rounded up to 8) and
-//    k = tap * Cpad + c, so every 8-wide K chunk of a row is one 8-byte load
-//    (16 bytes where Cpad is a multiple of 16);
+//  * channels-last (Cin >= 8, and fewer where a fused layer may take the
+//    search path): the spikes are first transposed to [N, H, W, Cpad] u8
+//    (Cpad = Cin rounded up to 8) and k = tap * Cpad + c, so every 8-wide K
+//    chunk of a row is one 8-byte load (16 bytes where Cpad is a multiple of
+//    16);
 //  * channel-major: k = c * KH*KW + tap (the reference's order), gathered
 //    element by element.
 //
@@ -3549,28 +3550,23 @@ FusedLayout fused_layout(int64_t b, int64_t t, int64_t cin, int64_t h, int64_t w
 }
 }  // namespace
 
-// The plan of the potentials kernel.  From 2 input channels on the spikes are
-// first copied channels-last (one 8-byte load per tap and 8 channels instead
-// of a byte per element: the three layers of the reward-modulated network on 200 images 2432 ->
-// 1757 us with the FP32 epilogue), where the
-// padded K and the workspace allow it.
+// The plan of the potentials kernel.  Channels-last from 8 input channels: with
+// fewer, K padded to 8 per tap takes more FP32 sums of the tensor cores (6
+// channels, 5x5: 4 K blocks instead of 3) and the potentials are further off
+// for weights near 0 and 1 (mean error 6.71e-8 against 6.39e-8 of the sums of
+// magnitudes, largest of 3 channels, 7x7 5.6e-7 against 3.9e-7), although the
+// copy's 8-byte loads are the faster ones (the three layers of the
+// reward-modulated network on 200 images 1246 us, from byte gathers 1905).
 static Plan potentials_plan(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh, int64_t kw,
-                            int precision, size_t ws_bytes)
+                            int precision)
 {
-    if (cin >= 2 && cin < 8)
-    {
-        const Plan pl = make_plan(n, cin, h, w, cout, kh, kw, precision, false, 0, false, 0, true);
-        if (pl.kblocks <= kMaxKBlocks && pl.stages >= 2 && pl.smem <= 227 * 1024 &&
-            ws_bytes >= align256(pl.wimg_bytes) + align256(pl.xt_bytes))
-            return pl;
-    }
     return make_plan(n, cin, h, w, cout, kh, kw, precision, false);
 }
 
 size_t conv_tc_workspace(int64_t n, int64_t cin, int64_t h, int64_t w, int64_t cout, int64_t kh, int64_t kw,
                          int precision)
 {
-    const Plan pl = potentials_plan(n, cin, h, w, cout, kh, kw, precision, SIZE_MAX);
+    const Plan pl = potentials_plan(n, cin, h, w, cout, kh, kw, precision);
     return align256(pl.wimg_bytes) + align256(pl.xt_bytes);
 }
 
@@ -3579,7 +3575,7 @@ void conv_tc(const void *in, spk_dtype itype, const float *kernel, float *out, i
              int precision, void *ws, size_t ws_bytes, cudaStream_t s)
 {
     if (itype != SPK_U8) throw Error(SPK_ERR_UNSUPPORTED, "the tensor-core path takes U8 spikes");
-    const Plan pl = potentials_plan(n, cin, h, w, cout, kh, kw, precision, ws_bytes);
+    const Plan pl = potentials_plan(n, cin, h, w, cout, kh, kw, precision);
     SPK_REQUIRE(ws != nullptr && ws_bytes >= align256(pl.wimg_bytes) + align256(pl.xt_bytes), "workspace is too small");
     TcParams P = prepare(pl, in, kernel, n, cin, h, w, cout, kh, kw, sy, sx, p, oh, ow, static_cast<uint8_t *>(ws), s);
     P.out = out;
